@@ -171,6 +171,9 @@ _SIGS = {
     "b12g_profile_enable": (C.c_int, [C.c_void_p, C.c_int]),
     "b12g_profile_read": (C.c_int, [C.c_void_p, C.c_uint32, C.POINTER(C.c_double), C.POINTER(C.c_uint64), C.c_int]),
     "b12g_launch_count": (C.c_int, [C.POINTER(C.c_uint64)]),
+    "b12g_screen_probe": (C.c_int, [C.POINTER(Domain), C.POINTER(Map), C.c_uint8, C.c_double, C.c_void_p, C.c_void_p,
+                                    C.c_uint64, C.c_int, C.POINTER(C.c_int), C.c_void_p, C.c_void_p, C.c_void_p,
+                                    C.c_void_p]),
     "b12g_probe_fp64_fma": (C.c_int, [C.c_double, C.POINTER(C.c_double), C.POINTER(C.c_double)]),
 }
 

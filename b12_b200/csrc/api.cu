@@ -141,6 +141,31 @@ bool stored_rows_fit(b12g_tree* t, const b12g_scheme* sc, const Prepared& pr)
   return same_scheme(*sc, t->tgt_scheme);
 }
 
+void fill_domain(const b12g_domain& domain, Domain& dom)
+{
+  for (uint32_t j = 0; j < B12G_MAX_DIM; ++j) {
+    const double c = j < domain.dim ? domain.center[j] : 0.0, r = j < domain.dim ? domain.radius[j] : 1.0;
+    dom.c[j] = c;
+    dom.r[j] = r;
+    dom.lo[j] = c - r;
+    dom.hi[j] = c + r;
+    // the point-code fast path multiplies by RN(1/r) (checked against the IEEE quotient
+    // per point); radii far from 1 keep the division alone
+    dom.inv_r[j] = (r >= 0x1p-500 && r <= 0x1p500) ? 1.0 / r : 0.0;
+  }
+}
+
+void fill_map(const b12g_map& m, MapParams& mp)
+{
+  mp.h = m.h;
+  mp.h2 = m.h / 2.0;
+  mp.h3 = m.h / 3.0;
+  mp.h6 = m.h / 6.0;
+  for (int i = 0; i < 6; ++i) mp.p[i] = m.p[i];
+  mp.steps = m.steps;
+  mp.table = nullptr;
+}
+
 b12g_status prepare(b12g_tree* t, const b12g_scheme* sc, Prepared& pr)
 {
   if (!sc) return fail(B12G_ERR_INVALID, "scheme is NULL");
@@ -153,13 +178,7 @@ b12g_status prepare(b12g_tree* t, const b12g_scheme* sc, Prepared& pr)
   ImageArgs& a = pr.a;
   a.dom = t->dom;
   MapParams& mp = a.map;
-  mp.h = m.h;
-  mp.h2 = m.h / 2.0;
-  mp.h3 = m.h / 3.0;
-  mp.h6 = m.h / 6.0;
-  for (int i = 0; i < 6; ++i) mp.p[i] = m.p[i];
-  mp.steps = m.steps;
-  mp.table = nullptr;
+  fill_map(m, mp);
   if (m.kind == B12G_MAP_FORCED_DUFFING) {
     // cos at the stage times t = j * h / 2 (period = steps * h)
     std::vector<double> tab(2 * size_t(m.steps) + 1);
@@ -398,16 +417,7 @@ b12g_status b12g_tree_create(const b12g_domain* domain, b12g_tree** out)
   b12g_tree* t = new b12g_tree();
   cudaGetDevice(&t->device);
   t->domain = *domain;
-  for (uint32_t j = 0; j < B12G_MAX_DIM; ++j) {
-    const double c = j < domain->dim ? domain->center[j] : 0.0, r = j < domain->dim ? domain->radius[j] : 1.0;
-    t->dom.c[j] = c;
-    t->dom.r[j] = r;
-    t->dom.lo[j] = c - r;
-    t->dom.hi[j] = c + r;
-    // the point-code fast path multiplies by RN(1/r) (checked against the IEEE quotient
-    // per point); radii far from 1 keep the division alone
-    t->dom.inv_r[j] = (r >= 0x1p-500 && r <= 0x1p500) ? 1.0 / r : 0.0;
-  }
+  fill_domain(*domain, t->dom);
   b12g_status st = B12G_OK;
   if (cudaStreamCreateWithFlags(&t->stream, cudaStreamNonBlocking) != cudaSuccess) st = cuda_fail(cudaGetLastError(), "stream");
   if (st == B12G_OK && cudaMallocHost(&t->h_ctr, C_COUNT * sizeof(uint32_t)) != cudaSuccess)

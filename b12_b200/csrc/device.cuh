@@ -688,34 +688,43 @@ template<class A>
 struct LorenzMap {
   static constexpr int D = 3;
   static __device__ __forceinline__ void rhs(const MapParams& m, const double* x, double* r);
+  // one RK4 step from x; x and res become the new state
+  static __device__ __forceinline__ void step(const MapParams& m, double (&x)[3], double* res)
+  {
+    double k[3], a[3];
+    rhs(m, x, k);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) { res[j] = A::madd(m.h6, k[j], x[j]); a[j] = A::madd(m.h2, k[j], x[j]); }
+    rhs(m, a, k);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) { res[j] = A::madd(m.h3, k[j], res[j]); a[j] = A::madd(m.h2, k[j], x[j]); }
+    rhs(m, a, k);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) { res[j] = A::madd(m.h3, k[j], res[j]); a[j] = A::madd(m.h, k[j], x[j]); }
+    rhs(m, a, k);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) { res[j] = A::madd(m.h6, k[j], res[j]); x[j] = res[j]; }
+  }
   static __device__ __forceinline__ void apply(const MapParams& m, const double* x0, double* res)
   {
-    double x0_ = x0[0], x1 = x0[1], x2 = x0[2];
-    double x[3] = {x0_, x1, x2}, k[3], a[3];
-    auto step = [&]() {
-      rhs(m, x, k);
-#pragma unroll
-      for (int j = 0; j < 3; ++j) { res[j] = A::madd(m.h6, k[j], x[j]); a[j] = A::madd(m.h2, k[j], x[j]); }
-      rhs(m, a, k);
-#pragma unroll
-      for (int j = 0; j < 3; ++j) { res[j] = A::madd(m.h3, k[j], res[j]); a[j] = A::madd(m.h2, k[j], x[j]); }
-      rhs(m, a, k);
-#pragma unroll
-      for (int j = 0; j < 3; ++j) { res[j] = A::madd(m.h3, k[j], res[j]); a[j] = A::madd(m.h, k[j], x[j]); }
-      rhs(m, a, k);
-#pragma unroll
-      for (int j = 0; j < 3; ++j) { res[j] = A::madd(m.h6, k[j], res[j]); x[j] = res[j]; }
-    };
+    double x[3] = {x0[0], x0[1], x0[2]};
     if (m.steps == 20) {
       // the configured step count with no loop instructions between the steps
 #pragma unroll
-      for (int s = 0; s < 20; ++s) step();
+      for (int s = 0; s < 20; ++s) step(m, x, res);
     } else {
       // four steps per trip: the loop's own counter and branch instructions would
       // otherwise take a twentieth of the issue slots at 20 steps
 #pragma unroll 4
-      for (uint32_t s = 0; s < m.steps; ++s) step();
+      for (uint32_t s = 0; s < m.steps; ++s) step(m, x, res);
     }
+  }
+  // the same in little code, for the few points that need it beside a screened evaluation
+  static __device__ __forceinline__ void apply_cold(const MapParams& m, const double* x0, double* res)
+  {
+    double x[3] = {x0[0], x0[1], x0[2]};
+#pragma unroll 1
+    for (uint32_t s = 0; s < m.steps; ++s) step(m, x, res);
   }
 };
 

@@ -40,26 +40,38 @@ struct PointImage {
     for (int j = 0; j < D; ++j) bits[j] = deinterleave<D>(code, a.depth, j);
   }
 
-  // returns whether the image point lies in the domain; `tbits` its box's per-dimension
-  // indices at a.depth.  `pts` is the block's grid-point table (dimension-major, P
-  // entries per dimension) when the grid has one, else the 1-D coordinate table.
-  // the same from the source box's centre (its radius is the launch's)
-  static __device__ __forceinline__ bool image_at(const ImageArgs& a, const double* pts, bool use_table,
-                                                  const double (&c)[D], uint64_t i, uint32_t k, uint32_t (&tbits)[D])
+  // grid point k of a box (point i of the launch).  `pts` is the block's grid-point table
+  // (dimension-major, P entries per dimension) when the grid has one, else the 1-D
+  // coordinate table.
+  static __device__ __forceinline__ void grid_point(const ImageArgs& a, const double* pts, bool use_table, uint64_t i,
+                                                    uint32_t k, double (&g)[D])
   {
-    double g[D], x[D], y[D];
     if (Grid::kTable && use_table) {
 #pragma unroll
       for (int j = 0; j < D; ++j) g[j] = pts[j * uint32_t(a.points) + k];
     } else {
       Grid::template point<D>(a.grid, pts, i, k, g);
     }
+  }
+
+  // returns whether the image point lies in the domain; `tbits` its box's per-dimension
+  // indices at a.depth; from the source box's centre (its radius is the launch's).
+  // kCold: the evaluation of the few points that a screened launch could not decide
+  template<bool kCold = false>
+  static __device__ __forceinline__ bool image_at(const ImageArgs& a, const double* pts, bool use_table,
+                                                  const double (&c)[D], uint64_t i, uint32_t k, uint32_t (&tbits)[D])
+  {
+    double g[D], x[D], y[D];
+    grid_point(a, pts, use_table, i, k, g);
 #pragma unroll
     for (int j = 0; j < D; ++j) x[j] = __dadd_rn(c[j], __dmul_rn(g[j], a.dc.ax[j].rk));
-    Map::apply(a.map, x, y);
+    if constexpr (kCold) Map::apply_cold(a.map, x, y);
+    else Map::apply(a.map, x, y);
     return point_bits<D>(a.dom, a.dc, y, tbits);
   }
 
+  // the same from the source box's indices
+  template<bool kCold = false>
   static __device__ __forceinline__ bool image(const ImageArgs& a, const double* pts, bool use_table,
                                                const uint32_t (&sbits)[D], uint64_t i, uint32_t k,
                                                uint32_t (&tbits)[D])
@@ -67,7 +79,34 @@ struct PointImage {
     double c[D], r;
 #pragma unroll
     for (int j = 0; j < D; ++j) box_axis(a.dom, a.dc.ax[j], j, sbits[j], c[j], r);
-    return image_at(a, pts, use_table, c, i, k, tbits);
+    return image_at<kCold>(a, pts, use_table, c, i, k, tbits);
+  }
+
+  // the screened evaluation from the source box's indices: whether it decided the point
+  static __device__ __forceinline__ bool screened(const ImageArgs& a, const double* pts, bool use_table,
+                                                  const uint32_t (&sbits)[D], uint64_t i, uint32_t k,
+                                                  uint32_t (&tbits)[D], bool& valid)
+  {
+    double g[D], x[D];
+    grid_point(a, pts, use_table, i, k, g);
+#pragma unroll
+    for (int j = 0; j < D; ++j)
+      x[j] = __fma_rn(g[j], a.sc.sR[j], __fma_rn(screen_index(sbits[j], a.sc.bits[j]), a.sc.sA[j], a.sc.sB[j]));
+    const bool kept = Screen<Map>::run(a.sc, a.map, x);
+    return screen_locate<D>(a.sc, x, tbits, valid) && kept;
+  }
+
+  // the same from its centre
+  static __device__ __forceinline__ bool screened_at(const ImageArgs& a, const double* pts, bool use_table,
+                                                     const double (&c)[D], uint64_t i, uint32_t k,
+                                                     uint32_t (&tbits)[D], bool& valid)
+  {
+    double g[D], x[D];
+    grid_point(a, pts, use_table, i, k, g);
+#pragma unroll
+    for (int j = 0; j < D; ++j) x[j] = __fma_rn(g[j], a.sc.sR[j], __fma_rn(c[j], a.sc.sC[j], a.sc.sD[j]));
+    const bool kept = Screen<Map>::run(a.sc, a.map, x);
+    return screen_locate<D>(a.sc, x, tbits, valid) && kept;
   }
 
   // centre of source `rank` from the launch's table
@@ -122,8 +161,13 @@ __device__ __forceinline__ bool load_points(const GridParams& g, uint64_t P, dou
   return table;
 }
 
-template<class Map, class Grid, ImageMode M>
-__global__ void __launch_bounds__(kThreads, 6) image_points_kernel(const ImageArgs a)
+// Bound by instruction issue: an FP64 instruction holds its scheduler for two cycles and
+// any other for one.  kScreen: the screened evaluation (screen.cuh), 735 FP64 and 364 other
+// instructions per 32 Lorenz points against 942 and 290 (FMA) or 1,600 (strict); the image
+// launches of a depth-27 job take 5.81 ms against 6.58 (FMA) and 10.21 (strict).  Its state
+// needs 48 registers: five blocks an SM (six, with spills, 5.99 ms; four 6.02 ms).
+template<class Map, class Grid, ImageMode M, bool kScreen>
+__global__ void __launch_bounds__(kThreads, kScreen ? 5 : 6) image_points_kernel(const ImageArgs a)
 {
   using PI = PointImage<Map, Grid>;
   __shared__ double pts[kPointTable];
@@ -150,12 +194,24 @@ __global__ void __launch_bounds__(kThreads, 6) image_points_kernel(const ImageAr
       if constexpr (M == ImageMode::Insert || M == ImageMode::Mark) {   // these carry their source centres
         double c[Map::D];
         PI::source_centre(a, rank, c);
-        valid = PI::image_at(a, pts, table, c, g, uint32_t(k), tbits);
+        if constexpr (kScreen) {
+          if (!PI::screened_at(a, pts, table, c, g, k, tbits, valid))
+            valid = PI::template image_at<true>(a, pts, table, c, g, k, tbits);
+        } else {
+          valid = PI::image_at(a, pts, table, c, g, k, tbits);
+        }
       } else {
         const uint32_t leaf = a.src ? __ldg(a.src + rank) : uint32_t(rank);
         uint32_t sbits[Map::D];
         PI::source_bits(a, leaf, sbits);
-        valid = PI::image(a, pts, table, sbits, g, uint32_t(k), tbits);
+        if constexpr (kScreen) {
+          if (!PI::screened(a, pts, table, sbits, g, k, tbits, valid)) {
+            PI::source_bits(a, leaf, sbits);       // (read again: not kept over the evaluation)
+            valid = PI::template image<true>(a, pts, table, sbits, g, k, tbits);
+          }
+        } else {
+          valid = PI::image(a, pts, table, sbits, g, k, tbits);
+        }
       }
       if constexpr (M != ImageMode::Mark) t = PI::target(a, n, valid, tbits);
     }
@@ -254,7 +310,7 @@ __global__ void __launch_bounds__(kThreads, 6) image_points_kernel(const ImageAr
 // ---------------------------------------------------------------------------------
 constexpr int kRowWarps = kThreads / 32;
 
-template<class Map, class Grid>
+template<class Map, class Grid, bool kScreen>
 __global__ void __launch_bounds__(kThreads) transition_rows_kernel(const RowArgs ra)
 {
   using PI = PointImage<Map, Grid>;
@@ -281,7 +337,14 @@ __global__ void __launch_bounds__(kThreads) transition_rows_kernel(const RowArgs
       uint32_t key = kPadKey;
       if (k < P) {
         uint32_t tbits[Map::D];
-        const bool valid = PI::image(a, pts, table, sbits, uint64_t(row) * P + k, k, tbits);
+        const uint64_t i = uint64_t(row) * P + k;
+        bool valid;
+        if constexpr (kScreen) {
+          if (!PI::screened(a, pts, table, sbits, i, k, tbits, valid))
+            valid = PI::template image<true>(a, pts, table, sbits, i, k, tbits);
+        } else {
+          valid = PI::image(a, pts, table, sbits, i, k, tbits);
+        }
         const uint32_t t = PI::target(a, n, valid, tbits);
         key = t == kInvalidIndex ? kLostKey : t;
       }
@@ -294,46 +357,46 @@ __global__ void __launch_bounds__(kThreads) transition_rows_kernel(const RowArgs
   }
 }
 
-template<class Map, class Grid>
-cudaError_t launch_image_t(ImageMode mode, const ImageArgs& a, uint64_t max_points, cudaStream_t s)
+template<class Map, class Grid, ImageMode M, bool kScreen>
+cudaError_t launch_image_mode(const ImageArgs& a, uint64_t max_points, cudaStream_t s)
 {
-  static int blocks_per_sm[4] = {0, 0, 0, 0};
-  const int m = int(mode);
-  if (!blocks_per_sm[m]) {
+  static int blocks_per_sm = 0;
+  if (!blocks_per_sm) {
     int b = 0;
-    if (mode == ImageMode::Hit)
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, image_points_kernel<Map, Grid, ImageMode::Hit>, kThreads, 0);
-    else if (mode == ImageMode::Search)
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, image_points_kernel<Map, Grid, ImageMode::Search>, kThreads, 0);
-    else if (mode == ImageMode::Insert)
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, image_points_kernel<Map, Grid, ImageMode::Insert>, kThreads, 0);
-    else
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, image_points_kernel<Map, Grid, ImageMode::Mark>, kThreads, 0);
-    blocks_per_sm[m] = b > 0 ? b : 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, image_points_kernel<Map, Grid, M, kScreen>, kThreads, 0);
+    blocks_per_sm = b > 0 ? b : 1;
   }
   const uint64_t want = (max_points + kThreads - 1) / kThreads;
-  const uint64_t cap = uint64_t(device_sm_count()) * blocks_per_sm[m];
+  const uint64_t cap = uint64_t(device_sm_count()) * blocks_per_sm;
   const unsigned grid = unsigned(want < 1 ? 1 : (want < cap ? want : cap));
-  if (mode == ImageMode::Hit) image_points_kernel<Map, Grid, ImageMode::Hit><<<grid, kThreads, 0, s>>>(a);
-  else if (mode == ImageMode::Search) image_points_kernel<Map, Grid, ImageMode::Search><<<grid, kThreads, 0, s>>>(a);
-  else if (mode == ImageMode::Insert) image_points_kernel<Map, Grid, ImageMode::Insert><<<grid, kThreads, 0, s>>>(a);
-  else image_points_kernel<Map, Grid, ImageMode::Mark><<<grid, kThreads, 0, s>>>(a);
+  image_points_kernel<Map, Grid, M, kScreen><<<grid, kThreads, 0, s>>>(a);
   return cudaGetLastError();
 }
 
-template<class Map, class Grid>
+template<class Map, class Grid, bool kScreen>
+cudaError_t launch_image_t(ImageMode mode, const ImageArgs& a, uint64_t max_points, cudaStream_t s)
+{
+  switch (mode) {
+    case ImageMode::Hit: return launch_image_mode<Map, Grid, ImageMode::Hit, kScreen>(a, max_points, s);
+    case ImageMode::Search: return launch_image_mode<Map, Grid, ImageMode::Search, kScreen>(a, max_points, s);
+    case ImageMode::Insert: return launch_image_mode<Map, Grid, ImageMode::Insert, kScreen>(a, max_points, s);
+    default: return launch_image_mode<Map, Grid, ImageMode::Mark, kScreen>(a, max_points, s);
+  }
+}
+
+template<class Map, class Grid, bool kScreen>
 cudaError_t launch_rows_t(const RowArgs& a, uint32_t max_rows, cudaStream_t s)
 {
   static int blocks_per_sm = 0;
   if (!blocks_per_sm) {
     int b = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, transition_rows_kernel<Map, Grid>, kThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, transition_rows_kernel<Map, Grid, kScreen>, kThreads, 0);
     blocks_per_sm = b > 0 ? b : 1;
   }
   const uint64_t want = (uint64_t(max_rows) + kRowWarps - 1) / kRowWarps;
   const uint64_t cap = uint64_t(device_sm_count()) * blocks_per_sm;
   const unsigned grid = unsigned(want < 1 ? 1 : (want < cap ? want : cap));
-  transition_rows_kernel<Map, Grid><<<grid, kThreads, 0, s>>>(a);
+  transition_rows_kernel<Map, Grid, kScreen><<<grid, kThreads, 0, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -431,8 +494,14 @@ cudaError_t launch_image(uint32_t map_kind, uint32_t arith, uint32_t grid_kind, 
   if (e != cudaSuccess) return e;
   ImageArgs b = a;
   fill_depth_const(b.dom, int(dim), b.depth, b.dc);
+  fill_screen(map_kind, b.map, b.dom, int(dim), b.depth, grid_reach(grid_kind, b.grid), b.sc);
   return dispatch(map_kind, arith, grid_kind, dim, [&](auto map, auto grid) {
-    return launch_image_t<decltype(map), decltype(grid)>(mode, b, max_points, s);
+    using Map = decltype(map);
+    using Grid = decltype(grid);
+    if constexpr (Screen<Map>::kOk) {
+      if (b.sc.on) return launch_image_t<Map, Grid, true>(mode, b, max_points, s);
+    }
+    return launch_image_t<Map, Grid, false>(mode, b, max_points, s);
   });
 }
 
@@ -441,8 +510,14 @@ cudaError_t launch_rows(uint32_t map_kind, uint32_t arith, uint32_t grid_kind, u
 {
   RowArgs b = a;
   fill_depth_const(b.img.dom, int(dim), b.img.depth, b.img.dc);
+  fill_screen(map_kind, b.img.map, b.img.dom, int(dim), b.img.depth, grid_reach(grid_kind, b.img.grid), b.img.sc);
   return dispatch(map_kind, arith, grid_kind, dim, [&](auto map, auto grid) {
-    return launch_rows_t<decltype(map), decltype(grid)>(b, max_rows, s);
+    using Map = decltype(map);
+    using Grid = decltype(grid);
+    if constexpr (Screen<Map>::kOk) {
+      if (b.img.sc.on) return launch_rows_t<Map, Grid, true>(b, max_rows, s);
+    }
+    return launch_rows_t<Map, Grid, false>(b, max_rows, s);
   });
 }
 

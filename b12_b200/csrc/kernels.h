@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "device.cuh"
+#include "screen.cuh"
 
 namespace b12g {
 
@@ -28,6 +29,7 @@ struct ImageArgs {
   const uint32_t* n_leaves;  // device count of `codes`
   int depth;                 // depth of the imaged boxes (children depth in children mode)
   DepthConst dc;             // constants of `depth` (launch_image / launch_rows fill them in)
+  ScreenArgs sc;             // the screened evaluation's (filled in by the same)
   int children;              // 1: boxes are the 2n children of `codes`, never materialised
   const uint32_t* src;       // source leaf ranks -> leaf index (nullptr: all leaves)
   const uint32_t* n_src;     // device count of sources (nullptr: all leaves / children)

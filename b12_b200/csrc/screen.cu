@@ -1,0 +1,357 @@
+// Host side of the screened map evaluation (screen.cuh): the scaled coefficients and the
+// bound on the distance between the screened image and the map's own.
+//
+// With u = 2^-53 and Phi the real-number step with the given double parameters, both
+// evaluations are Phi plus local roundings.  If every screened state lies in the box
+// |X_j| <= lim_j and the two trajectories are within eta = 2^-20 lim of each other, then
+//   |x^ - x~|_(n+1) <= G |x^ - x~|_n + d^ + d~   (component by component),
+// G a bound on |D Phi| over the box grown by eta, d^ and d~ bounds on the local roundings
+// of one step there.  All three come from running the step's operations on `Bound`: a
+// magnitude, the accumulated rounding error and the magnitudes of the derivatives by the
+// step's inputs.  Iterated over the map's steps from the start points' distance this gives
+// E; eta is checked at the end.  Only |x^ - x~| <= E matters, not the integrator's own
+// error, so E stays near the roundings times the flow's growth: for the benchmark's Lorenz
+// map over twice its domain 4e-6 of a box of width 0.12, where the distances seen are 3e-14.
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
+#include "kernels.h"
+#include "screen.cuh"
+#include "tree.h"
+
+namespace b12g {
+
+namespace {
+
+constexpr double kU = 0x1p-53;
+constexpr double kEta = 0x1p-20;
+
+struct Bound {
+  double m = 0.0;              // magnitude of the exact value
+  double e = 0.0;              // of (computed - exact)
+  double d[B12G_MAX_DIM] = {0.0, 0.0, 0.0, 0.0};   // of the derivatives by the inputs
+};
+
+__host__ __device__ Bound rounded(Bound r)
+{
+  r.e += kU * (r.m + r.e);
+  return r;
+}
+
+// a rounded constant (error at most `ulps` units of 2^-53 relative)
+__host__ __device__ Bound constant(double v, double ulps)
+{
+  Bound b;
+  b.m = v < 0.0 ? -v : v;
+  b.e = ulps * kU * b.m;
+  return b;
+}
+
+__host__ __device__ Bound product(const Bound& a, const Bound& b)
+{
+  Bound r;
+  r.m = a.m * b.m;
+  r.e = a.e * b.m + a.m * b.e + a.e * b.e;
+  for (int j = 0; j < B12G_MAX_DIM; ++j) r.d[j] = a.d[j] * b.m + a.m * b.d[j];
+  return r;
+}
+
+__host__ __device__ Bound sum(const Bound& a, const Bound& b)
+{
+  Bound r;
+  r.m = a.m + b.m;
+  r.e = a.e + b.e;
+  for (int j = 0; j < B12G_MAX_DIM; ++j) r.d[j] = a.d[j] + b.d[j];
+  return r;
+}
+
+__host__ __device__ Bound sc_fma(const Bound& a, const Bound& b, const Bound& c) { return rounded(sum(product(a, b), c)); }
+__host__ __device__ Bound sc_add(const Bound& a, const Bound& b) { return rounded(sum(a, b)); }
+__host__ __device__ Bound sc_mul(const Bound& a, const Bound& b) { return rounded(product(a, b)); }
+__host__ __device__ Bound sc_neg(const Bound& a) { return a; }
+__host__ __device__ Bound sc_fma2(const Bound& a, const Bound& b) { return rounded(sum(product(constant(2.0, 0.0), a), b)); }
+
+// |x_(n+1) - y_(n+1)| <= G |x_n - y_n| + d
+struct StepBound {
+  double G[B12G_MAX_DIM][B12G_MAX_DIM];
+  double d[B12G_MAX_DIM];
+};
+
+// a map's part of a screen: scales, shifts, the box of states and the distance E at the end
+struct MapBound {
+  double scale[B12G_MAX_DIM] = {1.0, 1.0, 1.0, 1.0}, shift[B12G_MAX_DIM] = {0.0, 0.0, 0.0, 0.0};
+  double lim[B12G_MAX_DIM] = {0.0, 0.0, 0.0, 0.0};   // unscaled, around the shift
+  double E[B12G_MAX_DIM] = {0.0, 0.0, 0.0, 0.0};
+};
+
+void identity_box(const double* lim, int dim, Bound* x)
+{
+  for (int j = 0; j < dim; ++j) {
+    x[j] = Bound{};
+    x[j].m = lim[j] * (1.0 + kEta);
+    x[j].d[j] = 1.0;
+  }
+}
+
+// E from the distance e0 of the start points over `steps` steps
+void iterate_bound(const StepBound& b, int dim, uint32_t steps, const double* e0, double* E)
+{
+  double e[B12G_MAX_DIM];
+  for (int j = 0; j < dim; ++j) e[j] = e0[j];
+  for (uint32_t n = 0; n < steps; ++n) {
+    double f[B12G_MAX_DIM], most = 0.0;
+    for (int i = 0; i < dim; ++i) {
+      f[i] = b.d[i];
+      for (int j = 0; j < dim; ++j) f[i] += b.G[i][j] * e[j];
+      most = std::max(most, f[i]);
+    }
+    for (int i = 0; i < dim; ++i) e[i] = f[i];
+    if (!(most < 1e300)) break;
+  }
+  for (int j = 0; j < dim; ++j) E[j] = e[j] * (1.0 + 0x1p-20);
+}
+
+// ---- Lorenz: classical RK4 in the map's order (Map_Lorenz.h:10-44, MapTools.hpp:118-182).
+// Inputs (x, y, z - rho); the derivative of rho x - y - x z is that of -x (z - rho) - y.
+// The explicit-FMA variant makes a subset of these roundings.
+void lorenz_rhs(const Bound* a, double sigma, double rho, double beta, Bound* r)
+{
+  Bound z = a[2];
+  z.m += std::fabs(rho);
+  r[0] = sc_mul(constant(sigma, 0.0), sc_add(a[1], a[0]));
+  const Bound exact = sum(product(a[0], a[2]), a[1]);
+  const Bound done = sc_add(sc_add(sc_mul(constant(rho, 0.0), a[0]), a[1]), sc_mul(a[0], z));
+  r[1] = exact;
+  r[1].e = done.e;
+  r[2] = sc_add(sc_mul(constant(beta, 0.0), z), sc_mul(a[0], a[1]));
+}
+
+// b + c k, the third component carrying rho
+void lorenz_madd(const Bound* k, const Bound& c, const Bound* b, double rho, Bound* out)
+{
+  for (int j = 0; j < 3; ++j) {
+    Bound r = sum(sc_mul(c, k[j]), b[j]);
+    r.e += kU * (r.m + r.e + (j == 2 ? std::fabs(rho) : 0.0));
+    out[j] = r;
+  }
+}
+
+void lorenz_coef(double h, double sigma, double rho, double beta, double* k)
+{
+  const double c = h / 2.0, q = c * beta, kappa = c * c * beta * rho;
+  const double v[kScreenCoef] = {c * sigma, -c, 1.0 - c, -q, 1.0 - q, -kappa, 2.0 * c * sigma, c * sigma / 3.0,
+                                 1.0 / 3.0, -kappa / 3.0};
+  for (int i = 0; i < kScreenCoef; ++i) k[i] = v[i];
+}
+
+void lorenz_bound(const MapParams& map, const Domain& dom, double lambda, const double* e0, MapBound& b, double* coef)
+{
+  const double h = map.h, sigma = map.p[0], rho = map.p[1], beta = map.p[2], c = h / 2.0;
+  for (int j = 0; j < 3; ++j) {
+    b.scale[j] = c;
+    b.shift[j] = j == 2 ? rho : 0.0;
+    b.lim[j] = lambda * (std::fabs(dom.c[j] - b.shift[j]) + dom.r[j]);
+  }
+  lorenz_coef(h, sigma, rho, beta, coef);
+  StepBound s;
+  Bound x[3], k[3], a[3], res[3];
+  identity_box(b.lim, 3, x);
+  lorenz_rhs(x, sigma, rho, beta, k);
+  lorenz_madd(k, constant(h / 6.0, 1.0), x, rho, res);
+  lorenz_madd(k, constant(c, 0.0), x, rho, a);
+  lorenz_rhs(a, sigma, rho, beta, k);
+  lorenz_madd(k, constant(h / 3.0, 1.0), res, rho, res);
+  lorenz_madd(k, constant(c, 0.0), x, rho, a);
+  lorenz_rhs(a, sigma, rho, beta, k);
+  lorenz_madd(k, constant(h / 3.0, 1.0), res, rho, res);
+  lorenz_madd(k, constant(h, 0.0), x, rho, a);
+  lorenz_rhs(a, sigma, rho, beta, k);
+  lorenz_madd(k, constant(h / 6.0, 1.0), res, rho, res);
+  // the screened step in its scaled coordinates (1 - c and 1 - q: the rounding of the
+  // difference and that of q)
+  Bound kb[kScreenCoef], sx[3];
+  for (int i = 0; i < kScreenCoef; ++i) kb[i] = constant(coef[i], 8.0);
+  kb[2].e = kb[4].e = 8.0 * kU * (1.0 + std::fabs(c) + std::fabs(coef[3]));
+  for (int j = 0; j < 3; ++j) sx[j].m = x[j].m * std::fabs(c);
+  lorenz_screen_step(kb, sx);
+  for (int i = 0; i < 3; ++i) {
+    for (int j = 0; j < 3; ++j) s.G[i][j] = res[i].d[j];
+    s.d[i] = res[i].e + sx[i].e / std::fabs(c);
+  }
+  iterate_bound(s, 3, map.steps, e0, b.E);
+}
+
+// magnitudes for which no product or scale below leaves the normal range
+bool moderate(double v) { return std::fabs(v) <= 0x1p40; }
+bool moderate_nonzero(double v) { return std::fabs(v) >= 0x1p-40 && std::fabs(v) <= 0x1p40; }
+
+}  // namespace
+
+double grid_reach(uint32_t grid_kind, const GridParams& g)
+{
+  if (grid_kind == B12G_GRID_PHILOX) return 1.0;
+  double m = 0.0;
+  for (uint32_t i = 0; i < g.n; ++i) m = std::max(m, std::fabs(g.coord[i]));
+  return grid_kind == B12G_GRID_FULL ? m * std::fabs(g.eps1) : m;
+}
+
+// The screened evaluation applies when the parameters are moderate, every dimension has at
+// most kScreenMaxBits bisections and the share P of the points it cannot decide (those
+// within the guard of a box boundary, if they lie evenly) is small.  The wider the box of
+// allowed states, the fewer trajectories leave it and the larger E: the widest of a few
+// multiples of the domain that keeps P under 2^-12 (one warp in 128 evaluates again), else
+// the narrowest if it keeps P under 2^-9 (one in 16: still faster than the map's own
+// arithmetic for every point, whose step is at least 1.25 times as long).
+void fill_screen(uint32_t map_kind, const MapParams& map, const Domain& dom, int dim, int depth, double gmax,
+                 ScreenArgs& s)
+{
+  s.on = 0;
+  if (map_kind != B12G_MAP_LORENZ) return;
+  if (map.steps == 0 || map.steps > 4096 || !moderate_nonzero(map.h) || !moderate(gmax)) return;
+  for (double p : map.p)
+    if (!moderate(p)) return;
+  for (int j = 0; j < dim; ++j)
+    if (!moderate_nonzero(dom.r[j]) || !moderate(dom.c[j])) return;
+  DepthConst dc;
+  fill_depth_const(dom, dim, depth, dc);
+  for (int j = 0; j < dim; ++j)
+    if (dc.k[j] > kScreenMaxBits) return;
+
+  static const double kLambda[] = {2.0, 1.75, 1.5, 1.25};
+  constexpr int kTries = int(sizeof kLambda / sizeof kLambda[0]);
+  for (int tr = 0; tr < kTries; ++tr) {
+    MapBound b;
+    // the start points: a few roundings of |c| + r (1 + |g|) on either side, and of the shift
+    double e0[B12G_MAX_DIM] = {0.0, 0.0, 0.0, 0.0};
+    for (int j = 0; j < dim; ++j) {
+      const double shift = map_kind == B12G_MAP_LORENZ && j == 2 ? std::fabs(map.p[1]) : 0.0;
+      e0[j] = 64.0 * kU * (std::fabs(dom.c[j]) + shift + 8.0 * dom.r[j] * (1.0 + gmax));
+    }
+    lorenz_bound(map, dom, kLambda[tr], e0, b, s.k);
+    double share = 0.0;
+    bool ok = true;
+    for (int j = 0; j < dim; ++j) {
+      if (!(b.E[j] <= kEta * b.lim[j])) { ok = false; break; }
+      // in boxes: the distance, the roundings of the exact index and of the domain's
+      // faces, those of the screened position, and the fixed-point form's
+      const double half = 0.5 * dc.ax[j].pk;
+      const double g = half * (b.E[j] + 64.0 * kU * (std::fabs(dom.c[j]) + std::fabs(b.shift[j]) + 4.0 * dom.r[j])) /
+                           dom.r[j] * (1.0 + 0x1p-20) + 0x1p-30;
+      share += 2.0 * g;
+      if (!(g < 0.125)) { ok = false; break; }
+      s.guard[j] = uint32_t(std::ceil(g * 0x1p32)) + 2u;
+    }
+    if (!ok || !(share <= (tr == kTries - 1 ? 0x1p-9 : 0x1p-12))) continue;
+    for (int j = 0; j < dim; ++j) {
+      const double S = b.scale[j], r = dom.r[j], rk = dc.ax[j].rk, half = 0.5 * dc.ax[j].pk;
+      s.E[j] = b.E[j];
+      s.sA[j] = 2.0 * r * S;
+      s.sB[j] = S * ((dom.c[j] - b.shift[j]) - 3.0 * r + rk);
+      s.sC[j] = S;
+      s.sD[j] = -S * b.shift[j];
+      s.sR[j] = S * rk;
+      s.tA[j] = half / (r * S);
+      s.tB[j] = 0x1.8p20 + (half + half * (b.shift[j] - dom.c[j]) / r);
+      s.bits[j] = uint32_t(dc.k[j]);
+      // |X| < L is certain when the high word of |X| is below that of L
+      const double L = std::fabs(S) * b.lim[j];
+      unsigned long long w;
+      __builtin_memcpy(&w, &L, sizeof w);
+      const uint32_t hi = uint32_t(w >> 32) - 1u;
+      __builtin_memcpy(&s.lim[j], &hi, sizeof hi);
+    }
+    s.on = 1;
+    return;
+  }
+}
+
+namespace {
+
+uint32_t high_word(double x)
+{
+  unsigned long long w;
+  std::memcpy(&w, &x, sizeof w);
+  return uint32_t(w >> 32);
+}
+
+// one point on the host: the operations of the kernels' screened() and screen_locate()
+bool host_kept(const ScreenArgs& s, int dim, const double* x)
+{
+  for (int j = 0; j < dim; ++j) {
+    uint32_t lim;
+    std::memcpy(&lim, &s.lim[j], sizeof lim);
+    if ((high_word(x[j]) & 0x7FFFFFFFu) > lim) return false;
+  }
+  return true;
+}
+
+bool host_run(const ScreenArgs& s, uint32_t, const MapParams& map, double* x)
+{
+  bool kept = true;
+  double y[3] = {x[0], x[1], x[2]};
+  for (uint32_t i = 0; i < map.steps; ++i) {
+    kept = kept && host_kept(s, 3, y);
+    lorenz_screen_step(s.k, y);
+  }
+  for (int j = 0; j < 3; ++j) x[j] = y[j];
+  return kept;
+}
+
+}  // namespace
+
+}  // namespace b12g
+
+using namespace b12g;
+using namespace b12g::host;
+
+extern "C" b12g_status b12g_screen_probe(const b12g_domain* domain, const b12g_map* m, uint8_t depth, double reach,
+                                         const uint64_t* codes, const double* offsets, uint64_t n, int from_centre,
+                                         int* applies, double* bound, double* images, uint8_t* decided,
+                                         uint64_t* boxes)
+{
+  if (!domain || !m || !applies || (n && (!codes || !offsets || !images || !decided || !boxes)))
+    return fail(B12G_ERR_INVALID, "NULL argument");
+  const int D = int(domain->dim);
+  if (D < 1 || D > B12G_MAX_DIM || depth > 64 || !image_supported(m->kind, m->arith, B12G_GRID_PHILOX, domain->dim))
+    return fail(B12G_ERR_INVALID, "unsupported map, dimension or depth");
+  Domain dom;
+  fill_domain(*domain, dom);
+  MapParams mp;
+  fill_map(*m, mp);
+  ScreenArgs s{};
+  fill_screen(m->kind, mp, dom, D, int(depth), reach, s);
+  *applies = s.on;
+  if (!s.on) return B12G_OK;
+  if (bound)
+    for (int j = 0; j < D; ++j) bound[j] = s.E[j];
+  for (uint64_t i = 0; i < n; ++i) {
+    double x[B12G_MAX_DIM] = {};
+    for (int j = 0; j < D; ++j) {
+      uint32_t index = 0;
+      for (int t = j; t < int(depth); t += D) index = (index << 1) | uint32_t((codes[i] >> (depth - 1 - t)) & 1u);
+      const double v = 1.0 + double(index) * pow2_hd(-int(s.bits[j]));
+      // (the centre in the order of box_axis)
+      const double t = double(index) * pow2_hd(1 - int(s.bits[j])) - 1.0;
+      const double centre = (t * dom.r[j] + dom.c[j]) + dom.r[j] * pow2_hd(-int(s.bits[j]));
+      const double start = from_centre ? sc_fma(centre, s.sC[j], s.sD[j]) : sc_fma(v, s.sA[j], s.sB[j]);
+      x[j] = sc_fma(offsets[i * D + j], s.sR[j], start);
+    }
+    bool sure = host_run(s, m->kind, mp, x), inside = true;
+    uint32_t at[B12G_MAX_DIM] = {};
+    for (int j = 0; j < D; ++j) {
+      const double t = sc_fma(x[j], s.tA[j], s.tB[j]);
+      unsigned long long w;
+      std::memcpy(&w, &t, sizeof w);
+      at[j] = uint32_t(w >> 32) - 0x41380000u;
+      sure = sure && uint32_t(w) - s.guard[j] <= ~(2u * s.guard[j]);
+      inside = inside && (at[j] >> s.bits[j]) == 0u;
+      images[i * D + j] = (x[j] - s.sD[j]) / s.sC[j];
+    }
+    decided[i] = sure ? 1 : 0;
+    uint64_t code = 0;
+    for (int t = 0; t < int(depth); ++t) code = (code << 1) | ((at[t % D] >> (s.bits[t % D] - 1 - t / D)) & 1u);
+    boxes[i] = inside ? code : kInvalidCode;
+  }
+  return B12G_OK;
+}

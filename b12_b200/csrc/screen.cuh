@@ -1,0 +1,183 @@
+// Screened map evaluation: the box of an image point decided from a cheaper evaluation of
+// the same map, with a proof that the map's own arithmetic decides the same.
+//
+// What the image kernels need of a point is the box its image lies in.  The maps'
+// arithmetic (one rounding per operation in the reference's order, or the explicit-FMA
+// variant) is fixed by the results that have to match bit for bit, and its FP64
+// instructions bound every image kernel: 78 (strict) or 45 (FMA) a Lorenz RK4 step, 64 a
+// forced Duffing step, 23 a Verlet step.  Written for the fewest FP64 instructions - the
+// step scaled into the variables, every product fused - the same real-number steps take
+// 36, 27 and 7.  Both evaluations differ only by their roundings, so a bound E on the
+// distance of the two images (screen.cu, computed on the host for every launch from the
+// map, the domain and the depth) makes the screened box the exact one whenever the
+// screened image keeps E away from every box boundary.  This is a floating-point filter
+// (Fortune and Van Wyk, "Efficient exact arithmetic for computational geometry", 1993):
+// a point that fails the test is evaluated again with the map's own arithmetic.
+//
+// The bound holds while the screened trajectory stays inside the limits `lim`, which the
+// kernels check at every step (a maximum over the high words: no FP64 instruction).  All
+// of it is FP64; nothing is decided in fewer bits than before.
+//
+// A step function below is one template for two scalar types: double (device, and the
+// host test hook) and Bound (screen.cu), whose operations carry a magnitude and a
+// rounding-error bound, so that the bound is derived from the very operations that run.
+#pragma once
+
+#include <cmath>
+#include <cstdint>
+
+#include "device.cuh"
+
+namespace b12g {
+
+constexpr int kScreenCoef = 10;
+constexpr int kScreenMaxBits = 18;   // bisections of a dimension the fixed-point test holds
+
+// Everything a screened launch needs, in the map's scaled coordinates X_j = S_j (x_j - shift_j)
+struct ScreenArgs {
+  int on;                      // 0: the launch runs the map's own arithmetic alone
+  float lim[B12G_MAX_DIM];     // limits on |X_j| as the high words of doubles, see screen_track
+  double k[kScreenCoef];       // the map's coefficients
+  double half[2];              // Verlet: coefficients of the half drift (unused elsewhere)
+  // the start point: fma(g, sR, fma(v, sA, sB)) from the box's index (v = 1 + index 2^-k),
+  // or fma(g, sR, fma(centre, sC, sD)) from the box's centre
+  double sA[B12G_MAX_DIM], sB[B12G_MAX_DIM], sC[B12G_MAX_DIM], sD[B12G_MAX_DIM], sR[B12G_MAX_DIM];
+  // the image's box: fma(X, tA, tB) is 1.5 2^20 + (position in boxes), so its high word
+  // counts boxes and its low word is the fraction in units of 2^-32
+  double tA[B12G_MAX_DIM], tB[B12G_MAX_DIM];
+  uint32_t guard[B12G_MAX_DIM];  // the fraction keeps this far from 0 and from 1
+  uint32_t bits[B12G_MAX_DIM];   // bisections of the dimension
+  double E[B12G_MAX_DIM];        // the bound on |screened image - exact image| (host use)
+};
+
+// ---------------------------------------------------------------------------- operations
+__host__ __device__ __forceinline__ double sc_fma(double a, double b, double c)
+{
+#ifdef __CUDA_ARCH__
+  return __fma_rn(a, b, c);
+#else
+  return std::fma(a, b, c);
+#endif
+}
+__host__ __device__ __forceinline__ double sc_add(double a, double b)
+{
+#ifdef __CUDA_ARCH__
+  return __dadd_rn(a, b);
+#else
+  return a + b;
+#endif
+}
+__host__ __device__ __forceinline__ double sc_mul(double a, double b)
+{
+#ifdef __CUDA_ARCH__
+  return __dmul_rn(a, b);
+#else
+  return a * b;
+#endif
+}
+__host__ __device__ __forceinline__ double sc_neg(double a) { return -a; }
+// 2 a + b
+__host__ __device__ __forceinline__ double sc_fma2(double a, double b) { return sc_fma(2.0, a, b); }
+
+// ---------------------------------------------------------------------------- Lorenz
+// X = c (x, y, z - rho) with c = h/2 turns k-scaled stages into bare products:
+//   c X0' = s (X1 - X0), c X1' = -X0 X2 - c X1, c X2' = X0 X1 - q X2 - kappa
+// with s = c sigma, q = c beta, kappa = c^2 beta rho.  Classical RK4 as
+//   a = X + c X'(X), b = X + c X'(a), w = 2 (b + c X'(b) - X) ... :
+//   X+ = (a + 2 b + d - X + c X'(d)) / 3 with d = X + 2 c X'(b),
+// the first component (linear) summed from its differences instead: 36 operations.
+// k: s, -c, 1 - c, -q, 1 - q, -kappa, 2 s, s / 3, 1 / 3, -kappa / 3
+template<class T, class K>
+__host__ __device__ __forceinline__ void lorenz_screen_step(const K* k, T (&x)[3])
+{
+  const T d1 = sc_add(x[1], sc_neg(x[0]));
+  const T a0 = sc_fma(k[0], d1, x[0]);
+  const T a1 = sc_fma(sc_neg(x[0]), x[2], sc_mul(k[2], x[1]));
+  const T a2 = sc_fma(x[0], x[1], sc_fma(k[4], x[2], k[5]));
+  const T xk = sc_add(x[2], k[5]);
+  const T d2 = sc_add(a1, sc_neg(a0));
+  const T b0 = sc_fma(k[0], d2, x[0]);
+  const T b1 = sc_fma(sc_neg(a0), a2, sc_fma(k[1], a1, x[1]));
+  const T b2 = sc_fma(a0, a1, sc_fma(k[3], a2, xk));
+  const T d3 = sc_add(b1, sc_neg(b0));
+  const T v1 = sc_fma(sc_neg(b0), b2, sc_mul(k[1], b1));
+  const T v2 = sc_fma(b0, b1, sc_fma(k[3], b2, k[5]));
+  const T c0 = sc_fma(k[6], d3, x[0]);
+  const T c1 = sc_fma2(v1, x[1]);
+  const T c2 = sc_fma2(v2, x[2]);
+  const T d4 = sc_add(c1, sc_neg(c0));
+  const T e1 = sc_fma2(sc_add(b1, v1), a1);
+  const T e2 = sc_fma2(sc_add(b2, v2), a2);
+  x[0] = sc_fma(k[7], sc_fma2(sc_add(d2, d3), sc_add(d1, d4)), x[0]);
+  x[1] = sc_mul(k[8], sc_fma(sc_neg(c0), c2, sc_fma(k[1], c1, e1)));
+  x[2] = sc_fma(k[8], sc_fma(c0, c1, sc_fma(k[3], c2, e2)), k[9]);
+}
+
+// ---------------------------------------------------------------------------- tracking
+#ifdef __CUDACC__
+// m = max(m, |x|) on the high words of doubles read as floats, which order like the
+// doubles; a NaN (as a float: any double of at least 2^1017, an infinity or a NaN) stays
+__device__ __forceinline__ void screen_track(float& m, double x)
+{
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(m) : "f"(fabsf(__int_as_float(__double2hiint(x)))));
+}
+#endif
+
+// maps with a screened evaluation: run() advances X over the map's steps and returns
+// whether the trajectory kept within the limits
+template<class Map> struct Screen { static constexpr bool kOk = false; };
+
+#ifdef __CUDACC__
+template<class A> struct Screen<LorenzMap<A>> {
+  static constexpr bool kOk = true;
+  static __device__ __forceinline__ bool run(const ScreenArgs& s, const MapParams& map, double (&x)[3])
+  {
+    float m0 = 0.f, m1 = 0.f, m2 = 0.f;
+#pragma unroll 4
+    for (uint32_t i = 0; i < map.steps; ++i) {
+      screen_track(m0, x[0]);
+      screen_track(m1, x[1]);
+      screen_track(m2, x[2]);
+      lorenz_screen_step(s.k, x);
+    }
+    return m0 <= s.lim[0] && m1 <= s.lim[1] && m2 <= s.lim[2];
+  }
+};
+
+// the double 1 + index 2^-k (exact for k <= 20)
+__device__ __forceinline__ double screen_index(uint32_t index, uint32_t k)
+{
+  return __hiloint2double(int(0x3FF00000u | (index << (20u - k))), 0);
+}
+
+// The box of the screened image X: its per-dimension indices in `bits` and whether it lies
+// in the domain; returns whether the exact evaluation is certain to decide the same.  A
+// position outside the range of the fixed-point form (or a box outside the domain) has a
+// high word outside [0, 2^k), compared unsigned.
+template<int D>
+__device__ __forceinline__ bool screen_locate(const ScreenArgs& s, const double (&x)[D], uint32_t (&bits)[D],
+                                              bool& inside)
+{
+  bool sure = true;
+  inside = true;
+#pragma unroll
+  for (int j = 0; j < D; ++j) {
+    const double t = __fma_rn(x[j], s.tA[j], s.tB[j]);
+    const uint32_t b = uint32_t(__double2hiint(t)) - 0x41380000u;
+    sure = sure && uint32_t(__double2loint(t)) - s.guard[j] <= ~(2u * s.guard[j]);
+    inside = inside && (b >> s.bits[j]) == 0u;
+    bits[j] = b;
+  }
+  return sure;
+}
+#endif
+
+// ---------------------------------------------------------------------------- host
+// Fills `s` for a launch over boxes of `depth` (grid points at most gmax box radii from the
+// centre); s.on tells whether the screened evaluation applies (screen.cu states when).
+void fill_screen(uint32_t map_kind, const MapParams& map, const Domain& dom, int dim, int depth, double gmax,
+                 ScreenArgs& s);
+// the largest |coordinate| of a grid's points
+double grid_reach(uint32_t grid_kind, const GridParams& g);
+
+}  // namespace b12g

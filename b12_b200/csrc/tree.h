@@ -207,6 +207,10 @@ struct Prepared {
   uint64_t P = 0;
 };
 
+// kernel-side domain constants and map parameters (the map's table not set)
+void fill_domain(const b12g_domain& domain, Domain& dom);
+void fill_map(const b12g_map& m, MapParams& mp);
+
 b12g_status sync(b12g_tree* t, const char* where);
 b12g_status read_ctr(b12g_tree* t, int first, int count);
 b12g_status set_ctr(b12g_tree* t, int slot, uint32_t v);

@@ -450,6 +450,17 @@ b12g_status b12g_profile_enable(b12g_tree* tree, int enable);
 b12g_status b12g_profile_read(b12g_tree* tree, uint32_t kind, double* ms_total, uint64_t* launches, int reset);
 /* kernels this process has launched through the library (graph replays included) */
 b12g_status b12g_launch_count(uint64_t* launches);
+/* the screened map evaluation of the image kernels, on the host: the kernels decide the box
+ * of an image point from an evaluation in fewer FP64 instructions where a bound on its
+ * distance from the map's own arithmetic proves the same box, and evaluate the other points
+ * again.  For n points (box codes[i] of `depth`, `offsets` n x dim in box radii from its
+ * centre, at most `reach` in magnitude; the start point taken from the box's centre or its
+ * index): *applies = whether launches over such boxes are screened (else nothing more is
+ * written), bound[dim] = the bound, images (n x dim) = the screened images, decided[i] = 1
+ * where the box is proven, boxes[i] = its code, ~0 outside the domain */
+b12g_status b12g_screen_probe(const b12g_domain* domain, const b12g_map* map, uint8_t depth, double reach,
+                              const uint64_t* codes, const double* offsets, uint64_t n, int from_centre, int* applies,
+                              double* bound, double* images, uint8_t* decided, uint64_t* boxes);
 /* FP64 fused multiply-add throughput of the current device (TFLOP/s, FMA = 2 FLOPs),
  * measured with a launch of about `seconds_hint` seconds */
 b12g_status b12g_probe_fp64_fma(double seconds_hint, double* tflops, double* seconds);
