@@ -788,29 +788,42 @@ __device__ __forceinline__ void LorenzMap<Fused>::rhs(const MapParams& m, const 
 // (MapTools.hpp:371-421): half q-step, full p-step, half q-step
 struct CoupledDuffingMap {
   static constexpr int D = 4;
-  static __device__ __forceinline__ void apply(const MapParams& m, const double* x, double* res)
+  // one step of (q0, q1, p0, p1)
+  static __device__ __forceinline__ void step(const MapParams& m, double (&x)[4])
   {
     double q0 = x[0], q1 = x[1], p0 = x[2], p1 = x[3];
-    auto step = [&]() {
-      q0 = __dadd_rn(q0, __dmul_rn(__dmul_rn(0.5, p0), m.h));
-      q1 = __dadd_rn(q1, __dmul_rn(__dmul_rn(0.5, p1), m.h));
-      const double f0 = __dsub_rn(__dsub_rn(q0, __dmul_rn(__dmul_rn(q0, q0), q0)),
-                                  __dmul_rn(__dmul_rn(__dmul_rn(0.2, q0), q1), q1));
-      const double f1 = __dsub_rn(__dmul_rn(-1.69, q1), __dmul_rn(__dmul_rn(__dmul_rn(0.2, q0), q0), q1));
-      p0 = __dadd_rn(p0, __dmul_rn(f0, m.h));
-      p1 = __dadd_rn(p1, __dmul_rn(f1, m.h));
-      q0 = __dadd_rn(q0, __dmul_rn(__dmul_rn(0.5, p0), m.h));
-      q1 = __dadd_rn(q1, __dmul_rn(__dmul_rn(0.5, p1), m.h));
-    };
+    q0 = __dadd_rn(q0, __dmul_rn(__dmul_rn(0.5, p0), m.h));
+    q1 = __dadd_rn(q1, __dmul_rn(__dmul_rn(0.5, p1), m.h));
+    const double f0 = __dsub_rn(__dsub_rn(q0, __dmul_rn(__dmul_rn(q0, q0), q0)),
+                                __dmul_rn(__dmul_rn(__dmul_rn(0.2, q0), q1), q1));
+    const double f1 = __dsub_rn(__dmul_rn(-1.69, q1), __dmul_rn(__dmul_rn(__dmul_rn(0.2, q0), q0), q1));
+    p0 = __dadd_rn(p0, __dmul_rn(f0, m.h));
+    p1 = __dadd_rn(p1, __dmul_rn(f1, m.h));
+    x[0] = __dadd_rn(q0, __dmul_rn(__dmul_rn(0.5, p0), m.h));
+    x[1] = __dadd_rn(q1, __dmul_rn(__dmul_rn(0.5, p1), m.h));
+    x[2] = p0;
+    x[3] = p1;
+  }
+  static __device__ __forceinline__ void apply(const MapParams& m, const double* x0, double* res)
+  {
+    double x[4] = {x0[0], x0[1], x0[2], x0[3]};
     if (m.steps == 10) {
       // the configured step count, without the loop's own instructions
 #pragma unroll
-      for (int s = 0; s < 10; ++s) step();
+      for (int s = 0; s < 10; ++s) step(m, x);
     } else {
 #pragma unroll 2
-      for (uint32_t s = 0; s < m.steps; ++s) step();
+      for (uint32_t s = 0; s < m.steps; ++s) step(m, x);
     }
-    res[0] = q0; res[1] = q1; res[2] = p0; res[3] = p1;
+    res[0] = x[0]; res[1] = x[1]; res[2] = x[2]; res[3] = x[3];
+  }
+  // the same in little code, for the few points that need it beside a screened evaluation
+  static __device__ __forceinline__ void apply_cold(const MapParams& m, const double* x0, double* res)
+  {
+    double x[4] = {x0[0], x0[1], x0[2], x0[3]};
+#pragma unroll 1
+    for (uint32_t s = 0; s < m.steps; ++s) step(m, x);
+    res[0] = x[0]; res[1] = x[1]; res[2] = x[2]; res[3] = x[3];
   }
 };
 

@@ -71,6 +71,12 @@ __host__ __device__ Bound sc_add(const Bound& a, const Bound& b) { return rounde
 __host__ __device__ Bound sc_mul(const Bound& a, const Bound& b) { return rounded(product(a, b)); }
 __host__ __device__ Bound sc_neg(const Bound& a) { return a; }
 __host__ __device__ Bound sc_fma2(const Bound& a, const Bound& b) { return rounded(sum(product(constant(2.0, 0.0), a), b)); }
+__host__ __device__ Bound sc_fma_half(const Bound& a, const Bound& b) { return rounded(sum(product(constant(0.5, 0.0), a), b)); }
+__host__ __device__ Bound sc_near(Bound a)
+{
+  a.e += 16.0 * kU * a.m;
+  return a;
+}
 
 // |x_(n+1) - y_(n+1)| <= G |x_n - y_n| + d
 struct StepBound {
@@ -182,6 +188,61 @@ void lorenz_bound(const MapParams& map, const Domain& dom, double lambda, const 
   iterate_bound(s, 3, map.steps, e0, b.E);
 }
 
+// ---- coupled Duffing: Stormer-Verlet in the map's order (MapTools.hpp:371-421).  The
+// limits hold for the positions at the kicks and the first momenta; the momenta then grow by
+// at most |h| max |force| a step, and the positions between the kicks differ from those at
+// them by half a drift.
+const double kDuffingStiff = 1.69, kDuffingCouple = 0.2;
+
+void cap(Bound& x, double m) { x.m = std::min(x.m, m); }
+
+void coupled_bound(const MapParams& map, const Domain& dom, double lambda, const double* e0, MapBound& b, double* coef)
+{
+  const double h = map.h, ah = std::fabs(h), root = std::sqrt(kDuffingCouple);
+  double q[2], grown[4];
+  for (int j = 0; j < 4; ++j) b.lim[j] = lambda * (std::fabs(dom.c[j]) + dom.r[j]);
+  for (int j = 0; j < 2; ++j) q[j] = b.lim[j] * (1.0 + kEta);
+  const double f[2] = {q[0] + q[0] * q[0] * q[0] + kDuffingCouple * q[0] * q[1] * q[1],
+                       kDuffingStiff * q[1] + kDuffingCouple * q[0] * q[0] * q[1]};
+  for (int j = 0; j < 2; ++j) {
+    grown[2 + j] = (b.lim[2 + j] + double(map.steps) * ah * f[j]) * (1.0 + kEta);
+    grown[j] = q[j] + 0.5 * ah * grown[2 + j] * (1.0 + kEta);
+    b.scale[j] = j == 0 ? h : root * h;
+    b.scale[2 + j] = j == 0 ? h * h : root * h * h;
+  }
+  coef[0] = h * h;
+  coef[1] = kDuffingCouple;
+  coef[2] = -(kDuffingStiff + kDuffingCouple) * h * h;
+  StepBound s;
+  Bound x[4];
+  identity_box(grown, 4, x);
+  auto half_drift = [&]() {
+    for (int j = 0; j < 2; ++j)
+      x[j] = sc_add(x[j], sc_mul(sc_mul(constant(0.5, 0.0), x[2 + j]), constant(h, 0.0)));
+  };
+  half_drift();
+  for (int j = 0; j < 2; ++j) cap(x[j], q[j]);
+  const Bound couple = constant(kDuffingCouple, 0.0);
+  const Bound f0 = sc_add(sc_add(x[0], sc_mul(sc_mul(x[0], x[0]), x[0])), sc_mul(sc_mul(sc_mul(couple, x[0]), x[1]), x[1]));
+  const Bound f1 = sc_add(sc_mul(constant(kDuffingStiff, 0.0), x[1]), sc_mul(sc_mul(sc_mul(couple, x[0]), x[0]), x[1]));
+  x[2] = sc_add(x[2], sc_mul(f0, constant(h, 0.0)));
+  x[3] = sc_add(x[3], sc_mul(f1, constant(h, 0.0)));
+  half_drift();
+  // the screened step with both its half drifts (joined, they make fewer roundings)
+  Bound sx[4], k[3];
+  for (int i = 0; i < 3; ++i) k[i] = constant(coef[i], i == 1 ? 0.0 : 8.0);
+  for (int j = 0; j < 4; ++j) sx[j].m = grown[j] * (1.0 + kEta) * std::fabs(b.scale[j]) * (1.0 + kEta);
+  duffing_screen_half_drift(sx);
+  for (int j = 0; j < 2; ++j) cap(sx[j], q[j] * std::fabs(b.scale[j]) * (1.0 + kEta));
+  duffing_screen_kick(k, sx);
+  duffing_screen_half_drift(sx);
+  for (int i = 0; i < 4; ++i) {
+    for (int j = 0; j < 4; ++j) s.G[i][j] = x[i].d[j];
+    s.d[i] = x[i].e + sx[i].e / std::fabs(b.scale[i]) * (1.0 + kEta);
+  }
+  iterate_bound(s, 4, map.steps, e0, b.E);
+}
+
 // magnitudes for which no product or scale below leaves the normal range
 bool moderate(double v) { return std::fabs(v) <= 0x1p40; }
 bool moderate_nonzero(double v) { return std::fabs(v) >= 0x1p-40 && std::fabs(v) <= 0x1p40; }
@@ -207,7 +268,7 @@ void fill_screen(uint32_t map_kind, const MapParams& map, const Domain& dom, int
                  ScreenArgs& s)
 {
   s.on = 0;
-  if (map_kind != B12G_MAP_LORENZ) return;
+  if (map_kind != B12G_MAP_LORENZ && map_kind != B12G_MAP_COUPLED_DUFFING) return;
   if (map.steps == 0 || map.steps > 4096 || !moderate_nonzero(map.h) || !moderate(gmax)) return;
   for (double p : map.p)
     if (!moderate(p)) return;
@@ -228,7 +289,8 @@ void fill_screen(uint32_t map_kind, const MapParams& map, const Domain& dom, int
       const double shift = map_kind == B12G_MAP_LORENZ && j == 2 ? std::fabs(map.p[1]) : 0.0;
       e0[j] = 64.0 * kU * (std::fabs(dom.c[j]) + shift + 8.0 * dom.r[j] * (1.0 + gmax));
     }
-    lorenz_bound(map, dom, kLambda[tr], e0, b, s.k);
+    if (map_kind == B12G_MAP_LORENZ) lorenz_bound(map, dom, kLambda[tr], e0, b, s.k);
+    else coupled_bound(map, dom, kLambda[tr], e0, b, s.k);
     double share = 0.0;
     bool ok = true;
     for (int j = 0; j < dim; ++j) {
@@ -276,9 +338,9 @@ uint32_t high_word(double x)
 }
 
 // one point on the host: the operations of the kernels' screened() and screen_locate()
-bool host_kept(const ScreenArgs& s, int dim, const double* x)
+bool host_kept(const ScreenArgs& s, int first, int end, const double* x)
 {
-  for (int j = 0; j < dim; ++j) {
+  for (int j = first; j < end; ++j) {
     uint32_t lim;
     std::memcpy(&lim, &s.lim[j], sizeof lim);
     if ((high_word(x[j]) & 0x7FFFFFFFu) > lim) return false;
@@ -286,15 +348,28 @@ bool host_kept(const ScreenArgs& s, int dim, const double* x)
   return true;
 }
 
-bool host_run(const ScreenArgs& s, uint32_t, const MapParams& map, double* x)
+bool host_run(const ScreenArgs& s, uint32_t kind, const MapParams& map, double* x)
 {
   bool kept = true;
-  double y[3] = {x[0], x[1], x[2]};
-  for (uint32_t i = 0; i < map.steps; ++i) {
-    kept = kept && host_kept(s, 3, y);
-    lorenz_screen_step(s.k, y);
+  if (kind == B12G_MAP_LORENZ) {
+    double y[3] = {x[0], x[1], x[2]};
+    for (uint32_t i = 0; i < map.steps; ++i) {
+      kept = kept && host_kept(s, 0, 3, y);
+      lorenz_screen_step(s.k, y);
+    }
+    std::copy(y, y + 3, x);
+  } else {
+    double y[4] = {x[0], x[1], x[2], x[3]};
+    kept = host_kept(s, 2, 4, y);
+    duffing_screen_half_drift(y);
+    for (uint32_t i = 0; i < map.steps; ++i) {
+      if (i) duffing_screen_drift(y);
+      kept = kept && host_kept(s, 0, 2, y);
+      duffing_screen_kick(s.k, y);
+    }
+    duffing_screen_half_drift(y);
+    std::copy(y, y + 4, x);
   }
-  for (int j = 0; j < 3; ++j) x[j] = y[j];
   return kept;
 }
 

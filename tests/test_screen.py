@@ -132,6 +132,30 @@ def test_lorenz_parameters(case):
     check(spec, depth, codes, off * reach, reach)
 
 
+def coupled(h=0.05, steps=10, center=(0.0,) * 4, radius=(2.0,) * 4):
+    return dict(dim=4, center=list(center), radius=list(radius),
+                map=dict(kind=O.MAP_COUPLED_DUFFING, steps=steps, h=h), grid=dict(kind=O.GRID_PHILOX, points=8))
+
+
+@pytest.mark.parametrize("depth", [0, 1, 3, 8, 16, 24, 30, 41])
+def test_coupled_duffing_depths(depth):
+    rng = np.random.default_rng([depth, 2])
+    codes, off = random_boxes(rng, 4, depth, 3000, 0.2)
+    on, share = check(coupled(), depth, codes, off)
+    # (points on the faces of coarse boxes stay on the planes q = 0 or p = 0 or meet them)
+    assert on and (share >= 0.99 or depth < 16)
+
+
+@pytest.mark.parametrize("case", range(16))
+def test_coupled_duffing_parameters(case):
+    rng = np.random.default_rng([case, 6])
+    spec = coupled(h=rng.choice([0.003, 0.05, -0.05, 0.11]), steps=int(rng.integers(1, 16)),
+                   center=rng.uniform(-1.0, 1.0, size=4), radius=np.exp(rng.uniform(np.log(0.2), np.log(6.0), size=4)))
+    codes, off = random_boxes(rng, 4, depth := int(rng.integers(0, 44)), 800)
+    reach = float(rng.choice([1.0, 2.0]))
+    check(spec, depth, codes, off * reach, reach)
+
+
 def test_points_beside_box_boundaries():
     """Images a few roundings, and a little more, beside a boundary."""
     spec = lorenz(h=2.0 ** -39, steps=1)     # the image is the point itself but for its last digits
