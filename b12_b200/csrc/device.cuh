@@ -859,6 +859,10 @@ struct ForcedDuffingMap {
       for (int j = 0; j < 2; ++j) { res[j] = Strict::madd(m.h6, k[j], res[j]); x[j] = res[j]; }
     }
   }
+  static __device__ __forceinline__ void apply_cold(const MapParams& m, const double* x0, double* res)
+  {
+    apply(m, x0, res);
+  }
 };
 
 // ForcedDuffingMap::apply for W points sharing the map parameters, interleaved so that one

@@ -243,6 +243,83 @@ void coupled_bound(const MapParams& map, const Domain& dom, double lambda, const
   iterate_bound(s, 4, map.steps, e0, b.E);
 }
 
+// ---- forced Duffing: classical RK4 of (x, v) in the map's order.  Over a period of 200
+// steps the component-wise bound, blind to the rotation of the flow, would grow by e^20;
+// here the distance is bounded in the norm |(w x, v)|_2.  With J the Jacobian of the right
+// hand side in that norm, mu >= the largest eigenvalue of its symmetric part and L >= |J|_2
+// over the stages, D Phi = I + h A + R with A the weighted mean of the stages' Jacobians,
+// |I + h A| <= sqrt(1 + 2 h mu + h^2 L^2) and |R| <= (hL)^2/2 + (hL)^3/6 + (hL)^4/24.  w is
+// the best of a few.
+void forced_rhs(const Bound* a, const double* p, Bound* r)
+{
+  r[0] = a[1];
+  r[1] = sc_add(sc_add(sc_add(sc_mul(constant(p[0], 0.0), a[1]), sc_mul(constant(p[1], 0.0), a[0])),
+                       sc_mul(constant(p[2], 0.0), sc_mul(sc_mul(a[0], a[0]), a[0]))),
+                constant(p[3], 1.0));                    // gamma cos: |cos| <= 1, one rounding
+}
+
+void forced_madd(const Bound* k, const Bound& c, const Bound* b, Bound* out)
+{
+  for (int j = 0; j < 2; ++j) out[j] = sc_add(sc_mul(c, k[j]), b[j]);
+}
+
+void forced_bound(const MapParams& map, const Domain& dom, double lambda, const double* e0, MapBound& b, double* coef)
+{
+  const double h = map.h, c = h / 2.0, delta = map.p[0], alpha = map.p[1], beta = map.p[2], root = std::sqrt(beta);
+  b.scale[0] = c * root;
+  b.scale[1] = c * c * root;
+  // (the velocity enters the bound little, so its limit is twice as wide)
+  for (int j = 0; j < 2; ++j) b.lim[j] = (j == 0 ? lambda : 2.0 * lambda) * (std::fabs(dom.c[j]) + dom.r[j]);
+  const double v[5] = {-c * c * alpha, -c * delta, 1.0 - c * delta, c * c * c * root * map.p[3], 1.0 / 3.0};
+  for (int i = 0; i < 5; ++i) coef[i] = v[i];
+  Bound x[2], k[2], a[2], res[2];
+  identity_box(b.lim, 2, x);
+  double sx = x[0].m;
+  forced_rhs(x, map.p, k);
+  forced_madd(k, constant(h / 6.0, 1.0), x, res);
+  forced_madd(k, constant(c, 0.0), x, a);
+  sx = std::max(sx, a[0].m);
+  forced_rhs(a, map.p, k);
+  forced_madd(k, constant(h / 3.0, 1.0), res, res);
+  forced_madd(k, constant(c, 0.0), x, a);
+  sx = std::max(sx, a[0].m);
+  forced_rhs(a, map.p, k);
+  forced_madd(k, constant(h / 3.0, 1.0), res, res);
+  forced_madd(k, constant(h, 0.0), x, a);
+  sx = std::max(sx, a[0].m);
+  forced_rhs(a, map.p, k);
+  forced_madd(k, constant(h / 6.0, 1.0), res, res);
+  // the screened step
+  Bound kb[5], sxv[2];
+  for (int i = 0; i < 5; ++i) kb[i] = constant(coef[i], 8.0);
+  kb[2].e = 8.0 * kU * (1.0 + std::fabs(c * delta));
+  for (int j = 0; j < 2; ++j) sxv[j].m = x[j].m * b.scale[j] * (1.0 + kEta);
+  const Bound f = sc_mul(kb[3], constant(1.0, 0.0));
+  forced_screen_step(kb, f, f, f, sxv);
+  double d[2];
+  for (int j = 0; j < 2; ++j) d[j] = res[j].e + sxv[j].e / b.scale[j] * (1.0 + kEta);
+  // -alpha - 3 beta x^2 over |x| <= sx lies between these
+  const double g0 = -alpha, g1 = -alpha - 3.0 * beta * sx * sx, gm = std::max(std::fabs(g0), std::fabs(g1));
+  double best = INFINITY, bw = 1.0;
+  for (int i = -8; i <= 24; ++i) {
+    const double w = std::exp2(0.25 * i);
+    const double q = 0.5 * std::max(std::fabs(w + g0 / w), std::fabs(w + g1 / w));
+    const double mu = 0.5 * (-delta + std::sqrt(delta * delta + 4.0 * q * q));
+    const double ad = std::fabs(delta);
+    const double L = std::sqrt(std::max(gm / w, w + ad) * std::max(w, gm / w + ad)), hl = h * L;
+    const double grow = std::sqrt(std::max(0.0, 1.0 + 2.0 * h * mu + hl * hl)) +
+                        hl * hl * (0.5 + hl * (1.0 / 6.0 + hl / 24.0));
+    if (grow < best) { best = grow; bw = w; }
+  }
+  best *= 1.0 + 0x1p-40;
+  const double step = std::hypot(bw * d[0], d[1]);
+  double e = std::hypot(bw * e0[0], e0[1]);
+  for (uint32_t n = 0; n < map.steps && e < 1e300; ++n) e = best * e + step;
+  e *= 1.0 + 0x1p-20;
+  b.E[0] = e / bw;
+  b.E[1] = e;
+}
+
 // magnitudes for which no product or scale below leaves the normal range
 bool moderate(double v) { return std::fabs(v) <= 0x1p40; }
 bool moderate_nonzero(double v) { return std::fabs(v) >= 0x1p-40 && std::fabs(v) <= 0x1p40; }
@@ -268,18 +345,19 @@ void fill_screen(uint32_t map_kind, const MapParams& map, const Domain& dom, int
                  ScreenArgs& s)
 {
   s.on = 0;
-  if (map_kind != B12G_MAP_LORENZ && map_kind != B12G_MAP_COUPLED_DUFFING) return;
+  if (map_kind == B12G_MAP_HENON) return;      // five operations: nothing to save
   if (map.steps == 0 || map.steps > 4096 || !moderate_nonzero(map.h) || !moderate(gmax)) return;
   for (double p : map.p)
     if (!moderate(p)) return;
   for (int j = 0; j < dim; ++j)
     if (!moderate_nonzero(dom.r[j]) || !moderate(dom.c[j])) return;
+  if (map_kind == B12G_MAP_FORCED_DUFFING && !(map.h > 0.0 && map.p[2] > 0.0 && moderate_nonzero(map.p[2]))) return;
   DepthConst dc;
   fill_depth_const(dom, dim, depth, dc);
   for (int j = 0; j < dim; ++j)
     if (dc.k[j] > kScreenMaxBits) return;
 
-  static const double kLambda[] = {2.0, 1.75, 1.5, 1.25};
+  static const double kLambda[] = {2.0, 1.75, 1.5, 1.25, 1.1, 1.0};
   constexpr int kTries = int(sizeof kLambda / sizeof kLambda[0]);
   for (int tr = 0; tr < kTries; ++tr) {
     MapBound b;
@@ -290,6 +368,7 @@ void fill_screen(uint32_t map_kind, const MapParams& map, const Domain& dom, int
       e0[j] = 64.0 * kU * (std::fabs(dom.c[j]) + shift + 8.0 * dom.r[j] * (1.0 + gmax));
     }
     if (map_kind == B12G_MAP_LORENZ) lorenz_bound(map, dom, kLambda[tr], e0, b, s.k);
+    else if (map_kind == B12G_MAP_FORCED_DUFFING) forced_bound(map, dom, kLambda[tr], e0, b, s.k);
     else coupled_bound(map, dom, kLambda[tr], e0, b, s.k);
     double share = 0.0;
     bool ok = true;
@@ -358,6 +437,16 @@ bool host_run(const ScreenArgs& s, uint32_t kind, const MapParams& map, double* 
       lorenz_screen_step(s.k, y);
     }
     std::copy(y, y + 3, x);
+  } else if (kind == B12G_MAP_FORCED_DUFFING) {
+    double y[2] = {x[0], x[1]};
+    const auto force = [&](uint32_t j) {      // the kernels read the cosines from a table made like this
+      return s.k[3] * std::cos(double(j) * (map.h * double(map.steps) / double(2 * map.steps)));
+    };
+    for (uint32_t i = 0; i < map.steps; ++i) {
+      kept = kept && host_kept(s, 0, 2, y);
+      forced_screen_step(s.k, force(2 * i), force(2 * i + 1), force(2 * i + 2), y);
+    }
+    std::copy(y, y + 2, x);
   } else {
     double y[4] = {x[0], x[1], x[2], x[3]};
     kept = host_kept(s, 2, 4, y);

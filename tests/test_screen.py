@@ -156,6 +156,39 @@ def test_coupled_duffing_parameters(case):
     check(spec, depth, codes, off * reach, reach)
 
 
+def forced(steps=200, p=(0.25, -1.0, 1.0, 0.3), center=(0.0, 0.0), radius=(2.0, 2.0)):
+    return dict(dim=2, center=list(center), radius=list(radius),
+                map=dict(kind=O.MAP_FORCED_DUFFING, steps=steps, h=O.FORCED_PERIOD / steps, p=list(p)),
+                grid=dict(kind=O.GRID_INNER, n=4))
+
+
+@pytest.mark.parametrize("depth", [0, 1, 6, 14, 19, 22, 26, 31])
+def test_forced_duffing_depths(depth):
+    rng = np.random.default_rng([depth, 4])
+    spec = forced()
+    codes, off = random_boxes(rng, 2, depth, 2000)
+    on, _ = check(spec, depth, codes, off)
+    assert on == (depth <= 26)       # 200 steps: the bound passes a sixteenth of the warps' budget at 14 bisections
+    if not on:
+        return
+    x = trajectory_points(spec, (0.5, 0.1), 500, 50)
+    codes = box_codes(spec, x, depth)
+    _, off = random_boxes(rng, 2, depth, len(codes))
+    on, share = check(spec, depth, codes, off)
+    assert on and (share >= 0.99 or depth < 14)
+
+
+@pytest.mark.parametrize("case", range(16))
+def test_forced_duffing_parameters(case):
+    rng = np.random.default_rng([case, 8])
+    p = (rng.uniform(-0.1, 0.6), rng.uniform(-1.5, 1.5), rng.uniform(0.1, 2.0), rng.uniform(-0.6, 0.6))
+    spec = forced(steps=int(rng.choice([40, 100, 200, 333])), p=p, center=rng.uniform(-0.5, 0.5, size=2),
+                  radius=np.exp(rng.uniform(np.log(0.3), np.log(3.0), size=2)))
+    depth = int(rng.integers(0, 34))
+    codes, off = random_boxes(rng, 2, depth, 600)
+    check(spec, depth, codes, off)
+
+
 def test_points_beside_box_boundaries():
     """Images a few roundings, and a little more, beside a boundary."""
     spec = lorenz(h=2.0 ** -39, steps=1)     # the image is the point itself but for its last digits
@@ -177,3 +210,5 @@ def test_screening_is_left_out_where_it_cannot_prove():
     assert not probe(lorenz(h=0.0), 27, *from_zero, 1.0, 0)[0]
     assert not probe(lorenz(sigma=float("nan")), 27, *from_zero, 1.0, 0)[0]
     assert not probe(lorenz(steps=0), 27, *from_zero, 1.0, 0)[0]
+    assert not probe(forced(p=(0.25, -1.0, -1.0, 0.3)), 16, np.zeros(1, np.uint64), np.zeros((1, 2)), 1.0, 0)[0]
+    assert not probe(forced(p=(0.25, -1.0, 0.0, 0.3)), 16, np.zeros(1, np.uint64), np.zeros((1, 2)), 1.0, 0)[0]
