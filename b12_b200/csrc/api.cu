@@ -220,7 +220,8 @@ b12g_status prepare(b12g_tree* t, const b12g_scheme* sc, Prepared& pr)
   a.hit_cap = uint32_t(std::min<size_t>(t->hit.n, 0xFFFFFFFFu));
   a.error = t->ctr.p + C_ERROR;
   a.cand_count = t->ctr.p + C_CAND;
-  a.work = reinterpret_cast<unsigned long long*>(t->ctr.p + C_WORK);
+  a.work = t->ctr.p + C_WORK;
+  a.work_turn = &t->work_turn;
   return B12G_OK;
 }
 
@@ -1067,8 +1068,12 @@ b12g_status b12g_subdivision_run(b12g_tree* t, const b12g_scheme* sc, uint32_t s
       CK(cudaStreamBeginCapture(t->stream, cudaStreamCaptureModeThreadLocal));
       int cur = t->cur, ncur = t->ncur;
       cudaError_t err = cudaSuccess;
+      // both work-queue counters start empty at every replay, whose first launch takes the
+      // first of them
+      err = cudaMemsetAsync(t->ctr.p + C_WORK, 0, 2 * sizeof(uint32_t), t->stream);
+      t->work_turn = 0;
       // the lookup table starts clean at every replay; step s builds with tag s + 1
-      if (use_hash) err = cudaMemsetAsync(t->hash.p, 0, t->hash.n * sizeof(ulonglong2), t->stream);
+      if (use_hash && err == cudaSuccess) err = cudaMemsetAsync(t->hash.p, 0, t->hash.n * sizeof(ulonglong2), t->stream);
       for (uint32_t s = 0; s < steps && err == cudaSuccess; ++s) {
         const int o = 1 - cur, no = 1 - ncur;
         ImageArgs a = pr.a;
@@ -1130,6 +1135,7 @@ b12g_status b12g_subdivision_run(b12g_tree* t, const b12g_scheme* sc, uint32_t s
     ST(set_ctr(t, C_TGT, 0));
     CK(cudaGraphLaunch(t->sub_graph, t->stream));
     count_launches(t->sub_graph_kernels);
+    t->work_turn = steps & 1u;
     if (use_hash) t->hash_tag = steps;
     std::vector<uint32_t> hc(steps);
     CK(cudaMemcpyAsync(hc.data(), t->step_counts.p, steps * 4, cudaMemcpyDeviceToHost, t->stream));

@@ -141,7 +141,10 @@ struct PointImage {
 };
 
 constexpr uint32_t kPointTable = 2048;  // doubles of grid-point table per block (16 KB)
-constexpr int kChunkTrips = 4;          // points per lane in a chunk of the image kernel's work queue
+constexpr int kChunkTrips = 4;          // units (a point a lane) a warp takes at a time from the work queue
+constexpr int kFineUnits = 4;           // units a warp left in the queue when it takes single ones (1: a
+                                        // depth-22 forced Duffing job's image launches 1.64 ms, 4: 1.48, 8: 1.45,
+                                        // while the continuation's take 11.07, 11.13 and 11.47 ms)
 
 // fills `pts` with the P x D grid points when they fit (returns true), else with the
 // 1-D coordinates for the per-point path
@@ -179,6 +182,8 @@ __global__ void __launch_bounds__(kThreads, kScreen ? 5 : 6) image_points_kernel
   const uint32_t P32 = uint32_t(P);
   const uint64_t total = uint64_t(nboxes) * P;
   const int lane = threadIdx.x & 31;
+  // the queue of the next launch on the tree's stream starts empty
+  if (blockIdx.x == 0 && threadIdx.x == 0) *a.work_next = 0u;
   if (M == ImageMode::Hit && a.children && 2ull * n > a.hit_cap) {
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(a.error, 1u);
     return;
@@ -271,21 +276,30 @@ __global__ void __launch_bounds__(kThreads, kScreen ? 5 : 6) image_points_kernel
     }
   };
 
-  // A device work queue (a.work, zeroed by launch_image): every warp takes chunks of 32 x
-  // kChunkTrips consecutive points until none is left, so that warps that run ahead take
-  // more work and the SM stays full to the end (a static split leaves the slower warps
-  // alone at the end: 47 % of the warp slots were active on average, of 75 % possible).
-  constexpr uint64_t kChunk = 32ull * kChunkTrips;
-  const uint64_t chunks = (total + kChunk - 1) / kChunk;
+  // A device work queue: every warp takes the next points until none is left, so that warps
+  // that run ahead take more work and the SM stays full to the end (a static split leaves
+  // the slower warps alone at the end: 47 % of the warp slots were active on average, of
+  // 75 % possible).  The queue counts units of 32 points (of 2^shift times as many where
+  // that many units would not fit 32 bits); a warp takes kChunkTrips units at a time while
+  // at least kFineUnits units a warp are left, and single ones after that: a warp works
+  // through its units one after another, so in a small launch, and at the end of a large
+  // one, larger pieces would leave the others idle (the small steps of a forced Duffing job
+  // took 68 us with four points a lane, 25 us with one).
+  uint32_t shift = 0;
+  while (((total + 31) >> (5 + shift)) >= 0x40000000ull) ++shift;
+  const uint32_t units = uint32_t((total + (32ull << shift) - 1) >> (5 + shift));
+  const uint32_t fine = gridDim.x * (kThreads / 32) * kFineUnits;
+  const uint32_t coarse_end = units > fine ? units - fine : 0;
+  uint32_t c = 0;
   for (;;) {
-    unsigned long long c = 0;
-    if (lane == 0) c = atomicAdd(a.work, 1ull);
+    const uint32_t size = c < coarse_end ? uint32_t(kChunkTrips) : 1u;
+    if (lane == 0) c = atomicAdd(a.work, size);
     c = __shfl_sync(0xFFFFFFFFu, c, 0);
-    if (c >= chunks) break;
+    if (c >= units) break;
     // (sources and points per box both fit 32 bits: the rank and the point index do)
-    const uint64_t g = c * kChunk + uint64_t(lane);
+    const uint64_t g = (uint64_t(c) << (5 + shift)) + uint64_t(lane);
     uint32_t rank, k;
-    if (total <= 0xFFFFFFFFull - kChunk) {
+    if (total <= 0xFFFFFFFFull - 64ull * kChunkTrips) {
       rank = uint32_t(g) / P32;
       k = uint32_t(g) - rank * P32;
     } else {
@@ -293,7 +307,7 @@ __global__ void __launch_bounds__(kThreads, kScreen ? 5 : 6) image_points_kernel
       k = uint32_t(g - uint64_t(rank) * P);
     }
 #pragma unroll 1
-    for (int j = 0; j < kChunkTrips; ++j) {
+    for (uint32_t j = 0; j < (size << shift); ++j) {
       const uint64_t gj = g + 32ull * uint64_t(j);
       point(gj, rank, k, gj < total);
       k += 32;
@@ -489,19 +503,22 @@ bool image_supported(uint32_t map_kind, uint32_t arith, uint32_t grid_kind, uint
 cudaError_t launch_image(uint32_t map_kind, uint32_t arith, uint32_t grid_kind, uint32_t dim, ImageMode mode,
                          const ImageArgs& a, uint64_t max_points, cudaStream_t s)
 {
-  if (!a.work) return cudaErrorInvalidValue;     // the image kernel takes its points from a work queue
-  const cudaError_t e = cudaMemsetAsync(a.work, 0, sizeof(unsigned long long), s);   // the queue starts empty
-  if (e != cudaSuccess) return e;
+  if (!a.work || !a.work_turn) return cudaErrorInvalidValue;   // the image kernel takes its points from a work queue
   ImageArgs b = a;
+  b.work = a.work + (*a.work_turn & 1u);
+  b.work_next = a.work + ((*a.work_turn & 1u) ^ 1u);
   fill_depth_const(b.dom, int(dim), b.depth, b.dc);
   fill_screen(map_kind, b.map, b.dom, int(dim), b.depth, grid_reach(grid_kind, b.grid), b.sc);
   return dispatch(map_kind, arith, grid_kind, dim, [&](auto map, auto grid) {
     using Map = decltype(map);
     using Grid = decltype(grid);
+    cudaError_t e = cudaErrorInvalidValue;
     if constexpr (Screen<Map>::kOk) {
-      if (b.sc.on) return launch_image_t<Map, Grid, true>(mode, b, max_points, s);
+      if (b.sc.on) e = launch_image_t<Map, Grid, true>(mode, b, max_points, s);
     }
-    return launch_image_t<Map, Grid, false>(mode, b, max_points, s);
+    if (!Screen<Map>::kOk || !b.sc.on) e = launch_image_t<Map, Grid, false>(mode, b, max_points, s);
+    if (e == cudaSuccess) *a.work_turn ^= 1u;
+    return e;
   });
 }
 

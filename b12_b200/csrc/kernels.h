@@ -54,7 +54,13 @@ struct ImageArgs {
   int claim;                 // Insert mode: claim each new box in `hash` (a kept table,
                              // log2_use set), so every candidate is a distinct new box
   uint32_t* error;           // bit 0: capacity overflow
-  unsigned long long* work;  // the image kernel's work-queue counter (launch_image zeroes it)
+  // The image kernel's work queue: two counters that the launches on one stream take in
+  // turn, each emptying the other for the launch after it (a memset between the kernels of
+  // a subdivision step cost 6 us of the step).  launch_image takes `work`, the pair, and
+  // sets the launch's own counter, its partner and the turn of the next launch.
+  unsigned* work;
+  unsigned* work_next;
+  unsigned* work_turn;       // host word of the stream's owner
 };
 
 // Transition rows: warp per source box, up to kMaxRowPoints points.

@@ -102,7 +102,7 @@ enum : int {
   C_SYNC = 9,      // 3 words for the grid barrier
   C_NNEW = 12,
   C_TGT = 13,      // the stored image targets overflowed their buffer
-  C_WORK = 14,     // 2 words (8-byte aligned): the image kernel's work-queue counter
+  C_WORK = 14,     // 2 words: the image kernel's work-queue counters
   C_DEFER = 16,    // error bits of launches whose status is read with a later read-back
   C_COUNT = 18
 };
@@ -124,6 +124,7 @@ struct b12g_tree {
   Buf<uint8_t> flags[2];
   Buf<uint8_t> hit;
   Buf<uint32_t> ctr;
+  unsigned work_turn = 0;      // which of the work-queue counters the next image launch takes
   Buf<uint32_t> tiles_a, tiles_b;
   Buf<uint32_t> src, out, stage_col, stage_cnt, row_count, rowptr;
   Buf<uint64_t> cand, cand2;

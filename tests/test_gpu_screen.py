@@ -1,0 +1,108 @@
+"""GPU: the image kernels' screened evaluation and work queue against the oracle, on leaf
+sets and launch sizes of every kind (search results, matrices and hits, all exact)."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from test_screen import coupled, forced, lorenz
+
+pytestmark = pytest.mark.gpu
+
+
+def scheme(spec):
+    import b12_b200 as B
+    ms, gs = spec["map"], spec["grid"]
+    m = B.MapSpec(ms["kind"], steps=ms.get("steps", 1), h=ms.get("h", 0.0), p=tuple(ms.get("p", ())),
+                  arith=ms.get("fma", 0))
+    g = B.GridSpec(gs["kind"], n=gs.get("n", 1), points=gs.get("points", 1), seed=gs.get("seed", 0),
+                   eps=gs.get("eps", 0.0))
+    return B.Scheme(m, g)
+
+
+def trees(spec, codes, depth):
+    """A tree and an oracle holding the boxes `codes` of one depth."""
+    import b12_b200 as B
+    codes = np.unique(np.asarray(codes, dtype=np.uint64))
+    dep, flags = np.full(len(codes), depth, np.uint8), np.zeros(len(codes), np.uint8)
+    t = B.ImplicitBoxTree(spec["center"], spec["radius"])
+    t.load_leaves(codes, dep, flags)
+    o = O.Oracle(spec)
+    o.load(codes, dep, flags)
+    return t, o
+
+
+def covering(spec, depth, n, seed):
+    """Boxes that hold images of one another: the boxes hit from random boxes, twice over."""
+    rng = np.random.default_rng(seed)
+    o = O.Oracle(spec)
+    c, r = np.array(spec["center"]), np.array(spec["radius"])
+    x = c + r * rng.uniform(-0.6, 0.6, size=(n, spec["dim"]))
+    out = []
+    for p in x:
+        for _ in range(3):
+            code, inside = o.point_code64(p)
+            if inside:
+                out.append(code >> (64 - depth) if depth else 0)
+            p = o.map_apply(p)
+    return np.array(out, dtype=np.uint64)
+
+
+CASES = [
+    (lorenz(), [0, 1, 5, 18, 27, 36, 54, 55, 60]),
+    (lorenz(fma=1), [3, 22, 30, 57]),
+    (dict(lorenz(rho=24.0, steps=7), grid=dict(kind=O.GRID_FULL, n=4, eps=0.1)), [9, 25]),
+    (dict(lorenz(h=-0.01, steps=3), grid=dict(kind=O.GRID_PHILOX, points=37, seed=5)), [12, 24]),
+    (forced(), [0, 2, 15, 20, 26, 27, 36, 40]),
+    (dict(forced(p=(0.1, 0.5, 0.7, 0.2)), grid=dict(kind=O.GRID_FULL, n=5, eps=-0.05)), [17]),
+    (coupled(), [0, 4, 16, 24, 29, 40, 60]),
+    (dict(coupled(h=-0.03, steps=4), grid=dict(kind=O.GRID_INNER, n=3)), [13, 20]),
+]
+
+
+@pytest.mark.parametrize("case,depth", [(i, d) for i, (_, ds) in enumerate(CASES) for d in ds])
+def test_search_matrix_and_hits(case, depth):
+    import b12_b200 as B
+    spec = CASES[case][0]
+    t, o = trees(spec, covering(spec, depth, 150, [case, depth]), depth)
+    sc = scheme(spec)
+    assert np.array_equal(t.search_by_image(sc), o.search_by_image())
+    m = t.transition_matrix(sc, invalid_column=True)
+    rp, cols, vals, nc = o.transition_matrix(invalid=True)
+    got = m.to_host()
+    assert m.n_cols == nc and np.array_equal(got[0], rp) and np.array_equal(got[1], cols)
+    assert np.array_equal(got[2], vals)
+    assert t.set_flags_by_image(sc, B.HIT) == o.set_flags_by_image(1)
+    assert np.array_equal(t.leaves()[2], o.leaves()[2])
+    m.close()
+    t.close()
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 5, 63, 64, 65, 3551, 56830, 56832, 56833, 60001])
+def test_work_queue_sizes(n):
+    """Launches of less than a unit of 32 points up to those that start with larger pieces
+    (888 blocks of 8 warps, 4 units each: 56,832 boxes of 16 points), ragged ones between."""
+    spec = O.henon_spec()
+    rng = np.random.default_rng(n)
+    codes = np.sort(rng.choice(2 ** 18, size=n, replace=False)).astype(np.uint64)
+    t, o = trees(spec, codes, 18)
+    sc = scheme(spec)
+    want = o.search_by_image()
+    for _ in range(3):                   # the launches take the two queue counters in turn
+        assert np.array_equal(t.search_by_image(sc), want)
+    t.close()
+
+
+def test_queue_turns_through_graphs_and_single_launches():
+    """Fused runs (an odd and an even number of launches) between single launches."""
+    spec = O.henon_spec()
+    import b12_b200 as B
+    t = B.ImplicitBoxTree(spec["center"], spec["radius"])
+    sc = scheme(spec)
+    for steps in (7, 8, 7, 1, 8):
+        t.delete_depth(0)
+        o = O.Oracle(spec)
+        want, _ = o.subdivision(steps)
+        assert list(t.subdivision_run(sc, steps)) == list(want)
+        assert np.array_equal(t.search_by_image(sc), o.search_by_image())
+        assert t.set_flags_by_image(sc, B.HIT) == o.set_flags_by_image(1)
+    t.close()
