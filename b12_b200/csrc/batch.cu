@@ -112,7 +112,8 @@ template<> struct Multi<ForcedDuffingMap> {
 };
 
 // the image of child point (child c of the concatenated children, grid index k)
-template<class Map, class Grid, int W>
+// kCold: for the few points a screened launch could not decide
+template<class Map, class Grid, int W, bool kCold = false>
 struct BatchPoint {
   static constexpr int D = Map::D;
   // W points: child[w], k[w]; returns their children-level targets (global child index,
@@ -158,6 +159,9 @@ struct BatchPoint {
 #pragma unroll
         for (int w = 0; w < W; ++w) Map::apply(mp[w], x[w], y[w]);
       }
+    } else if constexpr (kCold) {
+#pragma unroll
+      for (int w = 0; w < W; ++w) Map::apply_cold(mp[w], x[w], y[w]);
     } else {
 #pragma unroll
       for (int w = 0; w < W; ++w) Map::apply(mp[w], x[w], y[w]);
@@ -261,6 +265,117 @@ __global__ void __launch_bounds__(512) batch_image_kernel(const BatchArgs a)
   }
 }
 
+
+// The same with the screened evaluation (screen.cuh), a point a thread, and the work queue of
+// the single-tree image kernel (units of 32 points; four at a time while many are left): a
+// step of few points then still fills the GPU.  A block's queue items of 8,192 points left
+// all but a few SMs idle in the small steps of served jobs.  16 Lorenz instances of depth 24
+// run in 24.7 ms against 31.1 (FMA) and 45.6 (strict); with five blocks an SM (48 registers,
+// spills) 24.9, with six 25.2.  The forced Duffing ticks of 48 served jobs: 5.4 ms against
+// 32.3 (the shape with four points a thread).
+constexpr uint32_t kScreenTrips = 4, kScreenFine = 4;
+
+template<class Map, class Grid>
+__global__ void __launch_bounds__(256, 4) batch_screen_kernel(const BatchArgs a)
+{
+  constexpr int D = Map::D;
+  __shared__ uint32_t off_s[kMaxInstances + 1];
+  __shared__ double pts[kBatchTable];
+  for (uint32_t i = threadIdx.x; i <= a.n_inst; i += blockDim.x) off_s[i] = a.off[i];
+  load_batch_points<Map, Grid>(a.grid, a.points, pts);
+  __syncthreads();
+  const uint32_t n = off_s[a.n_inst];
+  const uint64_t children = 2ull * n;
+  if (children > a.hit_cap) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(a.error, 1u);
+    return;
+  }
+  const uint32_t P = uint32_t(a.points);
+  const uint64_t total = children * P;
+  const int lane = threadIdx.x & 31;
+  const bool uni = a.inst_depth == nullptr;
+  // (children < 2^32 and P <= 128: fewer than 2^34 units; two units a step of the counter
+  // and more keep it in 32 bits)
+  uint32_t shift = 0;
+  while (((total + 31) >> (5 + shift)) >= 0x40000000ull) ++shift;
+  const uint32_t units = uint32_t((total + (32ull << shift) - 1) >> (5 + shift));
+  const uint32_t fine = gridDim.x * (256 / 32) * kScreenFine;
+  const uint32_t coarse_end = units > fine ? units - fine : 0;
+  uint32_t c = 0;
+  for (;;) {
+    const uint32_t size = c < coarse_end ? kScreenTrips : 1u;
+    if (lane == 0) c = atomicAdd(a.queue, size);
+    c = __shfl_sync(0xFFFFFFFFu, c, 0);
+    if (c >= units) break;
+    const uint64_t g = (uint64_t(c) << (5 + shift)) + uint64_t(lane);
+    uint32_t child, k;
+    if (total <= 0xFFFFFFFFull - 64ull * kScreenTrips) {
+      child = uint32_t(g) / P;
+      k = uint32_t(g) - child * P;
+    } else {
+      child = uint32_t(g / P);
+      k = uint32_t(g - uint64_t(child) * P);
+    }
+    uint32_t inst = find_instance(off_s, a.n_inst, child >> 1);
+#pragma unroll 1
+    for (uint32_t trip = 0; trip < (size << shift); ++trip) {
+      const bool active = g + 32ull * trip < total;
+      uint32_t t = kInvalidIndex;
+      if (active) {
+        const uint64_t code = (__ldg(a.codes + (child >> 1)) << 1) | (child & 1u);
+        const int depth = uni ? a.depth : int(__ldg(a.inst_depth + inst));
+        const ScreenRec* r = a.screen + inst;
+        const uint32_t kb = __ldg(&r->k);
+        uint32_t sb[D], tb[D];
+        split_code<D>(code, depth, sb);
+        double x[D], kk[kScreenCoef];
+        float lim[D];
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+          lim[j] = __ldg(&r->lim[j]);
+          x[j] = __fma_rn(pts[j * P + k], __ldg(&r->sR[j]),
+                          __fma_rn(screen_index(sb[j], (kb >> (8 * j)) & 0xFFu), a.sA[j], __ldg(&r->sB[j])));
+        }
+#pragma unroll
+        for (int i = 0; i < kScreenCoef; ++i) kk[i] = a.sk[i];
+#pragma unroll
+        for (int i = 0; i < Screen<Map>::kOwnCount; ++i) kk[Screen<Map>::own(i)] = __ldg(&r->own[i]);
+        bool sure = Screen<Map>::run(kk, lim, a.map, x) && __ldg(&r->on) != 0u, inside = true;
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+          const double p = __fma_rn(x[j], __ldg(&r->tA[j]), __ldg(&r->tB[j]));
+          const uint32_t b = uint32_t(__double2hiint(p)) - 0x41380000u, gd = __ldg(&r->guard[j]);
+          sure = sure && uint32_t(__double2loint(p)) - gd <= ~(2u * gd);
+          inside = inside && (b >> ((kb >> (8 * j)) & 0xFFu)) == 0u;
+          tb[j] = b;
+        }
+        if (!sure) {
+          const uint64_t cc[1] = {child};
+          const uint32_t ck[1] = {k}, ci[1] = {inst};
+          const bool ca[1] = {true};
+          uint32_t ct[1];
+          BatchPoint<Map, Grid, 1, true>::run(a, off_s, pts, cc, ck, ca, ct, ci);
+          t = ct[0];
+        } else if (!inside) {
+          t = kOutsideIndex;
+        } else {
+          const uint64_t tcode = join_code<D>(tb, depth);
+          const uint32_t p = hash_locate(a.hash, n, inst_key(inst, tcode >> 1));
+          if (p != kInvalidIndex) t = 2u * p + uint32_t(tcode & 1u);
+        }
+      }
+      const unsigned peers = __match_any_sync(0xFFFFFFFFu, t);
+      if (active && t < kOutsideIndex && lane == __ffs(peers) - 1) a.hit[t] = 1;
+      if (a.targets && active) {
+        const uint64_t base = __ldg(a.tgt_base + inst);
+        if (base != ~0ull) a.targets[base + (uint64_t(child) - 2ull * off_s[inst]) * P + k] = t;
+      }
+      k += 32;
+      while (k >= P) { k -= P; ++child; }
+      while (inst + 1 < a.n_inst && (child >> 1) >= off_s[inst + 1]) ++inst;
+    }
+  }
+}
 
 // survivors per instance (children with a hit), one block per instance
 __global__ void inst_count_kernel(const uint8_t* hit, const uint32_t* off, uint32_t* cnt, uint64_t hit_cap,
@@ -493,6 +608,13 @@ cudaError_t launch_batch_image(uint32_t map_kind, uint32_t arith, uint32_t grid_
   return batch_dispatch(map_kind, arith, grid_kind, [&](auto map, auto grid) -> cudaError_t {
     using Map = decltype(map);
     using Grid = decltype(grid);
+    if constexpr (Screen<Map>::kOk) {
+      if (a.screen) {
+        const void* k = (const void*)batch_screen_kernel<Map, Grid>;
+        batch_screen_kernel<Map, Grid><<<batch_grid(k, 256), 256, 0, s>>>(a);
+        return cudaGetLastError();
+      }
+    }
     if constexpr (Map::D <= 2) {
       // four points per thread only for the two-dimensional maps (register budget)
       if (tu.ppt == 4) {
@@ -608,6 +730,8 @@ struct b12g_batch {
   std::vector<uint8_t> depth_sorted;
   std::vector<uint32_t> active;        // active[k] = instances with depth >= k (k = 0..max_depth+1)
   Buf<double> params;                  // sorted order
+  Buf<ScreenRec> screen;               // a record an instance and step (max_depth x N), when screened
+  ScreenArgs screen_common{};
   Buf<uint8_t> depths;                 // sorted order
   Buf<uint64_t> code[2];
   Buf<uint8_t> flags[2];
@@ -693,6 +817,39 @@ b12g_status batch_reset(b12g_batch* b)
   return B12G_OK;
 }
 
+// the records of every step: all instances share their map's coefficients but for their own
+// (rho of Lorenz, gamma of forced Duffing), else the batch runs the maps' own arithmetic
+b12g_status batch_screen_records(b12g_batch* b, const std::vector<double>& params)
+{
+  std::vector<ScreenRec> rec(size_t(b->max_depth) * b->N);
+  ScreenArgs common{};
+  for (uint32_t q = 0; q < b->N; ++q) {
+    MapParams mp = b->mp;
+    for (int j = 0; j < 6; ++j) mp.p[j] = params[size_t(q) * 6 + j];
+    ScreenPlan plan = screen_plan(b->scheme.map.kind, mp, b->dom, int(b->domain.dim),
+                                  grid_reach(b->scheme.grid.kind, b->gp));
+    for (uint32_t k = 1; k <= b->depth_sorted[q]; ++k) {
+      ScreenArgs s{};
+      screen_at(plan, int(k), s);
+      if (!screen_record(b->scheme.map.kind, int(b->domain.dim), s, common, rec[size_t(k - 1) * b->N + q]))
+        return B12G_OK;
+    }
+  }
+  if (!common.on) return B12G_OK;
+  ST(b->screen.ensure(rec.size(), "batch screen records"));
+  CK(cudaMemcpy(b->screen.p, rec.data(), rec.size() * sizeof(ScreenRec), cudaMemcpyHostToDevice));
+  b->screen_common = common;
+  return B12G_OK;
+}
+
+void batch_screen(const b12g_batch* b, uint32_t k, BatchArgs& a)
+{
+  if (!b->screen_common.on) return;
+  a.screen = b->screen.p + size_t(k - 1) * b->N;
+  for (int i = 0; i < kScreenCoef; ++i) a.sk[i] = b->screen_common.k[i];
+  for (int j = 0; j < 3; ++j) a.sA[j] = b->screen_common.sA[j];
+}
+
 // the launches of subdivision step k (1-based) reading offsets from off[k & 1 ^ 1]
 cudaError_t build_step_hash(b12g_batch* b, uint32_t k)
 {
@@ -732,6 +889,7 @@ cudaError_t enqueue_step(b12g_batch* b, uint32_t k, const Tuning& tu, bool with_
   a.queue = b->ctr.p + B_QUEUE;
   a.chunk = tu.chunk;
   a.error = b->ctr.p + B_ERROR;
+  batch_screen(b, k, a);
   cudaError_t e = launch_batch_image(b->scheme.map.kind, b->scheme.map.arith, b->scheme.grid.kind, tu, a, b->stream);
   if (e != cudaSuccess) return e;
   if (A > 0) inst_count_kernel<<<A, 256, 0, b->stream>>>(b->hit.p, b->off[in].p, b->cnt.p, b->hit.n,
@@ -956,12 +1114,17 @@ b12g_status b12g_batch_create(const b12g_domain* domain, const b12g_scheme* sche
     }
   }
   if (st == B12G_OK) st = batch_reserve(b, std::max<uint64_t>(1ull << 22, 4ull * n));
+  if (st == B12G_OK) st = batch_screen_records(b, ps);
   // start from the family's usual shape; the first run tunes it unless this process has
   b->tuning = batch_tuning(b->device, scheme->map.kind, scheme->map.arith, scheme->grid.kind, domain->dim);
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     auto it = g_tuned.find(tune_key(b->device, scheme->map.kind, scheme->map.arith, scheme->grid.kind));
     if (it != g_tuned.end()) { b->tuning = it->second; b->tuned = true; }
+  }
+  if (b->screen_common.on) {       // the screened kernel has one shape
+    b->tuning = Tuning{256, 1, 32 * kScreenTrips};
+    b->tuned = true;
   }
   if (st != B12G_OK) {
     b12g_batch_destroy(b);
@@ -977,7 +1140,7 @@ b12g_status b12g_batch_destroy(b12g_batch* b)
   if (b->stream) cudaStreamSynchronize(b->stream);
   if (b->graph) cudaGraphExecDestroy(b->graph);
   if (b->mp.table) cudaFree(const_cast<double*>(b->mp.table));
-  b->params.release(); b->depths.release(); b->hit.release(); b->cnt.release(); b->step_counts.release();
+  b->params.release(); b->screen.release(); b->depths.release(); b->hit.release(); b->cnt.release(); b->step_counts.release();
   b->ctr.release(); b->tiles_a.release(); b->tiles_b.release(); b->fin_lo.release(); b->fin_len.release();
   b->arena_off.release(); b->arena_inst.release(); b->hash.release();
   b->fin_code.release(); b->fin_flags.release(); b->stage_col.release(); b->stage_cnt.release();

@@ -42,6 +42,11 @@ struct BatchArgs {
   // tgt_base[i] != ~0: targets[tgt_base[i] + (child - 2 off[i]) * points + k]
   uint32_t* targets;
   const uint64_t* tgt_base;
+  // the screened evaluation, when `screen` is set: a record an instance for its children's
+  // depth, and what the instances share
+  const ScreenRec* screen;
+  double sk[kScreenCoef];
+  double sA[3];
 };
 
 // transition rows of the instances finishing in a step, from the targets their last

@@ -271,6 +271,38 @@ template<> struct Spread32<4> {
   }
 };
 
+// ... and its inverse
+template<int D> struct Compact32;
+template<> struct Compact32<2> {
+  static __device__ __forceinline__ uint32_t f(uint32_t x)
+  {
+    x &= 0x55555555u;
+    x = (x ^ (x >> 1)) & 0x33333333u;
+    x = (x ^ (x >> 2)) & 0x0F0F0F0Fu;
+    x = (x ^ (x >> 4)) & 0x00FF00FFu;
+    return (x ^ (x >> 8)) & 0x0000FFFFu;
+  }
+};
+template<> struct Compact32<3> {
+  static __device__ __forceinline__ uint32_t f(uint32_t x)
+  {
+    x &= 0x09249249u;
+    x = (x ^ (x >> 2)) & 0x030C30C3u;
+    x = (x ^ (x >> 4)) & 0x0300F00Fu;
+    x = (x ^ (x >> 8)) & 0xFF0000FFu;
+    return (x ^ (x >> 16)) & 0x3FFu;
+  }
+};
+template<> struct Compact32<4> {
+  static __device__ __forceinline__ uint32_t f(uint32_t x)
+  {
+    x &= 0x11111111u;
+    x = (x ^ (x >> 3)) & 0x03030303u;
+    x = (x ^ (x >> 6)) & 0x000F000Fu;
+    return (x ^ (x >> 12)) & 0xFFu;
+  }
+};
+
 template<int D>
 __device__ __forceinline__ uint64_t interleave(const uint32_t (&bits)[D], const int (&k)[D], int depth)
 {
@@ -307,6 +339,39 @@ __device__ __forceinline__ uint64_t code_of_bits(const DepthConst& dc, const uin
   int k[D];
 #pragma unroll
   for (int j = 0; j < D; ++j) k[j] = dc.k[j];
+  return interleave<D>(bits, k, depth);
+}
+
+// the per-dimension indices of a depth-d code, and the code of the indices, in 32 bits where
+// the code's full rounds fit them
+template<int D>
+__device__ __forceinline__ void split_code(uint64_t code, int depth, uint32_t (&bits)[D])
+{
+  const int K = (depth + D - 1) / D;
+  if (K <= Spread32<D>::kMax) {
+    const uint32_t c = uint32_t(code) << (D * K - depth);
+#pragma unroll
+    for (int j = 0; j < D; ++j)
+      bits[j] = Compact32<D>::f(c >> (D - 1 - j)) >> (K - bisections<D>(depth, j));
+  } else {
+#pragma unroll
+    for (int j = 0; j < D; ++j) bits[j] = deinterleave<D>(code, depth, j);
+  }
+}
+
+template<int D>
+__device__ __forceinline__ uint64_t join_code(const uint32_t (&bits)[D], int depth)
+{
+  const int K = (depth + D - 1) / D;
+  if (K <= Spread32<D>::kMax && depth > 0) {
+    uint32_t x = 0;
+#pragma unroll
+    for (int j = 0; j < D; ++j) x |= Spread32<D>::f(bits[j] << (K - bisections<D>(depth, j))) << (D - 1 - j);
+    return uint64_t(x >> (D * K - depth));
+  }
+  int k[D];
+#pragma unroll
+  for (int j = 0; j < D; ++j) k[j] = bisections<D>(depth, j);
   return interleave<D>(bits, k, depth);
 }
 

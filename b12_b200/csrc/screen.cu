@@ -84,13 +84,6 @@ struct StepBound {
   double d[B12G_MAX_DIM];
 };
 
-// a map's part of a screen: scales, shifts, the box of states and the distance E at the end
-struct MapBound {
-  double scale[B12G_MAX_DIM] = {1.0, 1.0, 1.0, 1.0}, shift[B12G_MAX_DIM] = {0.0, 0.0, 0.0, 0.0};
-  double lim[B12G_MAX_DIM] = {0.0, 0.0, 0.0, 0.0};   // unscaled, around the shift
-  double E[B12G_MAX_DIM] = {0.0, 0.0, 0.0, 0.0};
-};
-
 void identity_box(const double* lim, int dim, Bound* x)
 {
   for (int j = 0; j < dim; ++j) {
@@ -334,6 +327,25 @@ double grid_reach(uint32_t grid_kind, const GridParams& g)
   return grid_kind == B12G_GRID_FULL ? m * std::fabs(g.eps1) : m;
 }
 
+ScreenPlan screen_plan(uint32_t map_kind, const MapParams& map, const Domain& dom, int dim, double gmax)
+{
+  ScreenPlan p;
+  p.kind = map_kind;
+  p.map = map;
+  p.dom = dom;
+  p.dim = dim;
+  p.gmax = gmax;
+  if (map_kind == B12G_MAP_HENON) return p;      // five operations: nothing to save
+  if (map.steps == 0 || map.steps > 4096 || !moderate_nonzero(map.h) || !moderate(gmax)) return p;
+  for (double v : map.p)
+    if (!moderate(v)) return p;
+  for (int j = 0; j < dim; ++j)
+    if (!moderate_nonzero(dom.r[j]) || !moderate(dom.c[j])) return p;
+  if (map_kind == B12G_MAP_FORCED_DUFFING && !(map.h > 0.0 && map.p[2] > 0.0 && moderate_nonzero(map.p[2]))) return p;
+  p.possible = true;
+  return p;
+}
+
 // The screened evaluation applies when the parameters are moderate, every dimension has at
 // most kScreenMaxBits bisections and the share P of the points it cannot decide (those
 // within the guard of a box boundary, if they lie evenly) is small.  The wider the box of
@@ -341,35 +353,31 @@ double grid_reach(uint32_t grid_kind, const GridParams& g)
 // multiples of the domain that keeps P under 2^-12 (one warp in 128 evaluates again), else
 // the narrowest if it keeps P under 2^-9 (one in 16: still faster than the map's own
 // arithmetic for every point, whose step is at least 1.25 times as long).
-void fill_screen(uint32_t map_kind, const MapParams& map, const Domain& dom, int dim, int depth, double gmax,
-                 ScreenArgs& s)
+void screen_at(ScreenPlan& plan, int depth, ScreenArgs& s)
 {
+  static const double kLambda[kScreenBoxes] = {2.0, 1.75, 1.5, 1.25, 1.1, 1.0};
   s.on = 0;
-  if (map_kind == B12G_MAP_HENON) return;      // five operations: nothing to save
-  if (map.steps == 0 || map.steps > 4096 || !moderate_nonzero(map.h) || !moderate(gmax)) return;
-  for (double p : map.p)
-    if (!moderate(p)) return;
-  for (int j = 0; j < dim; ++j)
-    if (!moderate_nonzero(dom.r[j]) || !moderate(dom.c[j])) return;
-  if (map_kind == B12G_MAP_FORCED_DUFFING && !(map.h > 0.0 && map.p[2] > 0.0 && moderate_nonzero(map.p[2]))) return;
+  if (!plan.possible) return;
+  const Domain& dom = plan.dom;
+  const int dim = plan.dim;
   DepthConst dc;
   fill_depth_const(dom, dim, depth, dc);
   for (int j = 0; j < dim; ++j)
     if (dc.k[j] > kScreenMaxBits) return;
-
-  static const double kLambda[] = {2.0, 1.75, 1.5, 1.25, 1.1, 1.0};
-  constexpr int kTries = int(sizeof kLambda / sizeof kLambda[0]);
-  for (int tr = 0; tr < kTries; ++tr) {
-    MapBound b;
-    // the start points: a few roundings of |c| + r (1 + |g|) on either side, and of the shift
-    double e0[B12G_MAX_DIM] = {0.0, 0.0, 0.0, 0.0};
-    for (int j = 0; j < dim; ++j) {
-      const double shift = map_kind == B12G_MAP_LORENZ && j == 2 ? std::fabs(map.p[1]) : 0.0;
-      e0[j] = 64.0 * kU * (std::fabs(dom.c[j]) + shift + 8.0 * dom.r[j] * (1.0 + gmax));
+  for (int tr = 0; tr < kScreenBoxes; ++tr) {
+    MapBound& b = plan.bound[tr];
+    if (!plan.found[tr]) {
+      // the start points: a few roundings of |c| + r (1 + |g|) on either side, and of the shift
+      double e0[B12G_MAX_DIM] = {0.0, 0.0, 0.0, 0.0};
+      for (int j = 0; j < dim; ++j) {
+        const double shift = plan.kind == B12G_MAP_LORENZ && j == 2 ? std::fabs(plan.map.p[1]) : 0.0;
+        e0[j] = 64.0 * kU * (std::fabs(dom.c[j]) + shift + 8.0 * dom.r[j] * (1.0 + plan.gmax));
+      }
+      if (plan.kind == B12G_MAP_LORENZ) lorenz_bound(plan.map, dom, kLambda[tr], e0, b, plan.k);
+      else if (plan.kind == B12G_MAP_FORCED_DUFFING) forced_bound(plan.map, dom, kLambda[tr], e0, b, plan.k);
+      else coupled_bound(plan.map, dom, kLambda[tr], e0, b, plan.k);
+      plan.found[tr] = true;
     }
-    if (map_kind == B12G_MAP_LORENZ) lorenz_bound(map, dom, kLambda[tr], e0, b, s.k);
-    else if (map_kind == B12G_MAP_FORCED_DUFFING) forced_bound(map, dom, kLambda[tr], e0, b, s.k);
-    else coupled_bound(map, dom, kLambda[tr], e0, b, s.k);
     double share = 0.0;
     bool ok = true;
     for (int j = 0; j < dim; ++j) {
@@ -383,7 +391,7 @@ void fill_screen(uint32_t map_kind, const MapParams& map, const Domain& dom, int
       if (!(g < 0.125)) { ok = false; break; }
       s.guard[j] = uint32_t(std::ceil(g * 0x1p32)) + 2u;
     }
-    if (!ok || !(share <= (tr == kTries - 1 ? 0x1p-9 : 0x1p-12))) continue;
+    if (!ok || !(share <= (tr == kScreenBoxes - 1 ? 0x1p-9 : 0x1p-12))) continue;
     for (int j = 0; j < dim; ++j) {
       const double S = b.scale[j], r = dom.r[j], rk = dc.ax[j].rk, half = 0.5 * dc.ax[j].pk;
       s.E[j] = b.E[j];
@@ -402,9 +410,48 @@ void fill_screen(uint32_t map_kind, const MapParams& map, const Domain& dom, int
       const uint32_t hi = uint32_t(w >> 32) - 1u;
       __builtin_memcpy(&s.lim[j], &hi, sizeof hi);
     }
+    for (int i = 0; i < kScreenCoef; ++i) s.k[i] = plan.k[i];
     s.on = 1;
     return;
   }
+}
+
+void fill_screen(uint32_t map_kind, const MapParams& map, const Domain& dom, int dim, int depth, double gmax,
+                 ScreenArgs& s)
+{
+  ScreenPlan plan = screen_plan(map_kind, map, dom, dim, gmax);
+  screen_at(plan, depth, s);
+}
+
+bool screen_record(uint32_t map_kind, int dim, const ScreenArgs& s, ScreenArgs& common, ScreenRec& rec)
+{
+  rec = ScreenRec{};
+  if (!s.on) return true;
+  // the coefficients an instance may have of its own (Screen<Map>::own)
+  int own[2] = {-1, -1};
+  if (map_kind == B12G_MAP_LORENZ) { own[0] = 5; own[1] = 9; }
+  else if (map_kind == B12G_MAP_FORCED_DUFFING) own[0] = 3;
+  else return false;
+  if (!common.on) {
+    common = s;
+  } else {
+    for (int i = 0; i < kScreenCoef; ++i)
+      if (i != own[0] && i != own[1] && std::memcmp(&s.k[i], &common.k[i], sizeof(double)) != 0) return false;
+    for (int j = 0; j < dim; ++j)
+      if (std::memcmp(&s.sA[j], &common.sA[j], sizeof(double)) != 0) return false;
+  }
+  for (int i = 0; i < 2; ++i) rec.own[i] = own[i] >= 0 ? s.k[own[i]] : 0.0;
+  for (int j = 0; j < dim; ++j) {
+    rec.sB[j] = s.sB[j];
+    rec.tB[j] = s.tB[j];
+    rec.sR[j] = s.sR[j];
+    rec.tA[j] = s.tA[j];
+    rec.guard[j] = s.guard[j];
+    rec.lim[j] = s.lim[j];
+    rec.k |= s.bits[j] << (8 * j);
+  }
+  rec.on = 1;
+  return true;
 }
 
 namespace {

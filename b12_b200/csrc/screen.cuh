@@ -185,7 +185,13 @@ template<class Map> struct Screen { static constexpr bool kOk = false; };
 #ifdef __CUDACC__
 template<class A> struct Screen<LorenzMap<A>> {
   static constexpr bool kOk = true;
+  static constexpr int kOwnCount = 2;                     // rho: kappa and kappa / 3
+  static __host__ __device__ constexpr int own(int i) { return i == 0 ? 5 : 9; }
   static __device__ __forceinline__ bool run(const ScreenArgs& s, const MapParams& map, double (&x)[3])
+  {
+    return run(s.k, s.lim, map, x);
+  }
+  static __device__ __forceinline__ bool run(const double* k, const float* lim, const MapParams& map, double (&x)[3])
   {
     float m0 = 0.f, m1 = 0.f, m2 = 0.f;
 #pragma unroll 4
@@ -193,9 +199,9 @@ template<class A> struct Screen<LorenzMap<A>> {
       screen_track(m0, x[0]);
       screen_track(m1, x[1]);
       screen_track(m2, x[2]);
-      lorenz_screen_step(s.k, x);
+      lorenz_screen_step(k, x);
     }
-    return m0 <= s.lim[0] && m1 <= s.lim[1] && m2 <= s.lim[2];
+    return m0 <= lim[0] && m1 <= lim[1] && m2 <= lim[2];
   }
 };
 
@@ -226,20 +232,26 @@ template<> struct Screen<CoupledDuffingMap> {
 
 template<> struct Screen<ForcedDuffingMap> {
   static constexpr bool kOk = true;
+  static constexpr int kOwnCount = 1;                     // gamma: the scale of F
+  static __host__ __device__ constexpr int own(int) { return 3; }
   static __device__ __forceinline__ bool run(const ScreenArgs& s, const MapParams& map, double (&x)[2])
   {
+    return run(s.k, s.lim, map, x);
+  }
+  static __device__ __forceinline__ bool run(const double* k, const float* lim, const MapParams& map, double (&x)[2])
+  {
     float m0 = 0.f, m1 = 0.f;
-    double f0 = __dmul_rn(s.k[3], __ldg(map.table));
+    double f0 = __dmul_rn(k[3], __ldg(map.table));
 #pragma unroll 2
     for (uint32_t i = 0; i < map.steps; ++i) {
-      const double f1 = __dmul_rn(s.k[3], __ldg(map.table + 2 * i + 1));
-      const double f2 = __dmul_rn(s.k[3], __ldg(map.table + 2 * i + 2));
+      const double f1 = __dmul_rn(k[3], __ldg(map.table + 2 * i + 1));
+      const double f2 = __dmul_rn(k[3], __ldg(map.table + 2 * i + 2));
       screen_track(m0, x[0]);
       screen_track(m1, x[1]);
-      forced_screen_step(s.k, f0, f1, f2, x);
+      forced_screen_step(k, f0, f1, f2, x);
       f0 = f2;
     }
-    return m0 <= s.lim[0] && m1 <= s.lim[1];
+    return m0 <= lim[0] && m1 <= lim[1];
   }
 };
 
@@ -271,12 +283,53 @@ __device__ __forceinline__ bool screen_locate(const ScreenArgs& s, const double 
 }
 #endif
 
+// One instance's part of a batched launch (batch.cu): the start, position and limits of its
+// parameters at its depth.  The coefficients are the launch's (BatchArgs::sk) but for the
+// instance's own: coefficient Screen<Map>::own(i) is own[i], i < Screen<Map>::kOwnCount.
+struct alignas(16) ScreenRec {
+  double sB[3], tB[3], sR[3], tA[3];
+  double own[2];
+  uint32_t guard[3];
+  float lim[3];
+  uint32_t k;                  // bisections of the dimensions, a byte each
+  uint32_t on;
+};
+
 // ---------------------------------------------------------------------------- host
-// Fills `s` for a launch over boxes of `depth` (grid points at most gmax box radii from the
-// centre); s.on tells whether the screened evaluation applies (screen.cu states when).
+// a map's part of a screen over one box of states: scales, shifts, limits and the distance
+// E of the two images
+struct MapBound {
+  double scale[B12G_MAX_DIM] = {1.0, 1.0, 1.0, 1.0}, shift[B12G_MAX_DIM] = {0.0, 0.0, 0.0, 0.0};
+  double lim[B12G_MAX_DIM] = {0.0, 0.0, 0.0, 0.0};   // unscaled, around the shift
+  double E[B12G_MAX_DIM] = {0.0, 0.0, 0.0, 0.0};
+};
+
+// The depth-independent part of a screen: a map's bounds over multiples of the domain (found
+// when a depth first asks for them) and its coefficients.
+constexpr int kScreenBoxes = 6;
+struct ScreenPlan {
+  uint32_t kind = 0;
+  MapParams map{};
+  Domain dom{};
+  int dim = 0;
+  double gmax = 0.0;
+  bool possible = false;
+  bool found[kScreenBoxes] = {};
+  MapBound bound[kScreenBoxes];
+  double k[kScreenCoef] = {};
+};
+// grid points at most gmax box radii from the centre
+ScreenPlan screen_plan(uint32_t map_kind, const MapParams& map, const Domain& dom, int dim, double gmax);
+// fills `s` for launches over boxes of `depth`; s.on tells whether the screened evaluation
+// applies (screen.cu states when)
+void screen_at(ScreenPlan& plan, int depth, ScreenArgs& s);
+// both at once
 void fill_screen(uint32_t map_kind, const MapParams& map, const Domain& dom, int dim, int depth, double gmax,
                  ScreenArgs& s);
 // the largest |coordinate| of a grid's points
 double grid_reach(uint32_t grid_kind, const GridParams& g);
+// the record of a batched instance; false where it cannot share `common`'s coefficients and
+// scales (common.on == 0: the first one, which sets them)
+bool screen_record(uint32_t map_kind, int dim, const ScreenArgs& s, ScreenArgs& common, ScreenRec& rec);
 
 }  // namespace b12g

@@ -79,6 +79,7 @@ struct Job {
   uint64_t reserved = 0;          // admitted bytes
   uint32_t depth_done = 0;        // subdivision steps done
   std::vector<uint32_t> counts;   // leaves after each step
+  ScreenPlan plan;                // its screened evaluation (engine thread once running)
   // resident result: one block from the server's pool holding codes, vals, rowptr, cols
   void* mem = nullptr;
   uint64_t* codes = nullptr;
@@ -109,6 +110,8 @@ struct Engine {
   Buf<uint8_t> flags_a, flags_b, hit;
   Buf<uint32_t> off, new_off, cnt, ctr, tiles_a, tiles_b, keep_off, fin_off, fin_slot, fin_rank, row0;
   Buf<double> params, fin_params;
+  Buf<ScreenRec> screen;             // the running jobs' records of this tick
+  ScreenRec* hs = nullptr;           // pinned mirror
   Buf<uint8_t> depth_child, fin_depth;
   Buf<ulonglong2> hash;
   uint32_t hash_log2 = 0, tag = 0;
@@ -348,6 +351,8 @@ b12g_status engine_init(Engine* e, const b12g_job& key)
   CK(cudaMallocHost(&e->hp, size_t(kMaxSlots) * 6 * 8));
   CK(cudaMallocHost(&e->hd, 2 * size_t(kMaxSlots)));
   CK(cudaMallocHost(&e->ht, size_t(kMaxSlots) * 8));
+  CK(cudaMallocHost(&e->hs, size_t(kMaxSlots) * sizeof(ScreenRec)));
+  ST(e->screen.ensure(kMaxSlots, "engine screen records"));
   ST(e->tgt_base.ensure(kMaxSlots, "engine targets offsets"));
   ST(e->fin_child.ensure(2 * kMaxSlots + 1, "engine finishing children"));
   ST(e->off.ensure(kMaxSlots + 1, "engine offsets"));
@@ -580,6 +585,9 @@ b12g_status engine_tick(Engine* e, const std::vector<Job*>& joining)
     const double t = now_s();
     for (Job* j : joining) {
       j->t_start = t;
+      MapParams mp = e->mp;
+      for (int k = 0; k < 6; ++k) mp.p[k] = j->spec.map.p[k];
+      j->plan = screen_plan(e->key.map.kind, mp, e->dom, int(e->key.domain.dim), grid_reach(e->key.grid.kind, e->gp));
       e->slots.push_back(j);
     }
   }
@@ -661,6 +669,21 @@ b12g_status engine_tick(Engine* e, const std::vector<Job*>& joining)
   a.error = e->ctr.p + E_ERROR;
   a.targets = store ? e->targets.p : nullptr;
   a.tgt_base = store ? e->tgt_base.p : nullptr;
+  // the jobs' records at their children's depths; jobs that do not share their coefficients
+  // run the map's own arithmetic
+  ScreenArgs common{};
+  bool shared = true;
+  for (uint32_t i = 0; i < A && shared; ++i) {
+    ScreenArgs sa{};
+    screen_at(e->slots[i]->plan, int(e->hd[i]), sa);
+    shared = screen_record(e->key.map.kind, int(e->key.domain.dim), sa, common, e->hs[i]);
+  }
+  if (shared && common.on) {
+    CK(cudaMemcpyAsync(e->screen.p, e->hs, size_t(A) * sizeof(ScreenRec), cudaMemcpyHostToDevice, e->stream));
+    a.screen = e->screen.p;
+    for (int i = 0; i < kScreenCoef; ++i) a.sk[i] = common.k[i];
+    for (int j = 0; j < 3; ++j) a.sA[j] = common.sA[j];
+  }
   CK(launch_batch_image(e->key.map.kind, e->key.map.arith, e->key.grid.kind, e->tuning, a, e->stream));
   // 3. survivors per job, then one ordered compaction of all children
   CK(launch_inst_count(e->hit.p, e->off.p, A, e->cnt.p, e->hit.n, e->ctr.p + E_ERROR, e->stream));
@@ -778,11 +801,12 @@ void engine_release(Engine* e)
   if (e->hp) cudaFreeHost(e->hp);
   if (e->hd) cudaFreeHost(e->hd);
   if (e->ht) cudaFreeHost(e->ht);
+  if (e->hs) cudaFreeHost(e->hs);
   e->targets.release(); e->rank.release(); e->fin_child.release(); e->tgt_base.release();
   e->parents.release(); e->children.release(); e->flags_a.release(); e->flags_b.release(); e->hit.release();
   e->off.release(); e->new_off.release(); e->cnt.release(); e->ctr.release(); e->tiles_a.release();
   e->tiles_b.release(); e->keep_off.release(); e->fin_off.release(); e->fin_slot.release(); e->fin_rank.release();
-  e->row0.release(); e->params.release(); e->fin_params.release(); e->depth_child.release();
+  e->row0.release(); e->params.release(); e->screen.release(); e->fin_params.release(); e->depth_child.release();
   e->fin_depth.release(); e->hash.release(); e->arena.release(); e->stage_col.release(); e->stage_cnt.release();
   e->row_count.release(); e->rowptr.release(); e->cols_all.release(); e->vals_all.release();
   if (e->stream) cudaStreamDestroy(e->stream);

@@ -106,3 +106,60 @@ def test_queue_turns_through_graphs_and_single_launches():
         assert np.array_equal(t.search_by_image(sc), o.search_by_image())
         assert t.set_flags_by_image(sc, B.HIT) == o.set_flags_by_image(1)
     t.close()
+
+
+LORENZ_BATCHES = [
+    # one set of coefficients but rho: screened; strict and FMA, deep and shallow
+    ([(10.0, 28.0, 8.0 / 3.0), (10.0, 15.5, 8.0 / 3.0), (10.0, 34.9, 8.0 / 3.0)], [17, 3, 12], 0),
+    ([(10.0, 28.0, 8.0 / 3.0), (10.0, 21.0, 8.0 / 3.0)], [1, 16], 1),
+    # other sigma and beta too: each map's own arithmetic
+    ([(10.0, 28.0, 8.0 / 3.0), (9.5, 28.0, 8.0 / 3.0), (10.0, 28.0, 2.5)], [14, 15, 9], 1),
+    # an instance the bound does not cover beside one it does
+    ([(10.0, 28.0, 8.0 / 3.0), (10.0, 900.0, 8.0 / 3.0)], [12, 12], 0),
+]
+FORCED_BATCHES = [
+    ([(0.25, -1.0, 1.0, 0.3), (0.25, -1.0, 1.0, 0.05), (0.25, -1.0, 1.0, 0.42)], [13, 15, 6]),
+    ([(0.25, -1.0, 1.0, 0.3), (0.2, -1.0, 1.0, 0.3)], [11, 12]),
+    ([(0.25, -1.0, -0.01, 0.3), (0.25, -1.0, -0.01, 0.2)], [9, 10]),
+]
+
+
+@pytest.mark.parametrize("which", [("lorenz", i) for i in range(len(LORENZ_BATCHES))] +
+                         [("forced", i) for i in range(len(FORCED_BATCHES))])
+def test_batches_and_served_jobs_equal_single_trees(which):
+    import b12_b200 as B
+    from b12_b200.server import JobServer
+    name, i = which
+    if name == "lorenz":
+        params, depths, fma = LORENZ_BATCHES[i]
+        spec, maps = lorenz(), [B.lorenz(*p, fma=bool(fma)) for p in params]
+        grid = B.inner_grid(4)
+    else:
+        params, depths = FORCED_BATCHES[i]
+        spec, maps = forced(), [B.forced_duffing(200, *p) for p in params]
+        grid = B.inner_grid(3)
+    b = B.Batch(spec["center"], spec["radius"], B.Scheme(maps[0], grid), params, depths)
+    b.run()
+    b.run()
+    b.transition_matrices()
+    with JobServer() as srv:
+        ids = [srv.submit(spec["center"], spec["radius"], m, grid, d) for m, d in zip(maps, depths)]
+        srv.wait_all(ids)
+        for k, (m, d) in enumerate(zip(maps, depths)):
+            t = B.ImplicitBoxTree(spec["center"], spec["radius"])
+            sc = B.Scheme(m, grid)
+            counts = t.subdivision_run(sc, d)
+            codes = t.leaves()[0]
+            want = t.transition_matrix(sc).to_host()
+            r = srv.result(ids[k])
+            assert np.array_equal(b.counts(k), counts) and np.array_equal(r["counts"], counts)
+            if t.depth() != d:
+                t.close()
+                continue           # every box was lost: batches and jobs keep no rows for such an instance
+            assert np.array_equal(b.leaves(k)[0], codes) and np.array_equal(r["codes"], codes)
+            for x, y in zip(b.csr(k), want):
+                assert np.array_equal(x, y)
+            for x, y in zip((r["rowptr"], r["cols"], r["vals"]), want):
+                assert np.array_equal(x, y)
+            t.close()
+    b.close()
