@@ -455,7 +455,8 @@ b12g_status b12g_tree_destroy(b12g_tree* t)
   t->src.release(); t->out.release(); t->stage_col.release(); t->stage_cnt.release();
   t->row_count.release(); t->rowptr.release(); t->cand.release(); t->cand2.release();
   t->sort_idx.release(); t->table.release(); t->step_counts.release(); t->sort_tmp.release();
-  t->last_tgt.release(); t->last_rank.release();
+  t->last_tgt.release(); t->last_rank.release(); t->srcc.release(); t->bits.release(); t->pk.release();
+  t->route_runs.release(); t->route_cnt.release();
   if (t->h_ctr) cudaFreeHost(t->h_ctr);
   if (t->stream) cudaStreamDestroy(t->stream);
   delete t;
