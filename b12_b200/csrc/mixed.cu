@@ -29,6 +29,7 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr uint32_t kTable = 2048;   // doubles of the per-block grid-point table
+constexpr int kScreenBlocks = 6;    // resident blocks an SM of mixed_screen_kernel
 
 int grid_for_n(uint64_t n, int per_thread = 1)
 {
@@ -684,7 +685,29 @@ struct MixedArgs {
   uint32_t* row_count;
   int keep_lost;
   uint32_t lost_col;
+  // the screened evaluation (sc.on; sources are leaves): images located at the depth of the
+  // deepest leaf, from the leaves' centres (kSrcStride doubles a leaf)
+  ScreenArgs sc;
+  int depth;
+  const double* src_c;
+  uint32_t* work;              // the tree's work-queue counters in turn, as for the image kernel
+  uint32_t* work_next;
 };
+
+// the centre of every leaf's box (kSrcStride doubles a leaf), for the screened kernels: a
+// point then reads it instead of decoding the leaf's code and rebuilding the box
+template<int D>
+__global__ void leaf_centres_kernel(const uint64_t* __restrict__ code, const uint8_t* __restrict__ dep, uint32_t n,
+                                    Domain dom, double* __restrict__ out)
+{
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    double c[kSrcStride] = {0.0, 0.0, 0.0, 0.0}, r[D];
+    box_coordinates<D>(dom, code[i], int(dep[i]), c, r);
+    double2* o = reinterpret_cast<double2*>(out + size_t(kSrcStride) * i);
+    o[0] = make_double2(c[0], c[1]);
+    o[1] = make_double2(c[2], c[3]);
+  }
+}
 
 template<class Grid, int D>
 __device__ __forceinline__ bool load_table(const GridParams& g, uint64_t P, double* pts)
@@ -703,8 +726,9 @@ __device__ __forceinline__ bool load_table(const GridParams& g, uint64_t P, doub
 }
 
 // the depth-64 code of the image of point k of source leaf `leaf` (point index g);
-// false if the image left the domain
-template<class Map, class Grid>
+// false if the image left the domain.  kCold: for the few points a screened launch could
+// not decide
+template<class Map, class Grid, bool kCold = false>
 __device__ __forceinline__ bool image_code(const MixedArgs& a, const double* pts, bool table, uint32_t leaf,
                                            uint32_t k, uint64_t g, uint64_t& p64)
 {
@@ -726,18 +750,65 @@ __device__ __forceinline__ bool image_code(const MixedArgs& a, const double* pts
   }
 #pragma unroll
   for (int j = 0; j < D; ++j) x[j] = __dadd_rn(c[j], __dmul_rn(gp[j], r[j]));
-  Map::apply(a.map, x, y);
+  if constexpr (kCold) Map::apply_cold(a.map, x, y);
+  else Map::apply(a.map, x, y);
   p64 = 0;
   return point_code<D>(a.dom, y, 64, p64);
 }
 
-// the leaf the image of point k of source leaf `leaf` lands in (point index g)
+// the same from the screened evaluation: the code's first a.depth bits (the deepest leaf's
+// depth), zeros below, which lead to the same leaf - every leaf is a prefix of at most that
+// many bits, and the leaves before the one that holds the point lie below its first code.
+// Returns whether the evaluation decided the point.
 template<class Map, class Grid>
+__device__ __forceinline__ bool screened_code(const MixedArgs& a, const double* pts, bool table, uint32_t leaf,
+                                              uint32_t k, uint64_t g, uint64_t& p64, bool& valid)
+{
+  constexpr int D = Map::D;
+  double c[4], gp[D], x[D];
+  const int depth = int(__ldg(a.dep + leaf));
+  const double2* p = reinterpret_cast<const double2*>(a.src_c + kSrcStride * size_t(leaf));
+  const double2 c01 = __ldg(p);
+  c[0] = c01.x;
+  c[1] = c01.y;
+  if (D > 2) {
+    const double2 c23 = __ldg(p + 1);
+    c[2] = c23.x;
+    c[3] = c23.y;
+  }
+  if (Grid::kTable && table) {
+#pragma unroll
+    for (int j = 0; j < D; ++j) gp[j] = pts[j * uint32_t(a.points) + k];
+  } else {
+    Grid::template point<D>(a.grid, pts, g, k, gp);
+  }
+#pragma unroll
+  for (int j = 0; j < D; ++j) {
+    // the leaf's radius: sR is scaled for the deepest leaf's, an exact power of two smaller
+    const int up = int(a.sc.bits[j]) - bisections<D>(depth, j);
+    const double rs = __hiloint2double(__double2hiint(a.sc.sR[j]) + (up << 20), __double2loint(a.sc.sR[j]));
+    x[j] = __fma_rn(gp[j], rs, __fma_rn(c[j], a.sc.sC[j], a.sc.sD[j]));
+  }
+  uint32_t tb[D];
+  const bool kept = Screen<Map>::run(a.sc, a.map, x);
+  const bool sure = screen_locate<D>(a.sc, x, tb, valid) && kept;
+  p64 = valid ? join_code<D>(tb, a.depth) << (64 - a.depth) : 0ull;
+  return sure;
+}
+
+// the leaf the image of point k of source leaf `leaf` lands in (point index g)
+template<class Map, class Grid, bool kScreen = false>
 __device__ __forceinline__ uint32_t image_of(const MixedArgs& a, const double* pts, bool table, uint32_t leaf,
                                              uint32_t k, uint64_t g)
 {
   uint64_t p64;
-  const bool valid = image_code<Map, Grid>(a, pts, table, leaf, k, g, p64);
+  bool valid;
+  if constexpr (kScreen) {
+    if (!screened_code<Map, Grid>(a, pts, table, leaf, k, g, p64, valid))
+      valid = image_code<Map, Grid, true>(a, pts, table, leaf, k, g, p64);
+  } else {
+    valid = image_code<Map, Grid>(a, pts, table, leaf, k, g, p64);
+  }
   return locate_mixed(CmpIndex{a.cmp, a.tab, a.n, a.tab_bits}, a.code, a.dep, valid, p64);
 }
 
@@ -816,8 +887,58 @@ __global__ void __launch_bounds__(kThreads) mixed_image_kernel(const MixedArgs a
   }
 }
 
+// modes 0 and 1 with the screened evaluation and the image kernel's work queue (units of 32
+// points, four at a time while many are left).  Bound by FP64 issue, like that kernel; the
+// leaves' centres come from a table of one pass over the leaves instead of being rebuilt for
+// every point.  Six selective steps of Lorenz (FMA) from depth 20: 1.95 ms against 2.46 (five
+// blocks an SM 1.98, four 1.98).
+template<class Map, class Grid, int kMode>
+__global__ void __launch_bounds__(kThreads, kScreenBlocks) mixed_screen_kernel(const MixedArgs a)
+{
+  __shared__ double pts[kTable];
+  const bool table = load_table<Grid, Map::D>(a.grid, a.points, pts);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *a.work_next = 0u;
+  const uint64_t P = a.points, total = uint64_t(a.n_src) * P;
+  const uint32_t P32 = uint32_t(P);
+  const int lane = threadIdx.x & 31;
+  constexpr uint32_t kTrips = 4, kFine = 4;
+  uint32_t shift = 0;
+  while (((total + 31) >> (5 + shift)) >= 0x40000000ull) ++shift;
+  const uint32_t units = uint32_t((total + (32ull << shift) - 1) >> (5 + shift));
+  const uint32_t fine = gridDim.x * (kThreads / 32) * kFine;
+  const uint32_t coarse_end = units > fine ? units - fine : 0;
+  uint32_t c = 0;
+  for (;;) {
+    const uint32_t size = c < coarse_end ? kTrips : 1u;
+    if (lane == 0) c = atomicAdd(a.work, size);
+    c = __shfl_sync(0xFFFFFFFFu, c, 0);
+    if (c >= units) break;
+    const uint64_t g = (uint64_t(c) << (5 + shift)) + uint64_t(lane);
+    uint32_t rank, k;
+    if (total <= 0xFFFFFFFFull - 64ull * kTrips) {
+      rank = uint32_t(g) / P32;
+      k = uint32_t(g) - rank * P32;
+    } else {
+      rank = uint32_t(g / P);
+      k = uint32_t(g - uint64_t(rank) * P);
+    }
+#pragma unroll 1
+    for (uint32_t j = 0; j < (size << shift); ++j) {
+      const uint64_t gj = g + 32ull * j;
+      if (gj < total) {
+        const uint32_t leaf = a.src ? __ldg(a.src + rank) : rank;
+        const uint32_t t = image_of<Map, Grid, true>(a, pts, table, leaf, k, gj);
+        if constexpr (kMode == 1) a.out[gj] = t;
+        else if (t != kInvalidIndex) a.hit[t] = 1;
+      }
+      k += 32;
+      while (k >= P32) { k -= P32; ++rank; }
+    }
+  }
+}
+
 // a warp per leaf: its P <= 128 targets sorted and run-length counted (as for uniform trees)
-template<class Map, class Grid>
+template<class Map, class Grid, bool kScreen>
 __global__ void __launch_bounds__(kThreads) mixed_rows_kernel(const MixedArgs a)
 {
   constexpr int kWarps = kThreads / 32;
@@ -834,7 +955,7 @@ __global__ void __launch_bounds__(kThreads) mixed_rows_kernel(const MixedArgs a)
       const uint32_t k = uint32_t(lane) + 32u * q;
       uint32_t key = kPadKey;
       if (k < P) {
-        const uint32_t t = image_of<Map, Grid>(a, pts, table, row, k, uint64_t(row) * P + k);
+        const uint32_t t = image_of<Map, Grid, kScreen>(a, pts, table, row, k, uint64_t(row) * P + k);
         key = t == kInvalidIndex ? kLostKey : t;
       }
       s[lane + 32 * q] = key;
@@ -1042,6 +1163,53 @@ b12g_status mixed_args(b12g_tree* t, const b12g_scheme* sc, MixedArgs& a)
   a.cmp = t->cmp.p;
   a.tab = t->cmp_tab.p;
   a.tab_bits = t->cmp_bits;
+  return B12G_OK;
+}
+
+// the screened evaluation's arguments (a.sc.on: it applies) with the leaves' centres
+b12g_status mixed_screen(b12g_tree* t, const b12g_scheme* sc, MixedArgs& a)
+{
+  if (a.src_depth || t->depth == 0) return B12G_OK;
+  a.depth = int(t->depth);
+  fill_screen(sc->map.kind, a.map, a.dom, int(t->domain.dim), a.depth, grid_reach(sc->grid.kind, a.grid), a.sc);
+  if (!a.sc.on) return B12G_OK;
+  ST(t->srcc.ensure_room(uint64_t(std::max<uint32_t>(t->n, 1)) * kSrcStride, "leaf centres", 2));
+  a.src_c = t->srcc.p;
+  const int g = grid_for_n(t->n);
+  switch (t->domain.dim) {
+    case 2: leaf_centres_kernel<2><<<g, kThreads, 0, t->stream>>>(a.code, a.dep, a.n, a.dom, t->srcc.p); break;
+    case 3: leaf_centres_kernel<3><<<g, kThreads, 0, t->stream>>>(a.code, a.dep, a.n, a.dom, t->srcc.p); break;
+    default: leaf_centres_kernel<4><<<g, kThreads, 0, t->stream>>>(a.code, a.dep, a.n, a.dom, t->srcc.p); break;
+  }
+  CK(cudaGetLastError());
+  count_launches(1);
+  return B12G_OK;
+}
+
+// an image launch over the prepared sources: kMode 0 hit marks, 1 leaf indices
+template<int kMode>
+b12g_status mixed_image_launch(b12g_tree* t, const b12g_scheme* sc, MixedArgs& a)
+{
+  ST(mixed_screen(t, sc, a));
+  const uint64_t np = uint64_t(a.n_src) * a.points;
+  CK(dispatch(sc->map.kind, sc->map.arith, sc->grid.kind, t->domain.dim, [&](auto map, auto grid) -> cudaError_t {
+    using Map = decltype(map);
+    using Grid = decltype(grid);
+    if constexpr (Screen<Map>::kOk) {
+      if (a.sc.on) {
+        a.work = t->ctr.p + C_WORK + (t->work_turn & 1u);
+        a.work_next = t->ctr.p + C_WORK + ((t->work_turn & 1u) ^ 1u);
+        const uint64_t want = std::max<uint64_t>((np + kThreads - 1) / kThreads, 1);
+        const uint64_t cap = uint64_t(device_sm_count()) * kScreenBlocks;
+        mixed_screen_kernel<Map, Grid, kMode><<<unsigned(std::min(want, cap)), kThreads, 0, t->stream>>>(a);
+        const cudaError_t e = cudaGetLastError();
+        if (e == cudaSuccess) t->work_turn ^= 1u;
+        return e;
+      }
+    }
+    mixed_image_kernel<Map, Grid, kMode><<<grid_for_n(np), kThreads, 0, t->stream>>>(a);
+    return cudaGetLastError();
+  }));
   return B12G_OK;
 }
 
@@ -1278,11 +1446,7 @@ b12g_status mixed_set_flags_by_image(b12g_tree* t, const b12g_scheme* sc, uint8_
     CK(cudaMemsetAsync(t->hit.p, 0, t->hit.n, t->stream));
   }
   a.hit = t->hit.p;
-  CK(dispatch(sc->map.kind, sc->map.arith, sc->grid.kind, t->domain.dim, [&](auto map, auto grid) -> cudaError_t {
-    mixed_image_kernel<decltype(map), decltype(grid), 0>
-        <<<grid_for_n(uint64_t(a.n_src) * a.points), kThreads, 0, t->stream>>>(a);
-    return cudaGetLastError();
-  }));
+  ST(mixed_image_launch<0>(t, sc, a));
   ST(set_ctr(t, C_CHANGED, 0));
   apply_hits_kernel<<<grid_for_n(t->n), kThreads, 0, t->stream>>>(t->flg(), t->hit.p, t->n, flags,
                                                                    t->ctr.p + C_CHANGED);
@@ -1301,10 +1465,7 @@ b12g_status mixed_search(b12g_tree* t, const b12g_scheme* sc, uint64_t* n_points
   const uint64_t np = uint64_t(a.n_src) * a.points;
   ST(t->out.ensure(std::max<uint64_t>(np, 1), "search output"));
   a.out = t->out.p;
-  CK(dispatch(sc->map.kind, sc->map.arith, sc->grid.kind, t->domain.dim, [&](auto map, auto grid) -> cudaError_t {
-    mixed_image_kernel<decltype(map), decltype(grid), 1><<<grid_for_n(np), kThreads, 0, t->stream>>>(a);
-    return cudaGetLastError();
-  }));
+  ST(mixed_image_launch<1>(t, sc, a));
   count_launches(1);
   *n_points = np;
   return B12G_OK;
@@ -1325,9 +1486,18 @@ b12g_status mixed_rows(b12g_tree* t, const b12g_scheme* sc, int invalid_column)
   a.keep_lost = invalid_column ? 1 : 0;
   a.lost_col = t->n + 1;
   a.n_src = t->n;
+  ST(mixed_screen(t, sc, a));
   CK(dispatch(sc->map.kind, sc->map.arith, sc->grid.kind, t->domain.dim, [&](auto map, auto grid) -> cudaError_t {
-    mixed_rows_kernel<decltype(map), decltype(grid)>
-        <<<std::max(1, std::min<int>(int((t->n + 7) / 8), device_sm_count() * 8)), kThreads, 0, t->stream>>>(a);
+    using Map = decltype(map);
+    using Grid = decltype(grid);
+    const int g = std::max(1, std::min<int>(int((t->n + 7) / 8), device_sm_count() * 8));
+    if constexpr (Screen<Map>::kOk) {
+      if (a.sc.on) {
+        mixed_rows_kernel<Map, Grid, true><<<g, kThreads, 0, t->stream>>>(a);
+        return cudaGetLastError();
+      }
+    }
+    mixed_rows_kernel<Map, Grid, false><<<g, kThreads, 0, t->stream>>>(a);
     return cudaGetLastError();
   }));
   count_launches(1);

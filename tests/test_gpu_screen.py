@@ -163,3 +163,40 @@ def test_batches_and_served_jobs_equal_single_trees(which):
                 assert np.array_equal(x, y)
             t.close()
     b.close()
+
+
+@pytest.mark.parametrize("case,depth", [(0, 4), (0, 24), (0, 50), (1, 21), (2, 17), (3, 20), (4, 13), (4, 25), (5, 16),
+                                        (6, 23), (6, 60), (7, 18)])
+def test_leaves_of_several_depths(case, depth):
+    """A covering with a third of its boxes split once and a third twice."""
+    import b12_b200 as B
+    spec = CASES[case][0]
+    rng = np.random.default_rng([case, depth, 9])
+    base = np.unique(covering(spec, depth, 150, [case, depth]))
+    cut = rng.integers(0, 3, size=len(base))
+    leaves = []
+    for code, c in zip(base, cut):
+        for low in range(1 << int(c)):
+            if c == 0 or rng.random() < 0.7:
+                leaves.append(((int(code) << int(c)) | low, depth + int(c)))
+    codes = np.array([x[0] for x in leaves], dtype=np.uint64)
+    deps = np.array([x[1] for x in leaves], dtype=np.uint8)
+    flags = np.where(rng.random(len(codes)) < 0.5, 8, 0).astype(np.uint8)
+    t = B.ImplicitBoxTree(spec["center"], spec["radius"])
+    t.load_leaves(codes, deps, flags)
+    o = O.Oracle(spec)
+    o.load(codes, deps, flags)
+    sc = scheme(spec)
+    assert np.array_equal(t.search_by_image(sc), o.search_by_image())
+    some = B.Scheme(sc.map, sc.grid, flags_to_check=8)
+    assert np.array_equal(t.search_by_image(some), o.search_by_image(np.nonzero(flags & 8)[0]))
+    m = t.transition_matrix(sc, invalid_column=True)
+    rp, cols, vals, nc = o.transition_matrix(invalid=True)
+    got = m.to_host()
+    assert m.n_cols == nc and np.array_equal(got[0], rp) and np.array_equal(got[1], cols)
+    assert np.array_equal(got[2], vals)
+    for _ in range(2):
+        assert t.set_flags_by_image(sc, B.HIT) == o.set_flags_by_image(1)
+    assert np.array_equal(t.leaves()[2], o.leaves()[2])
+    m.close()
+    t.close()
