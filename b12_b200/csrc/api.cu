@@ -259,9 +259,11 @@ b12g_status select_sources(b12g_tree* t, const b12g_scheme* sc, Prepared& pr, ui
   return B12G_OK;
 }
 
-b12g_status check_error(b12g_tree* t, const char* where)
+b12g_status check_error(b12g_tree* t, const char* where) { return read_checked(t, C_ERROR, 1, where); }
+
+b12g_status read_checked(b12g_tree* t, int first, int count, const char* where)
 {
-  ST(read_ctr(t, C_ERROR, 1));
+  ST(read_ctr(t, first, count));
   if (t->h_ctr[C_ERROR]) {
     const uint32_t e = t->h_ctr[C_ERROR];
     set_ctr(t, C_ERROR, 0);
@@ -274,15 +276,17 @@ b12g_status check_error(b12g_tree* t, const char* where)
 // make the tree the single surrounding box (insertSurroundingBoxIfEmpty)
 b12g_status set_root(b12g_tree* t, uint8_t flags)
 {
-  const uint64_t zero = 0;
-  CK(cudaMemcpyAsync(t->codes(), &zero, 8, cudaMemcpyHostToDevice, t->stream));
+  // (always in the first of the two buffers: a fused run's graph, captured for one of them,
+  // is then the same for the next tree of the handle, whatever the number of steps)
+  t->cur = 0;
+  t->ncur = C_N0;
+  CK(cudaMemsetAsync(t->codes(), 0, 8, t->stream));
   CK(cudaMemsetAsync(t->flg(), flags, 1, t->stream));
   t->n = 1;
   ++t->leaf_gen;
   t->depth = 0;
   t->mixed = false;
-  ST(set_ctr(t, t->ncur, 1));
-  return sync(t, "set root");
+  return set_ctr(t, t->ncur, 1);
 }
 
 b12g_status flag_call(b12g_tree* t, int op, uint8_t u, uint8_t f, uint8_t depth, uint32_t* n_changed)
@@ -421,10 +425,10 @@ b12g_status b12g_tree_create(const b12g_domain* domain, b12g_tree** out)
   fill_domain(*domain, t->dom);
   b12g_status st = B12G_OK;
   if (cudaStreamCreateWithFlags(&t->stream, cudaStreamNonBlocking) != cudaSuccess) st = cuda_fail(cudaGetLastError(), "stream");
-  if (st == B12G_OK && cudaMallocHost(&t->h_ctr, C_COUNT * sizeof(uint32_t)) != cudaSuccess)
+  if (st == B12G_OK && cudaMallocHost(&t->h_ctr, C_ALL * sizeof(uint32_t)) != cudaSuccess)
     st = cuda_fail(cudaGetLastError(), "pinned counters");
-  if (st == B12G_OK) st = t->ctr.ensure(C_COUNT, "counters");
-  if (st == B12G_OK && cudaMemsetAsync(t->ctr.p, 0, C_COUNT * sizeof(uint32_t), t->stream) != cudaSuccess)
+  if (st == B12G_OK) st = t->ctr.ensure(C_ALL, "counters");
+  if (st == B12G_OK && cudaMemsetAsync(t->ctr.p, 0, C_ALL * sizeof(uint32_t), t->stream) != cudaSuccess)
     st = cuda_fail(cudaGetLastError(), "memset");
   if (st == B12G_OK) st = reserve(t, 1024);
   if (st == B12G_OK) st = set_root(t, B12G_NONE);
@@ -454,7 +458,7 @@ b12g_status b12g_tree_destroy(b12g_tree* t)
   t->hit.release(); t->ctr.release(); t->tiles_a.release(); t->tiles_b.release();
   t->src.release(); t->out.release(); t->stage_col.release(); t->stage_cnt.release();
   t->row_count.release(); t->rowptr.release(); t->cand.release(); t->cand2.release();
-  t->sort_idx.release(); t->table.release(); t->step_counts.release(); t->sort_tmp.release();
+  t->sort_idx.release(); t->table.release(); t->snap_code.release(); t->snap_flags.release(); t->sort_tmp.release();
   t->last_tgt.release(); t->last_rank.release(); t->srcc.release(); t->bits.release(); t->pk.release();
   t->route_runs.release(); t->route_cnt.release();
   if (t->h_ctr) cudaFreeHost(t->h_ctr);
@@ -571,7 +575,6 @@ b12g_status b12g_subdivide(b12g_tree* t, uint8_t flags, uint32_t* n_subdivided)
     const int o = 1 - t->cur, no = 1 - t->ncur;
     CK(split_codes(t->codes(), t->flg(), t->dn(), t->code[o].p, t->flags[o].p, t->ctr.p + no, t->n, t->stream));
     count_launches(1);
-    ST(sync(t, "subdivide"));
     t->cur = o;
     ++t->leaf_gen;
     t->ncur = no;
@@ -599,8 +602,7 @@ b12g_status b12g_remove(b12g_tree* t, uint8_t flags, uint32_t* n_removed)
   ca.error = t->ctr.p + C_ERROR;
   CK(compact(ca, {t->tiles_a.p, t->tiles_b.p}, t->n, t->stream));
   count_launches(compact_launches(false, t->n));
-  ST(read_ctr(t, no, 1));
-  ST(check_error(t, "remove"));
+  ST(read_checked(t, C_N0, C_ERROR - C_N0 + 1, "remove"));    // one read-back: both counts and the error word
   const uint32_t kept = t->h_ctr[no];
   const uint32_t removed = t->n - kept;
   t->cur = o;
@@ -657,9 +659,8 @@ b12g_status b12g_set_flags_by_image(b12g_tree* t, const b12g_scheme* sc, uint8_t
   prof_mark(t, 0);
   CK(apply_hits(t->flg(), t->hit.p, t->dn(), flags, t->ctr.p + C_CHANGED, t->n, t->stream));
   count_launches(2);
-  ST(read_ctr(t, C_CHANGED, 1));
+  ST(read_checked(t, C_CHANGED, C_ERROR - C_CHANGED + 1, "set_flags_by_image"));
   ST(prof_collect(t));
-  ST(check_error(t, "set_flags_by_image"));
   if (n_changed) *n_changed = t->h_ctr[C_CHANGED];
   return B12G_OK;
 }
@@ -789,6 +790,12 @@ b12g_status finish_rows(b12g_tree* t, uint32_t P, uint32_t n_cols, int absolute,
   if (st == B12G_OK) st = m->cols.ensure(std::max<uint64_t>(m->nnz, 1), "cols");
   if (st == B12G_OK) st = m->vals.ensure(std::max<uint64_t>(m->nnz, 1), "vals");
   if (st == B12G_OK) st = m->ctr.ensure(256, "csr counters");
+  // the matrix's own stream waits for its rows; a refill waits for the fill before (which
+  // another tree's stream may have queued)
+  if (st == B12G_OK && !m->ready && cudaEventCreateWithFlags(&m->ready, cudaEventDisableTiming) != cudaSuccess)
+    st = cuda_fail(cudaGetLastError(), "event");
+  else if (st == B12G_OK && !fresh && cudaStreamWaitEvent(t->stream, m->ready, 0) != cudaSuccess)
+    st = cuda_fail(cudaGetLastError(), "refill");
   const bool find_lost = invalid_column && nnz32 != 0;
   if (st == B12G_OK && find_lost) st = set_ctr(t, C_TMP, 0);
   if (st == B12G_OK) {
@@ -800,7 +807,10 @@ b12g_status finish_rows(b12g_tree* t, uint32_t P, uint32_t n_cols, int absolute,
       value_present(m->cols.p, nnz32, n_cols + 1, t->ctr.p + C_TMP, t->stream);
       count_launches(1);
     }
-    st = sync(t, "gather rows");
+    if (cudaGetLastError() != cudaSuccess || cudaEventRecord(m->ready, t->stream) != cudaSuccess ||
+        cudaStreamWaitEvent(m->stream, m->ready, 0) != cudaSuccess)
+      st = cuda_fail(cudaGetLastError(), "gather rows");
+    if (st == B12G_OK && t->profile) st = sync(t, "gather rows");      // the timing events are read next
   }
   if (st == B12G_OK && find_lost) {
     st = read_ctr(t, C_TMP, 1);
@@ -846,6 +856,7 @@ b12g_status b12g_csr_destroy(b12g_csr* m)
   m->work.release(); m->tiles.release(); m->tvals.release(); m->w0.release(); m->w1.release();
   m->partial.release(); m->vout.release(); m->ctr.release(); m->vstart.release(); m->change.release();
   m->long_flag.release(); m->long_pos.release(); m->long_list.release(); m->mid_list.release();
+  if (m->ready) cudaEventDestroy(m->ready);
   if (m->stream) cudaStreamDestroy(m->stream);
   delete m;
   return B12G_OK;
@@ -1021,12 +1032,12 @@ b12g_status b12g_subdivision_run(b12g_tree* t, const b12g_scheme* sc, uint32_t s
   // keep the initial state so that a capacity overflow can be retried with more room
   const uint32_t n0 = t->n;
   const uint8_t d0 = t->depth;
-  std::vector<uint64_t> c0(n0);
-  std::vector<uint8_t> f0(n0);
-  CK(cudaMemcpyAsync(c0.data(), t->codes(), size_t(n0) * 8, cudaMemcpyDeviceToHost, t->stream));
-  CK(cudaMemcpyAsync(f0.data(), t->flg(), n0, cudaMemcpyDeviceToHost, t->stream));
-  ST(sync(t, "snapshot"));
-  ST(t->step_counts.ensure(steps + 1, "step counts"));
+  ST(t->snap_code.ensure(n0, "initial leaves"));
+  ST(t->snap_flags.ensure(n0, "initial leaves"));
+  CK(cudaMemcpyAsync(t->snap_code.p, t->codes(), size_t(n0) * 8, cudaMemcpyDeviceToDevice, t->stream));
+  CK(cudaMemcpyAsync(t->snap_flags.p, t->flg(), n0, cudaMemcpyDeviceToDevice, t->stream));
+  // the steps' counts follow the counters, so that one read-back brings both
+  uint32_t* const step_counts = t->ctr.p + C_COUNT;
 
   uint64_t cap = std::max<uint64_t>(t->code[0].n, std::max<uint64_t>(4ull * n0, 1ull << 16));
   t->tgt_ok = false;
@@ -1109,7 +1120,7 @@ b12g_status b12g_subdivision_run(b12g_tree* t, const b12g_scheme* sc, uint32_t s
         ca.out_code = t->code[o].p;
         ca.out_flags = t->flags[o].p;
         ca.n_out = t->ctr.p + no;
-        ca.n_out2 = t->step_counts.p + s;
+        ca.n_out2 = step_counts + s;
         ca.out_cap = uint32_t(std::min<size_t>(t->code[o].n, 0xFFFFFFFFu));
         ca.error = t->ctr.p + C_ERROR;
         ca.out_rank = last ? store_rank : nullptr;
@@ -1138,11 +1149,8 @@ b12g_status b12g_subdivision_run(b12g_tree* t, const b12g_scheme* sc, uint32_t s
     count_launches(t->sub_graph_kernels);
     t->work_turn = steps & 1u;
     if (use_hash) t->hash_tag = steps;
-    std::vector<uint32_t> hc(steps);
-    CK(cudaMemcpyAsync(hc.data(), t->step_counts.p, steps * 4, cudaMemcpyDeviceToHost, t->stream));
-    CK(cudaMemcpyAsync(t->h_ctr + C_ERROR, t->ctr.p + C_ERROR, 4, cudaMemcpyDeviceToHost, t->stream));
-    CK(cudaMemcpyAsync(t->h_ctr + C_TGT, t->ctr.p + C_TGT, 4, cudaMemcpyDeviceToHost, t->stream));
-    ST(sync(t, "subdivision run"));
+    ST(read_ctr(t, C_ERROR, C_COUNT - C_ERROR + int(steps)));
+    std::vector<uint32_t> hc(t->h_ctr + C_COUNT, t->h_ctr + C_COUNT + steps);
     if (t->profile)
       for (int k = 0; k < 2; ++k)
         sum_pairs(t->graph_prof[k], t->graph_prof[k].size(), t->prof_ms[k], t->prof_launches[k]);
@@ -1152,8 +1160,8 @@ b12g_status b12g_subdivision_run(b12g_tree* t, const b12g_scheme* sc, uint32_t s
       cap *= 4;
       ST(reserve(t, cap));
       CK(cudaMemsetAsync(t->hit.p, 0, t->hit.n, t->stream));
-      CK(cudaMemcpyAsync(t->codes(), c0.data(), size_t(n0) * 8, cudaMemcpyHostToDevice, t->stream));
-      CK(cudaMemcpyAsync(t->flg(), f0.data(), n0, cudaMemcpyHostToDevice, t->stream));
+      CK(cudaMemcpyAsync(t->codes(), t->snap_code.p, size_t(n0) * 8, cudaMemcpyDeviceToDevice, t->stream));
+      CK(cudaMemcpyAsync(t->flg(), t->snap_flags.p, n0, cudaMemcpyDeviceToDevice, t->stream));
       ST(set_ctr(t, t->ncur, n0));
       ST(sync(t, "restore"));
       t->n = n0;

@@ -274,8 +274,7 @@ b12g_status insert_points_impl(b12g_tree* t, const double* points, uint64_t n_po
                             pr.a.hash, root_only, hit_flags ? t->hit.p : nullptr, t->cand.p, t->ctr.p + C_CAND,
                             uint32_t(t->cand.n), t->ctr.p + C_ERROR, t->stream));
     count_launches(1);
-    ST(read_ctr(t, C_CAND, 1));
-    ST(check_error(t, "insert_points"));
+    ST(read_checked(t, C_ERROR, C_CAND - C_ERROR + 1, "insert_points"));
     const uint32_t m = t->h_ctr[C_CAND];
     if (!root_only) ST(apply_hit_flags(t, hit_flags));
     ST(sort_unique_candidates(t, m, depth, &u));

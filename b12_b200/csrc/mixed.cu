@@ -1389,8 +1389,9 @@ b12g_status mixed_subdivide(b12g_tree* t, uint8_t flags, uint32_t* n_subdivided)
   split_count_kernel<<<grid_for_n(n), kThreads, 0, t->stream>>>(t->flg(), dep_cur(t), n, flags, t->row_count.p);
   count_launches(2);
   uint32_t total = 0;
+  // (the scan's read-back brings the count too)
+  CK(cudaMemcpyAsync(t->h_ctr + C_CAND, t->ctr.p + C_CAND, 4, cudaMemcpyDeviceToHost, t->stream));
   ST(scan_marks(t, t->row_count.p, t->rowptr.p, n, &total));
-  ST(read_ctr(t, C_CAND, 1));
   if (n_subdivided) *n_subdivided = t->h_ctr[C_CAND];
   if (total == n) return B12G_OK;
   ST(reserve(t, total));
@@ -1404,7 +1405,6 @@ b12g_status mixed_subdivide(b12g_tree* t, uint8_t flags, uint32_t* n_subdivided)
   t->n = total;
   ++t->leaf_gen;
   ST(set_ctr(t, t->ncur, total));
-  ST(sync(t, "subdivide"));
   return mixed_settle(t);
 }
 
@@ -1427,7 +1427,6 @@ b12g_status mixed_remove(b12g_tree* t, uint8_t flags, uint32_t* n_removed)
   t->n = kept;
   ++t->leaf_gen;
   ST(set_ctr(t, t->ncur, kept));
-  ST(sync(t, "remove"));
   if (n_removed) *n_removed = n - kept;
   if (kept == 0) return set_root(t, B12G_NONE);  // insertSurroundingBoxIfEmpty; one depth again
   return mixed_settle(t);
@@ -1585,8 +1584,7 @@ b12g_status mixed_insert_boxes(b12g_tree* t, uint64_t np, uint8_t depth, uint8_t
     count_launches(1);
   }
   if (a.box_hit) ST(apply_box_hits(t, depth, inner, hit, nullptr));
-  ST(read_ctr(t, C_CAND, 1));
-  ST(check_error(t, "insert"));
+  ST(read_checked(t, C_ERROR, C_CAND - C_ERROR + 1, "insert"));
   const uint32_t m = t->h_ctr[C_CAND];
   if (m == 0) return mixed_settle(t);
 

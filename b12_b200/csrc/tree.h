@@ -104,7 +104,8 @@ enum : int {
   C_TGT = 13,      // the stored image targets overflowed their buffer
   C_WORK = 14,     // 2 words: the image kernel's work-queue counters
   C_DEFER = 16,    // error bits of launches whose status is read with a later read-back
-  C_COUNT = 18
+  C_COUNT = 18,
+  C_ALL = C_COUNT + 64   // and the leaf counts after a fused run's steps (at most 64)
 };
 
 }  // namespace host
@@ -133,7 +134,8 @@ struct b12g_tree {
   Buf<uint32_t> sort_idx;
   Buf<double> table;
   Buf<double> points;
-  Buf<uint32_t> step_counts;
+  Buf<uint64_t> snap_code;     // a fused run's initial leaves, kept for a retry with more room
+  Buf<uint8_t> snap_flags;
   Buf<uint8_t> sort_tmp;
   // leaves of different depths: per-leaf depths (with code/flags) and comparable patterns
   bool mixed = false;
@@ -185,6 +187,7 @@ struct b12g_csr {
   template<class T> using Buf = b12g::host::Buf<T>;
   int device = 0;
   cudaStream_t stream = nullptr;
+  cudaEvent_t ready = nullptr;   // the last fill by a tree's stream
   uint32_t n_rows = 0, n_cols = 0;
   uint64_t nnz = 0;
   Buf<uint32_t> rowptr, cols;
@@ -221,6 +224,8 @@ bool stored_rows_fit(b12g_tree* t, const b12g_scheme* sc, const Prepared& pr);
 b12g_status check_depth(b12g_tree* t, uint8_t depth);
 b12g_status select_sources(b12g_tree* t, const b12g_scheme* sc, Prepared& pr, uint32_t& n_src);
 b12g_status check_error(b12g_tree* t, const char* where);
+// read_ctr of a range that holds C_ERROR, and check_error of what it read
+b12g_status read_checked(b12g_tree* t, int first, int count, const char* where);
 // log2 of the lookup-table slots n leaves use (the device's hash_log2)
 uint32_t host_hash_log2(uint64_t n);
 b12g_status set_root(b12g_tree* t, uint8_t flags);
