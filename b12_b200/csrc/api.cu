@@ -783,6 +783,7 @@ b12g_status finish_rows(b12g_tree* t, uint32_t P, uint32_t n_cols, int absolute,
   m->n_cols = n_cols;
   m->nnz = nnz32;
   m->has_transpose = false;
+  m->count_points = absolute ? 1 : P;
   b12g_status st = B12G_OK;
   if (!m->stream && cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) != cudaSuccess)
     st = cuda_fail(cudaGetLastError(), "stream");
@@ -855,6 +856,7 @@ b12g_status b12g_csr_destroy(b12g_csr* m)
   m->rowptr.release(); m->cols.release(); m->vals.release(); m->tptr.release(); m->trows.release();
   m->work.release(); m->tiles.release(); m->tvals.release(); m->w0.release(); m->w1.release();
   m->partial.release(); m->vout.release(); m->ctr.release(); m->vstart.release(); m->change.release();
+  m->pack.release(); m->dlist.release(); m->dcount.release();
   m->long_flag.release(); m->long_pos.release(); m->long_list.release(); m->mid_list.release();
   if (m->ready) cudaEventDestroy(m->ready);
   if (m->stream) cudaStreamDestroy(m->stream);
@@ -890,10 +892,27 @@ b12g_status ensure_transpose(b12g_csr* m)
     ST(m->mid_list.ensure(n + 1, "row classes"));
     CK(max_row_length(m->tptr.p, n, m->ctr.p + 6, s));
     count_launches(7);
-    uint32_t max_row = 0;
-    CK(cudaMemcpyAsync(&max_row, m->ctr.p + 6, 4, cudaMemcpyDeviceToHost, s));
+    // a matrix of counts of a size that fits: its packed form, whose outcome comes back with
+    // the longest row (ctr words 6, and 7 to 9)
+    const bool pack = m->count_points > 0 && m->count_points <= 255 &&
+                      count_plan_possible(m->nnz, n, uint32_t(measure_partial_slots()));
+    if (pack) {
+      ST(m->pack.ensure(m->nnz, "packed matrix"));
+      ST(m->dlist.ensure(size_t(device_sm_count()) * count_distinct_cap(m->nnz), "packed matrix"));
+      ST(m->dcount.ensure(device_sm_count(), "packed matrix"));
+      CK(count_plan(m->tptr.p, m->trows.p, m->tvals.p, n, m->nnz, m->count_points, m->pack.p, m->dlist.p,
+                    m->dcount.p, m->ctr.p + 7, s));
+      count_launches(1);
+    }
+    uint32_t got[4] = {0, 0, 0, 0};
+    CK(cudaMemcpyAsync(got, m->ctr.p + 6, sizeof got, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    if (measure_on_chip(m->nnz, max_row, uint32_t(measure_partial_slots()))) {
+    const uint32_t max_row = got[0];
+    m->plan = CountPlan{};
+    if (pack)
+      m->plan = CountPlan{m->pack.p, m->dlist.p, m->dcount.p, double(m->count_points), got[3], got[2],
+                          count_chunk(m->nnz, max_row, got[1], got[2], got[3])};
+    if (m->plan.chunk || measure_on_chip(m->nnz, max_row, uint32_t(measure_partial_slots()))) {
       // the power iteration keeps the matrix on chip and reads no row-class lists
       m->n_mid = 0;
       m->n_long = 0;
@@ -935,7 +954,7 @@ b12g_status b12g_invariant_measure(b12g_csr* m, uint32_t iters, double* v)
   ST(m->partial.ensure(slots, "measure"));
   CK(invariant_measure(m->tptr.p, m->trows.p, m->tvals.p, m->mid_list.p, m->n_mid, m->long_list.p, m->n_long, n,
                        iters, m->w0.p, m->w1.p, m->partial.p, uint32_t(slots), m->vout.p, m->ctr.p + 64, s,
-                       m->nnz));
+                       m->nnz, nullptr, nullptr, &m->plan));
   count_launches(1);
   if (v) CK(cudaMemcpyAsync(v, m->vout.p, size_t(n) * 8, cudaMemcpyDeviceToHost, s));
   uint32_t err = 0;
@@ -975,7 +994,7 @@ b12g_status b12g_invariant_measure_tol(b12g_csr* m, double tol, uint32_t max_ite
     CK(cudaMemsetAsync(m->change.p, 0, size_t(nchg) * 8, s));
     CK(invariant_measure(m->tptr.p, m->trows.p, m->tvals.p, m->mid_list.p, m->n_mid, m->long_list.p, m->n_long, n,
                          k, m->w0.p, m->w1.p, m->partial.p, uint32_t(slots), m->vout.p, m->ctr.p + 64, s, m->nnz,
-                         start, m->change.p));
+                         start, m->change.p, &m->plan));
     count_launches(1);
     uint32_t err = 0;
     CK(cudaMemcpyAsync(chg.data(), m->change.p, size_t(nchg) * 8, cudaMemcpyDeviceToHost, s));

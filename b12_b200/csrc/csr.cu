@@ -9,6 +9,7 @@
 //                        matrix on chip, bounded waits between dependent blocks)
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "kernels.h"
@@ -613,6 +614,300 @@ __global__ void __launch_bounds__(kMeasureThreads, 1) invariant_measure_smem_ker
   write_result(a, inv, inv_prev);
 }
 
+// ---- power iteration on a matrix of counts ------------------------------------------------
+// A transition matrix holds counts of test points over their number, RN(c / P).  An entry
+// then fits 32 bits - the source's place among the block's distinct sources (16), the count
+// (8), the end of a row (1) and the empty rows that follow it (7) - against 16 bytes in the
+// kernel above, so four times as many entries stay on chip, and an iteration gathers each
+// distinct source once (a block's 10,900 entries have about 2,000 at depth 27) and takes the
+// rest from shared memory.  The values come from a table of RN(c / P), and the entries are
+// split over the threads as above: the same operations in the same order, so the measure has
+// the same bits.  count_plan_kernel packs the entries and lists every block's distinct
+// sources in increasing order, once per matrix.
+constexpr uint32_t kCountEnd = 1u << 24;
+constexpr uint32_t kCountMaxChunk = 52;        // entries a thread
+constexpr uint32_t kCountMaxRows = 1200000;    // bits and 16-bit ranks of the sources in the plan's shared memory
+constexpr size_t kCountSmemLimit = 227 * 1024 - 2560;   // dynamic bytes beside the static ones
+
+// per block: its distinct sources (dlist[b * cap ..], dcount[b]); flags: {bit 0: a block or
+// an entry does not fit, most distinct sources of a block, largest count}
+__global__ void __launch_bounds__(kMeasureThreads, 1) count_plan_kernel(const uint32_t* tptr, const uint32_t* trows,
+                                                                        const double* tvals, uint32_t n, uint32_t nnz,
+                                                                        double points, uint32_t cap,
+                                                                        uint32_t* pack, uint32_t* dlist,
+                                                                        uint32_t* dcount, uint32_t* flags)
+{
+  extern __shared__ __align__(16) unsigned char smem[];
+  const uint32_t words = (n + 31) / 32;
+  uint32_t* s_bits = reinterpret_cast<uint32_t*>(smem);
+  uint16_t* s_rank = reinterpret_cast<uint16_t*>(s_bits + words);
+  __shared__ uint32_t s_edge[2];
+  __shared__ uint32_t s_warp[kMeasureThreads / 32];
+  const uint32_t t = threadIdx.x, lane = t & 31;
+  const uint32_t per = (nnz + gridDim.x - 1) / gridDim.x;
+  if (t < 2) s_edge[t] = blockIdx.x + t == gridDim.x ? n : min(lower_bound_u32(tptr, n + 1, (blockIdx.x + t) * per), n);
+  for (uint32_t w = t; w < words; w += blockDim.x) s_bits[w] = 0u;
+  __syncthreads();
+  const uint32_t r0 = s_edge[0], r1 = max(r0, s_edge[1]);
+  const uint32_t e0 = __ldg(tptr + r0), e1 = __ldg(tptr + r1);
+  bool ok = e1 - e0 <= kCountMaxChunk * kMeasureThreads;
+  for (uint32_t k = e0 + t; k < e1; k += blockDim.x) {
+    const uint32_t s = __ldg(trows + k), m = 1u << (s & 31u);
+    if (!(s_bits[s >> 5] & m)) atomicOr(s_bits + (s >> 5), m);
+  }
+  __syncthreads();
+  // ranks: every thread's words are consecutive
+  const uint32_t per_t = (words + blockDim.x - 1) / blockDim.x;
+  const uint32_t w0 = min(t * per_t, words), w1 = min(w0 + per_t, words);
+  uint32_t c = 0;
+  for (uint32_t w = w0; w < w1; ++w) c += __popc(s_bits[w]);
+  uint32_t x = c;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, d);
+    if (lane >= uint32_t(d)) x += y;
+  }
+  if (lane == 31) s_warp[t >> 5] = x;
+  __syncthreads();
+  uint32_t before = x - c, total = 0;
+  for (uint32_t w = 0; w < blockDim.x / 32; ++w) {
+    const uint32_t y = s_warp[w];
+    before += w < (t >> 5) ? y : 0u;
+    total += y;
+  }
+  ok = ok && total <= cap && total <= 65535u;
+  if (t == 0) {
+    dcount[blockIdx.x] = total;
+    atomicMax(flags + 1, total);
+  }
+  for (uint32_t w = w0; w < w1; ++w) {
+    uint32_t b = s_bits[w];
+    s_rank[w] = uint16_t(before);
+    while (b) {
+      const int bit = __ffs(b) - 1;
+      if (before < cap) dlist[size_t(blockIdx.x) * cap + before] = 32u * w + uint32_t(bit);
+      ++before;
+      b &= b - 1u;
+    }
+  }
+  __syncthreads();
+  uint32_t most = 0;
+  // a thread a row: its entries, and at the last one the empty rows behind it
+  for (uint32_t r = r0 + t; r < r1; r += blockDim.x) {
+    const uint32_t b = __ldg(tptr + r), e = __ldg(tptr + r + 1);
+    if (b == e) continue;
+    uint32_t skip = 0;
+    while (r + 1 + skip < r1 && __ldg(tptr + r + 2 + skip) == e && skip < 128) ++skip;
+    if (skip > 127) { ok = false; skip = 127; }
+    for (uint32_t k = b; k < e; ++k) {
+      const uint32_t s = __ldg(trows + k);
+      const double v = __ldg(tvals + k);
+      const double cd = rint(__dmul_rn(v, points));
+      const bool exact = cd >= 1.0 && cd <= 255.0 && __ddiv_rn(cd, points) == v;
+      ok = ok && exact;
+      const uint32_t id = s_rank[s >> 5] + __popc(s_bits[s >> 5] & ((1u << (s & 31u)) - 1u));
+      most = max(most, exact ? uint32_t(cd) : 0u);
+      pack[k] = (id & 0xFFFFu) | (exact ? uint32_t(cd) << 16 : 0u) | (k + 1 == e ? kCountEnd | skip << 25 : 0u);
+    }
+  }
+  if (!ok) atomicOr(flags, 1u);
+  most = __reduce_max_sync(0xFFFFFFFFu, most);
+  if (lane == 0 && most) atomicMax(flags + 2, most);
+}
+
+// The same iteration from the packed entries.  Thread t's run is entries [t run, (t + 1) run)
+// of the block, run = entries / threads rounded up, four to a 16-byte word, word g of all
+// threads side by side (conflict-free reads); the places past a run's entries are zero: a
+// count of 0, value 0, of the first source.
+// Everything else - the rows split over runs, the normalising iterations, the waits - is
+// invariant_measure_smem_kernel's.  Bound by the latency of an iteration's chain: the wait
+// for the blocks it depends on, one gather, the walk over shared memory (a random 8-byte
+// read an entry), the release.
+__global__ void __launch_bounds__(kMeasureThreads, 1) invariant_measure_count_kernel(MeasureArgs a, uint32_t nnz,
+                                                                                     const uint32_t* pack,
+                                                                                     const uint32_t* dlist,
+                                                                                     const uint32_t* dcount,
+                                                                                     uint32_t cap, uint32_t chunk,
+                                                                                     double points, uint32_t counts)
+{
+  extern __shared__ __align__(16) unsigned char smem[];
+  uint4* s_ent = reinterpret_cast<uint4*>(smem);
+  uint32_t* s_ent1 = reinterpret_cast<uint32_t*>(smem);
+  double* s_val = reinterpret_cast<double*>(smem + size_t(chunk) * kMeasureThreads * 4);   // RN(c / P), c < counts
+  double* s_v = s_val + counts;
+  // after an iteration's walk the staged values' place holds the runs' first parts
+  double* s_head = s_v;
+  uint32_t* s_head_end = reinterpret_cast<uint32_t*>(s_v + kMeasureThreads);
+  __shared__ double red[kMeasureThreads / 32];
+  __shared__ uint32_t s_bnd[32 * kDepWords + 1];
+  __shared__ uint32_t s_dep[kDepWords];
+  const uint32_t n = a.n;
+  const uint32_t t = threadIdx.x, lane = t & 31;
+  const uint32_t per = (nnz + gridDim.x - 1) / gridDim.x;
+  if (t <= gridDim.x) s_bnd[t] = t == gridDim.x ? n : min(lower_bound_u32(a.tptr, n + 1, t * per), n);
+  if (t < kDepWords) s_dep[t] = 0u;
+  __syncthreads();
+  const uint32_t r0 = s_bnd[blockIdx.x], r1 = max(r0, s_bnd[blockIdx.x + 1]);
+  const uint32_t e0 = __ldg(a.tptr + r0), e1 = __ldg(a.tptr + r1);
+  const uint32_t nd = __ldg(dcount + blockIdx.x);
+  const uint32_t* list = dlist + size_t(blockIdx.x) * cap;
+  uint32_t nloc = e1 - e0;
+  if (nloc > chunk * kMeasureThreads) {
+    // more entries than the host planned for: flag it and take part in the barriers only
+    if (t == 0) atomicOr(a.error, 4u);
+    nloc = 0;
+  }
+  for (uint32_t c = t; c < counts; c += blockDim.x) s_val[c] = __ddiv_rn(double(c), points);
+  const uint32_t run = (nloc + kMeasureThreads - 1) / kMeasureThreads;
+  for (uint32_t k = t; k < chunk * kMeasureThreads; k += blockDim.x) {
+    const uint32_t owner = k / chunk, q = k - owner * chunk, e = owner * run + q;
+    s_ent1[((q >> 2) * kMeasureThreads + owner) * 4 + (q & 3u)] = q < run && e < nloc ? __ldg(pack + e0 + e) : 0u;
+  }
+  for (uint32_t r = r0 + t; r < r1; r += blockDim.x)
+    if (__ldg(a.tptr + r) == __ldg(a.tptr + r + 1)) { a.w0[r] = 0.0; a.w1[r] = 0.0; }   // no entries: 0 in every iterate
+  const uint32_t k0 = min(t * run, nloc), k1 = min(k0 + run, nloc);
+  const bool any = k0 < k1;
+  const bool head_open = any && k0 > 0 && !(__ldg(pack + e0 + k0 - 1) & kCountEnd);
+  const bool tail_open = any && !(__ldg(pack + e0 + k1 - 1) & kCountEnd);
+  // the row holding this run's first entry: the last row starting at or before it
+  uint32_t row0 = 0;
+  if (any) {
+    uint32_t lo = r0, len = r1 - r0;
+    while (len > 0) {
+      const uint32_t half = len >> 1;
+      if (__ldg(a.tptr + lo + half) <= e0 + k0) { lo += half + 1; len -= half + 1; }
+      else len = half;
+    }
+    row0 = lo - 1;
+  }
+  // the blocks owning this block's sources, published for the blocks whose rows they are
+  {
+    uint32_t m[kDepWords] = {};
+    for (uint32_t k = t; k < nd; k += blockDim.x) {
+      const uint32_t o = owner_block(s_bnd, gridDim.x, __ldg(list + k));
+#pragma unroll
+      for (int w = 0; w < kDepWords; ++w) m[w] |= (o >> 5) == uint32_t(w) ? 1u << (o & 31u) : 0u;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int w = 0; w < kDepWords; ++w) {
+      m[w] = __reduce_or_sync(0xFFFFFFFFu, m[w]);
+      if (lane == 0 && m[w]) atomicOr(s_dep + w, m[w]);
+    }
+  }
+  __syncthreads();
+  if (t < kDepWords) a.dep_mask[blockIdx.x * kDepWords + t] = s_dep[t];
+  if (t == 0) a.epoch[blockIdx.x * kEpochStride] = 0u;
+  uint32_t bars = 0;         // full barriers passed
+  if (!barrier_wait(a, bars++)) return;
+  const uint32_t me = blockIdx.x;
+  const bool waits = t < gridDim.x && t != me &&
+                     (((s_dep[t >> 5] >> (t & 31u)) & 1u) ||
+                      ((__ldcg(a.dep_mask + t * kDepWords + (me >> 5)) >> (me & 31u)) & 1u));
+  const double v0 = __ddiv_rn(1.0, double(n));
+  double inv = 1.0, inv_prev = 1.0;
+  uint32_t norms = 0;        // normalising iterations done: their partial sums alternate slots
+  bool after_barrier = true;
+  for (uint32_t it = 0; it < a.iters; ++it) {
+    const double* wp = (it & 1u) ? a.w0 : a.w1;
+    double* wc = (it & 1u) ? a.w1 : a.w0;
+    double local = 0.0;
+    if (!after_barrier && !epoch_wait(a, waits, it)) return;
+    // stage the distinct sources (the last iterate, scaled when its norm was summed)
+    const bool scale = it > 0 && measure_normalises(it - 1, a.iters);
+    if (scale) {
+      const double s_prev = barrier_total(a.partial + ((norms - 1u) & 1u) * gridDim.x);
+      inv_prev = inv;
+      inv = __ddiv_rn(1.0, s_prev);
+    }
+    for (uint32_t k = t; k < nd; k += 4 * kMeasureThreads) {
+      double v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t j = k + q * kMeasureThreads;
+        v[q] = 0.0;
+        if (j < nd) {
+          const uint32_t src = __ldg(list + j);
+          v[q] = it == 0 ? (a.start ? __ldg(a.start + src) : v0) : __ldcg(wp + src);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t j = k + q * kMeasureThreads;
+        if (j < nd) s_v[j] = scale ? __dmul_rn(v[q], inv) : v[q];
+      }
+    }
+    __syncthreads();
+    // walk the run: a row that ends inside it is written here unless it began earlier
+    uint32_t row = row0;
+    double acc = 0.0, head = 0.0;
+    bool first = true;
+    if (any) {
+      for (uint32_t g = 0; g < (run + 3) / 4; ++g) {
+        const uint4 e4 = s_ent[g * kMeasureThreads + t];
+        const uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
+        double v[4], c[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          v[q] = s_v[e[q] & 0xFFFFu];
+          c[q] = s_val[(e[q] >> 16) & 0xFFu];
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          acc = __fma_rn(c[q], v[q], acc);
+          if (e[q] & kCountEnd) {
+            if (first && head_open) head = acc;
+            else { __stcg(wc + row, acc); local = __dadd_rn(local, fabs(acc)); }
+            first = false;
+            row += 1u + (e[q] >> 25);
+            acc = 0.0;
+          }
+        }
+      }
+    }
+    __syncthreads();
+    if (any && head_open) {
+      // (a run inside one row has its whole sum in acc and leaves the row open)
+      s_head[t] = first ? acc : head;
+      s_head_end[t] = first && tail_open ? 0u : 1u;
+    }
+    __syncthreads();
+    if (any && tail_open && !(first && head_open)) {
+      // this run holds the row's first entry: add the later runs' parts in order
+      double sum = acc;
+      for (uint32_t j = t + 1; j < blockDim.x; ++j) {
+        sum = __dadd_rn(sum, s_head[j]);
+        if (s_head_end[j]) break;
+      }
+      __stcg(wc + row, sum);
+      local = __dadd_rn(local, fabs(sum));
+    }
+    if (measure_normalises(it, a.iters)) {
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) local = __dadd_rn(local, __shfl_xor_sync(0xFFFFFFFFu, local, d));
+      if (lane == 0) red[t >> 5] = local;
+      __syncthreads();
+      if (t == 0) {
+        double sum = 0.0;
+        for (int i = 0; i < kMeasureThreads / 32; ++i) sum = __dadd_rn(sum, red[i]);
+        __stcg(a.partial + (norms & 1u) * gridDim.x + blockIdx.x, sum);
+      }
+      if (!barrier_wait(a, bars++)) return;
+      ++norms;
+      after_barrier = true;
+    } else {
+      epoch_publish(a, it + 1u);
+      after_barrier = false;
+    }
+  }
+  if (a.iters) {
+    const double s_last = barrier_total(a.partial + ((norms - 1u) & 1u) * gridDim.x);
+    inv_prev = inv;
+    inv = __ddiv_rn(1.0, s_last);
+  }
+  write_result(a, inv, inv_prev);
+}
+
 // the rows of P^T of one length class (1: medium, 2: long), ascending (flag, scan, scatter)
 __device__ __forceinline__ uint32_t row_class(const uint32_t* tptr, uint32_t j)
 {
@@ -677,6 +972,7 @@ namespace {
 struct MeasureLaunch
 {
   bool smem_ok;        // the shared-memory kernel may take kSmemMeasureBytes and fits one block per SM
+  bool count_ok;       // the same of the counts' kernels and kCountSmemLimit
   int blocks_per_sm;   // resident blocks per SM of the L2 kernel
 };
 
@@ -691,7 +987,7 @@ MeasureLaunch g_measure_cfg[64];
 MeasureLaunch measure_launch()
 {
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); return {false, 1}; }
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); return {false, false, 1}; }
   std::lock_guard<std::mutex> lock(g_measure_mu);
   if (!g_measure_ready[dev]) {
     int b = 0;
@@ -700,6 +996,14 @@ MeasureLaunch measure_launch()
                                      int(kSmemMeasureBytes)) == cudaSuccess &&
                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, invariant_measure_smem_kernel, kMeasureThreads,
                                                               kSmemMeasureBytes) == cudaSuccess && b >= 1;
+    cudaGetLastError();
+    b = 0;
+    c.count_ok = cudaFuncSetAttribute(invariant_measure_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      int(kCountSmemLimit)) == cudaSuccess &&
+                 cudaFuncSetAttribute(count_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      int(kCountSmemLimit)) == cudaSuccess &&
+                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, invariant_measure_count_kernel, kMeasureThreads,
+                                                               kCountSmemLimit) == cudaSuccess && b >= 1;
     cudaGetLastError();
     b = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, invariant_measure_kernel, kMeasureThreads, 0);
@@ -725,6 +1029,52 @@ bool measure_on_chip(uint64_t nnz, uint32_t max_row, uint32_t partial_cap)
          blocks <= 32u * kDepWords && slots <= partial_cap;
 }
 
+uint32_t count_distinct_cap(uint64_t nnz)
+{
+  const uint64_t blocks = uint64_t(device_sm_count());
+  return uint32_t(std::min<uint64_t>((nnz + blocks - 1) / blocks + kMidRow, 16384));
+}
+
+bool count_plan_possible(uint64_t nnz, uint32_t n, uint32_t partial_cap)
+{
+  const uint32_t blocks = uint32_t(device_sm_count());
+  const uint64_t slots = 2ull * blocks + 2 + (uint64_t(blocks) * kEpochStride + uint64_t(kDepWords) * blocks + 1) / 2;
+  return measure_launch().count_ok && nnz > 0 && n <= kCountMaxRows && blocks <= 32u * kDepWords &&
+         slots <= partial_cap &&
+         (nnz + blocks - 1) / blocks + kMidRow <= uint64_t(kCountMaxChunk) * kMeasureThreads;
+}
+
+cudaError_t count_plan(const uint32_t* tptr, const uint32_t* trows, const double* tvals, uint32_t n, uint64_t nnz,
+                       uint32_t points, uint32_t* pack, uint32_t* dlist, uint32_t* dcount, uint32_t* flags,
+                       cudaStream_t s)
+{
+  cudaMemsetAsync(flags, 0, 3 * sizeof(uint32_t), s);
+  const size_t words = (size_t(n) + 31) / 32;
+  count_plan_kernel<<<device_sm_count(), kMeasureThreads, words * 6 + 16, s>>>(
+      tptr, trows, tvals, n, uint32_t(nnz), double(points), count_distinct_cap(nnz), pack, dlist, dcount, flags);
+  return cudaGetLastError();
+}
+
+namespace {
+
+size_t count_bytes(uint32_t chunk, uint32_t distinct, uint32_t counts)
+{
+  return size_t(chunk) * kMeasureThreads * 4 + size_t(counts) * 8 +
+         std::max<size_t>(size_t(distinct) * 8, size_t(kMeasureThreads) * 12);
+}
+
+}  // namespace
+
+uint32_t count_chunk(uint64_t nnz, uint32_t max_row, uint32_t flags, uint32_t distinct, uint32_t largest)
+{
+  const uint32_t blocks = uint32_t(device_sm_count());
+  if (flags != 0 || max_row > kMidRow) return 0;
+  // a block's rows begin in its share of the entries and have at most kMidRow entries
+  const uint64_t most = (nnz + blocks - 1) / blocks + kMidRow;
+  const uint32_t chunk = uint32_t((most + 4 * kMeasureThreads - 1) / (4 * kMeasureThreads)) * 4;
+  return chunk <= kCountMaxChunk && count_bytes(chunk, distinct, largest + 1) <= kCountSmemLimit ? chunk : 0;
+}
+
 cudaError_t max_row_length(const uint32_t* tptr, uint32_t n, uint32_t* out, cudaStream_t s)
 {
   cudaMemsetAsync(out, 0, sizeof(uint32_t), s);
@@ -736,13 +1086,27 @@ cudaError_t invariant_measure(const uint32_t* tptr, const uint32_t* trows, const
                               const uint32_t* mid_list, uint32_t n_mid, const uint32_t* long_list, uint32_t n_long,
                               uint32_t n, uint32_t iters, double* w0, double* w1, double* partial,
                               uint32_t partial_cap, double* out, unsigned* sync_words, cudaStream_t s, uint64_t nnz,
-                              const double* start, double* change)
+                              const double* start, double* change, const CountPlan* plan)
 {
   // the matrix on chip: one block per SM, every block's rows within its shared memory
   // (a row of P^T has at most kMidRow entries when there are no long rows)
   const MeasureLaunch cfg = measure_launch();
   const uint32_t blocks = uint32_t(device_sm_count());
   const uint32_t epoch_words = blocks * kEpochStride;
+  if (plan && plan->chunk) {
+    cudaMemsetAsync(sync_words, 0, 65 * sizeof(unsigned), s);
+    unsigned* words = reinterpret_cast<unsigned*>(partial + 2 * size_t(blocks) + 2);
+    MeasureArgs a{tptr, trows, tvals, nullptr, 0u, nullptr, 0u, kShortRow, n, iters, w0, w1, partial, out,
+                  sync_words, sync_words + 32, sync_words + 64, partial + 2 * size_t(blocks), 0u, start, change,
+                  words, words + epoch_words};
+    uint32_t nnz32 = uint32_t(nnz), cap = count_distinct_cap(nnz), chunk = plan->chunk;
+    const uint32_t *pack = plan->pack, *dlist = plan->dlist, *dcount = plan->dcount;
+    double points = plan->points;
+    uint32_t counts = plan->largest + 1;
+    void* params[] = {&a, &nnz32, &pack, &dlist, &dcount, &cap, &chunk, &points, &counts};
+    return cudaLaunchCooperativeKernel((const void*)invariant_measure_count_kernel, dim3(blocks), dim3(kMeasureThreads),
+                                       params, count_bytes(chunk, plan->distinct, counts), s);
+  }
   if (mid_list && long_list && n_long == 0 && measure_on_chip(nnz, 0u, partial_cap)) {
     cudaMemsetAsync(sync_words, 0, 65 * sizeof(unsigned), s);
     unsigned* words = reinterpret_cast<unsigned*>(partial + 2 * size_t(blocks) + 2);

@@ -8,6 +8,8 @@
 // "[" + "\n    value" items separated by "," + "\n  ]", then "\n}" (the matrix writer
 // leaves a "," after its last entry, as the reference's does).  Doubles carry 17
 // significant digits (max_digits10), integers are decimal.  Host code only.
+#include <algorithm>
+#include <cmath>
 #include <cerrno>
 #include <cinttypes>
 #include <cstdio>
@@ -355,6 +357,30 @@ b12g_status b12g_csr_save_json(const b12g_csr* m, const char* path)
   return write_coo(with_extension(path), m->n_rows, m->n_cols, rowptr.data(), cols.data(), vals.data());
 }
 
+}  // extern "C"
+
+namespace {
+
+// the smallest P <= 255 over which the first values are counts RN(c / P), c = 1..255, as a
+// saved transition matrix's are; 0: none.  (Only a hint: the packing checks every value.)
+uint32_t counts_over(const std::vector<double>& vals)
+{
+  const size_t n = std::min<size_t>(vals.size(), 1024);
+  for (uint32_t p = 1; n && p <= 255; ++p) {
+    size_t i = 0;
+    for (; i < n; ++i) {
+      const double c = std::rint(vals[i] * double(p));
+      if (!(c >= 1.0 && c <= 255.0 && c / double(p) == vals[i])) break;
+    }
+    if (i == n) return p;
+  }
+  return 0;
+}
+
+}  // namespace
+
+extern "C" {
+
 b12g_status b12g_csr_load_json(const char* path, b12g_csr** out)
 {
   if (!path || !out) return fail(B12G_ERR_INVALID, "NULL argument");
@@ -367,6 +393,7 @@ b12g_status b12g_csr_load_json(const char* path, b12g_csr** out)
   m->n_rows = uint32_t(f.n_rows);
   m->n_cols = uint32_t(f.n_cols);
   m->nnz = f.vals.size();
+  m->count_points = counts_over(f.vals);
   b12g_status st = B12G_OK;
   if (cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) != cudaSuccess)
     st = cuda_fail(cudaGetLastError(), "stream");

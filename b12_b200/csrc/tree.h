@@ -6,6 +6,7 @@
 #include <string>
 #include <vector>
 
+#include "csr.h"
 #include "kernels.h"
 
 namespace b12g {
@@ -199,6 +200,11 @@ struct b12g_csr {
   Buf<double> vstart, change;   // tolerance-driven runs: the iterate carried between launches, change partials
   Buf<uint32_t> ctr;
   bool has_transpose = false;
+  // transition matrices: the values are counts over count_points (0: not known to be).
+  // plan: their packed form for the invariant measure (with the transpose)
+  uint32_t count_points = 0;
+  Buf<uint32_t> pack, dlist, dcount;
+  b12g::CountPlan plan;
 };
 
 namespace b12g {
