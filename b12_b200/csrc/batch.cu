@@ -364,8 +364,7 @@ __global__ void __launch_bounds__(256, 4) batch_screen_kernel(const BatchArgs a)
           if (p != kInvalidIndex) t = 2u * p + uint32_t(tcode & 1u);
         }
       }
-      const unsigned peers = __match_any_sync(0xFFFFFFFFu, t);
-      if (active && t < kOutsideIndex && lane == __ffs(peers) - 1) a.hit[t] = 1;
+      if (t < kOutsideIndex) a.hit[t] = 1;
       if (a.targets && active) {
         const uint64_t base = __ldg(a.tgt_base + inst);
         if (base != ~0ull) a.targets[base + (uint64_t(child) - 2ull * off_s[inst]) * P + k] = t;

@@ -165,12 +165,13 @@ __device__ __forceinline__ bool load_points(const GridParams& g, uint64_t P, dou
 }
 
 // Bound by instruction issue: an FP64 instruction holds its scheduler for two cycles and
-// any other for one.  kScreen: the screened evaluation (screen.cuh), 735 FP64 and 364 other
-// instructions per 32 Lorenz points against 942 and 290 (FMA) or 1,600 (strict); the image
-// launches of a depth-27 job take 5.81 ms against 6.58 (FMA) and 10.21 (strict).  Its state
-// needs 48 registers: five blocks an SM (six, with spills, 5.99 ms; four 6.02 ms).
+// any other for one.  kScreen: the screened evaluation (screen.cuh), 735 FP64 and about 330
+// other instructions per 32 Lorenz points against 942 and 290 (FMA) or 1,600 (strict); the
+// image launches of a depth-27 job take 5.52 ms against 6.58 (FMA) and 10.21 (strict).  Four
+// blocks an SM, 64 registers: the coefficients stay in registers over the unrolled steps
+// (five blocks with 48: 5.72 ms, three: 5.52).
 template<class Map, class Grid, ImageMode M, bool kScreen>
-__global__ void __launch_bounds__(kThreads, kScreen ? 5 : 6) image_points_kernel(const ImageArgs a)
+__global__ void __launch_bounds__(kThreads, kScreen ? 4 : 6) image_points_kernel(const ImageArgs a)
 {
   using PI = PointImage<Map, Grid>;
   __shared__ double pts[kPointTable];
@@ -221,9 +222,9 @@ __global__ void __launch_bounds__(kThreads, kScreen ? 5 : 6) image_points_kernel
       if constexpr (M != ImageMode::Mark) t = PI::target(a, n, valid, tbits);
     }
     if constexpr (M == ImageMode::Hit) {
-      // one store per distinct target in the warp
-      const unsigned peers = __match_any_sync(0xFFFFFFFFu, t);
-      if (active && t != kInvalidIndex && lane == __ffs(peers) - 1) a.hit[t] = 1;
+      // (a store of all lanes: the warp's few distinct bytes leave the SM as so many sectors
+      // either way, and finding one lane for each cost more than it saved)
+      if (t != kInvalidIndex) a.hit[t] = 1;
       if (a.targets && active) {
         if (g < a.targets_cap) a.targets[g] = valid ? t : kOutsideIndex;
         else *a.targets_over = 1;
@@ -232,23 +233,26 @@ __global__ void __launch_bounds__(kThreads, kScreen ? 5 : 6) image_points_kernel
       if (active) a.out[g] = t;
     } else if constexpr (M == ImageMode::Mark) {
       // the image's box, unless its bit is set already (a stale read only sends the point
-      // on to the atomic), deduplicated within the warp; the lane whose atomic sets the bit
-      // marks the box in `fresh`, and the warp counts its new boxes with one atomic
-      uint64_t code = kInvalidCode;
+      // on to the atomic), deduplicated within the warp: most warps find no new box.  The lane
+      // whose atomic sets the bit marks the box in `fresh`, and the warp counts its new boxes
+      // with one atomic.
+      uint32_t code = 0;
       bool fresh = false;
       if (active && valid) {
-        code = code_of_bits<Map::D>(a.dc, tbits, a.depth);
-        fresh = !((a.bits[code >> 5] >> uint32_t(code & 31u)) & 1u);
+        code = uint32_t(code_of_bits<Map::D>(a.dc, tbits, a.depth));
+        fresh = !((a.bits[code >> 5] >> (code & 31u)) & 1u);
       }
-      const unsigned peers = __match_any_sync(0xFFFFFFFFu, fresh ? code : kInvalidCode) & __ballot_sync(0xFFFFFFFFu, fresh);
-      bool leader = fresh && lane == __ffs(peers) - 1;
-      if (leader) {
-        const uint32_t m = 1u << uint32_t(code & 31u);
-        leader = !(atomicOr(a.bits + (code >> 5), m) & m);
-        if (leader) atomicOr(a.fresh + (code >> 5), m);
+      if (__any_sync(0xFFFFFFFFu, fresh)) {
+        const unsigned peers = __match_any_sync(0xFFFFFFFFu, fresh ? code : ~0u) & __ballot_sync(0xFFFFFFFFu, fresh);
+        fresh = fresh && lane == __ffs(peers) - 1;
+        if (fresh) {
+          const uint32_t m = 1u << (code & 31u);
+          fresh = !(atomicOr(a.bits + (code >> 5), m) & m);
+          if (fresh) atomicOr(a.fresh + (code >> 5), m);
+        }
+        const unsigned lead_mask = __ballot_sync(0xFFFFFFFFu, fresh);
+        if (lane == 0 && lead_mask) atomicAdd(a.cand_count, uint32_t(__popc(lead_mask)));
       }
-      const unsigned lead_mask = __ballot_sync(0xFFFFFFFFu, leader);
-      if (lane == 0 && lead_mask) atomicAdd(a.cand_count, uint32_t(__popc(lead_mask)));
     } else {
       // candidates: valid images that are not leaves, as packed keys (the caller turns them
       // into codes); deduplicated within the warp and appended with one atomic per warp

@@ -176,6 +176,12 @@ __device__ __forceinline__ void screen_track(float& m, double x)
 {
   asm("max.NaN.f32 %0, %0, %1;" : "+f"(m) : "f"(fabsf(__int_as_float(__double2hiint(x)))));
 }
+// of two values in one instruction
+__device__ __forceinline__ float screen_high(double x) { return __int_as_float(__double2hiint(x)); }
+__device__ __forceinline__ void screen_track2(float& m, float x, float y)
+{
+  asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(x), "f"(y));
+}
 #endif
 
 // maps with a screened evaluation: run() advances X over the map's steps and returns
@@ -194,11 +200,20 @@ template<class A> struct Screen<LorenzMap<A>> {
   static __device__ __forceinline__ bool run(const double* k, const float* lim, const MapParams& map, double (&x)[3])
   {
     float m0 = 0.f, m1 = 0.f, m2 = 0.f;
-#pragma unroll 4
-    for (uint32_t i = 0; i < map.steps; ++i) {
+    if (map.steps & 1u) {
       screen_track(m0, x[0]);
       screen_track(m1, x[1]);
       screen_track(m2, x[2]);
+      lorenz_screen_step(k, x);
+    }
+    // twenty steps a trip (the usual number): the coefficients are loaded once for them
+#pragma unroll 10
+    for (uint32_t i = map.steps >> 1; i > 0; --i) {
+      const float h0 = screen_high(x[0]), h1 = screen_high(x[1]), h2 = screen_high(x[2]);
+      lorenz_screen_step(k, x);
+      screen_track2(m0, h0, screen_high(x[0]));
+      screen_track2(m1, h1, screen_high(x[1]));
+      screen_track2(m2, h2, screen_high(x[2]));
       lorenz_screen_step(k, x);
     }
     return m0 <= lim[0] && m1 <= lim[1] && m2 <= lim[2];
@@ -242,14 +257,26 @@ template<> struct Screen<ForcedDuffingMap> {
   {
     float m0 = 0.f, m1 = 0.f;
     double f0 = __dmul_rn(k[3], __ldg(map.table));
-#pragma unroll 2
-    for (uint32_t i = 0; i < map.steps; ++i) {
-      const double f1 = __dmul_rn(k[3], __ldg(map.table + 2 * i + 1));
-      const double f2 = __dmul_rn(k[3], __ldg(map.table + 2 * i + 2));
-      screen_track(m0, x[0]);
-      screen_track(m1, x[1]);
+    const double* tab = map.table;
+    auto step = [&]() {
+      const double f1 = __dmul_rn(k[3], __ldg(tab + 1));
+      const double f2 = __dmul_rn(k[3], __ldg(tab + 2));
       forced_screen_step(k, f0, f1, f2, x);
       f0 = f2;
+      tab += 2;
+    };
+    if (map.steps & 1u) {
+      screen_track(m0, x[0]);
+      screen_track(m1, x[1]);
+      step();
+    }
+#pragma unroll 1
+    for (uint32_t i = map.steps >> 1; i > 0; --i) {
+      const float h0 = screen_high(x[0]), h1 = screen_high(x[1]);
+      step();
+      screen_track2(m0, h0, screen_high(x[0]));
+      screen_track2(m1, h1, screen_high(x[1]));
+      step();
     }
     return m0 <= lim[0] && m1 <= lim[1];
   }
