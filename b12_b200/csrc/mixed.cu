@@ -29,7 +29,7 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr uint32_t kTable = 2048;   // doubles of the per-block grid-point table
-constexpr int kScreenBlocks = 6;    // resident blocks an SM of mixed_screen_kernel
+constexpr int kScreenBlocks = 4;    // resident blocks an SM of mixed_screen_kernel
 
 int grid_for_n(uint64_t n, int per_thread = 1)
 {
@@ -891,7 +891,7 @@ __global__ void __launch_bounds__(kThreads) mixed_image_kernel(const MixedArgs a
 // points, four at a time while many are left).  Bound by FP64 issue, like that kernel; the
 // leaves' centres come from a table of one pass over the leaves instead of being rebuilt for
 // every point.  Six selective steps of Lorenz (FMA) from depth 20: 1.95 ms against 2.46 (five
-// blocks an SM 1.98, four 1.98).
+// blocks an SM 1.99, six 2.01).
 template<class Map, class Grid, int kMode>
 __global__ void __launch_bounds__(kThreads, kScreenBlocks) mixed_screen_kernel(const MixedArgs a)
 {
