@@ -461,6 +461,7 @@ b12g_status b12g_tree_destroy(b12g_tree* t)
   t->sort_idx.release(); t->table.release(); t->snap_code.release(); t->snap_flags.release(); t->sort_tmp.release();
   t->last_tgt.release(); t->last_rank.release(); t->srcc.release(); t->bits.release(); t->pk.release();
   t->route_runs.release(); t->route_cnt.release();
+  if (t->sweep_read) cudaEventDestroy(t->sweep_read);
   if (t->h_ctr) cudaFreeHost(t->h_ctr);
   if (t->stream) cudaStreamDestroy(t->stream);
   delete t;

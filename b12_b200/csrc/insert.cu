@@ -75,7 +75,7 @@ __global__ void source_centres_kernel(const uint64_t* __restrict__ codes, const 
                                       const uint32_t* n_src, uint32_t n_all, Domain dom, DepthConst dc, int depth,
                                       double* __restrict__ out)
 {
-  const uint32_t n = n_src ? *n_src : n_all;
+  const uint32_t n = n_src ? min(*n_src, n_all) : n_all;    // (n_all: the room in `out`)
   for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
     const uint64_t code = __ldg(codes + (src ? __ldg(src + r) : r));
     double c[kSrcStride] = {0.0, 0.0, 0.0, 0.0};
@@ -128,7 +128,8 @@ int grid_over(uint64_t n, int per_sm = 8)
 b12g_status centres_of(b12g_tree* t, const uint64_t* codes, const uint32_t* src, const uint32_t* n_src,
                        uint32_t max_src)
 {
-  ST(t->srcc.ensure_room(uint64_t(std::max<uint32_t>(max_src, 1)) * kSrcStride, "source centres", 2));
+  const uint64_t need = uint64_t(std::max<uint32_t>(max_src, 1)) * kSrcStride;
+  if (t->srcc.n < need) ST(t->srcc.ensure_room(need, "source centres", 2));
   DepthConst dc;
   fill_depth_const(t->dom, int(t->domain.dim), t->depth, dc);
   const int g = grid_over(max_src);
@@ -524,10 +525,25 @@ __device__ __forceinline__ uint32_t block_sum_u32(uint32_t v, uint32_t* red)
   return t;
 }
 
+// `sweep` (optional): the sweep's count of new boxes and the error word for the host, and the
+// next sweep's count, set to zero
+struct SweepWords {
+  const uint32_t* count;
+  const uint32_t* error;
+  uint32_t* next;
+  volatile uint32_t* host_count;   // pinned host memory
+  volatile uint32_t* host_error;
+};
+
 __global__ void __launch_bounds__(kThreads) tile_count_kernel(const uint32_t* __restrict__ bits, uint32_t words,
-                                                              uint32_t* __restrict__ tile_count)
+                                                              uint32_t* __restrict__ tile_count, SweepWords sweep)
 {
   __shared__ uint32_t red[kThreads / 32];
+  if (sweep.count && blockIdx.x == 0 && threadIdx.x == 0) {
+    *sweep.host_count = *sweep.count;
+    *sweep.host_error = *sweep.error;
+    *sweep.next = 0u;
+  }
   const uint32_t tiles = (words + kWordTile - 1) / kWordTile;
   for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
     uint32_t c = 0;
@@ -538,16 +554,19 @@ __global__ void __launch_bounds__(kThreads) tile_count_kernel(const uint32_t* __
   }
 }
 
-// tile_first: the tiles' first positions (a scan of the counts), or nullptr: summed here
+// tile_first: the tiles' first positions (a scan of the counts), or nullptr: summed here.
+// total (optional): the number of codes; with more than `room` nothing is done
 __global__ void __launch_bounds__(kThreads) tile_scatter_kernel(uint32_t* __restrict__ bits, uint32_t words,
                                                                 const uint32_t* __restrict__ tile_count,
                                                                 const uint32_t* __restrict__ tile_first,
                                                                 uint64_t* __restrict__ out, int clear,
                                                                 const uint32_t* __restrict__ mark,
-                                                                uint8_t* __restrict__ flags, uint8_t f)
+                                                                uint8_t* __restrict__ flags, uint8_t f,
+                                                                const uint32_t* total, uint32_t room)
 {
   __shared__ uint32_t red[kThreads / 32];
   __shared__ uint32_t wsum[kThreads / 32];
+  if (total && *total > room) return;
   const uint32_t tiles = (words + kWordTile - 1) / kWordTile;
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
   for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
@@ -594,27 +613,40 @@ __global__ void __launch_bounds__(kThreads) tile_scatter_kernel(uint32_t* __rest
   }
 }
 
-// the codes of the set bits of `bits` (words u32) in increasing order into `out`, and
-// flags into `flags` when not null (f where `mark` has the bit); clears the bitmap when
-// asked
-b12g_status bitmap_codes(b12g_tree* t, uint32_t* bits, uint32_t words, uint64_t* out, bool clear,
-                         const uint32_t* mark = nullptr, uint8_t* flags = nullptr, uint8_t f = 0)
+// The codes of the set bits of `bits` (words u32) in increasing order into `out`, in two
+// launches: the tiles' counts, and the codes with flags into `flags` when not null (f where
+// `mark` has the bit); clears the bitmap when asked.  total, room: see tile_scatter_kernel.
+struct BitmapTiles {
+  uint32_t* count = nullptr;
+  uint32_t* first = nullptr;       // with many tiles: their first positions
+  int grid = 1;
+};
+
+b12g_status bitmap_counts(b12g_tree* t, const uint32_t* bits, uint32_t words, BitmapTiles& bt,
+                          const SweepWords& sweep = SweepWords{})
 {
   const uint32_t tiles = (words + kWordTile - 1) / kWordTile;
   ST(t->sort_idx.ensure(2 * (size_t(tiles) + 1) + compact_tiles(uint64_t(tiles) + 1) + 8, "bitmap tile counts"));
-  uint32_t* count = t->sort_idx.p;
-  uint32_t* first = nullptr;
-  const int g = int(std::min<uint64_t>(tiles, uint64_t(device_sm_count()) * 8));
-  tile_count_kernel<<<g, kThreads, 0, t->stream>>>(bits, words, count);
+  bt.count = t->sort_idx.p;
+  bt.grid = int(std::min<uint64_t>(tiles, uint64_t(device_sm_count()) * 8));
+  tile_count_kernel<<<bt.grid, kThreads, 0, t->stream>>>(bits, words, bt.count, sweep);
   CK(cudaGetLastError());
   count_launches(1);
   if (tiles > kLocalTiles) {
-    first = count + tiles + 1;
+    bt.first = bt.count + tiles + 1;
     ST(set_ctr(t, C_TMP, tiles));
-    CK(exclusive_scan_u32(count, first, t->ctr.p + C_TMP, first + tiles + 1, tiles, t->stream));
+    CK(exclusive_scan_u32(bt.count, bt.first, t->ctr.p + C_TMP, bt.first + tiles + 1, tiles, t->stream));
     count_launches(3);
   }
-  tile_scatter_kernel<<<g, kThreads, 0, t->stream>>>(bits, words, count, first, out, clear ? 1 : 0, mark, flags, f);
+  return B12G_OK;
+}
+
+b12g_status bitmap_scatter(b12g_tree* t, uint32_t* bits, uint32_t words, const BitmapTiles& bt, uint64_t* out,
+                           bool clear, const uint32_t* mark = nullptr, uint8_t* flags = nullptr, uint8_t f = 0,
+                           const uint32_t* total = nullptr, uint32_t room = 0)
+{
+  tile_scatter_kernel<<<bt.grid, kThreads, 0, t->stream>>>(bits, words, bt.count, bt.first, out, clear ? 1 : 0, mark,
+                                                           flags, f, total, room);
   CK(cudaGetLastError());
   count_launches(1);
   return B12G_OK;
@@ -642,14 +674,20 @@ b12g_status continuation_bitmap(b12g_tree* t, const b12g_scheme* s, uint8_t dept
   pr.a.n_src = nullptr;
   pr.a.bits = bits;
   pr.a.fresh = fresh;
-  pr.a.cand_count = t->ctr.p + C_CAND;
   uint64_t n = t->n;
   uint32_t n_src = t->n, u = 0, k = 0, nb0 = 0, nb1 = t->n;
+  // two counters of new boxes, taken in turn: each sweep's compaction empties the next one's
+  ST(set_ctr(t, C_CAND, 0));
+  ST(set_ctr(t, C_NNEW, 0));
+  uint32_t* found = t->ctr.p + C_CAND;
+  if (!t->sweep_read && cudaEventCreateWithFlags(&t->sweep_read, cudaEventDisableTiming) != cudaSuccess)
+    return cuda_fail(cudaGetLastError(), "event");
   while (nb1 > nb0 && k < max_sweeps) {
     const uint64_t points = uint64_t(n_src) * pr.P;
-    ST(set_ctr(t, C_CAND, 0));
     pr.a.n_src_value = n_src;
     pr.a.src_c = t->srcc.p;
+    found = t->ctr.p + (k & 1u ? C_NNEW : C_CAND);
+    pr.a.cand_count = found;
     u = 0;
     if (points > 0) {
       prof_mark(t, 0);
@@ -657,21 +695,39 @@ b12g_status continuation_bitmap(b12g_tree* t, const b12g_scheme* s, uint8_t dept
                       t->stream));
       prof_mark(t, 0);
       count_launches(1);
-      ST(read_ctr(t, C_ERROR, C_DEFER - C_ERROR + 1));
+      // The next sources: the new boxes in code order, their codes and centres (the centres
+      // by a thread per box: inside the compaction's loop over a word's bits they would
+      // serialise, 1.9 ms against 0.95 ms for the run's compactions and centres apart).  They
+      // are queued for as many boxes as there is room for before the host knows the number,
+      // which the first of the kernels writes to host memory: the host reads it while the
+      // others run (waiting for it first left the GPU idle for 29 us a sweep).
+      const SweepWords sweep{found, t->ctr.p + C_ERROR, t->ctr.p + (k & 1u ? C_CAND : C_NNEW), t->h_ctr + C_CAND,
+                             t->h_ctr + C_ERROR};
+      BitmapTiles bt;
+      ST(bitmap_counts(t, fresh, words, bt, sweep));
+      CK(cudaEventRecord(t->sweep_read, t->stream));
+      uint64_t room = std::min<uint64_t>(boxes, std::max<uint64_t>(2ull * n_src, 1ull << 16));
+      auto next_sources = [&]() -> b12g_status {
+        // (the centres overwrite the image launch's: the stream runs them after it)
+        ST(bitmap_scatter(t, fresh, words, bt, t->cand.p, true, nullptr, nullptr, 0, found, uint32_t(room)));
+        return centres_of(t, t->cand.p, nullptr, found, uint32_t(room));
+      };
+      if (t->cand.ensure(room, "new boxes") != B12G_OK || t->srcc.ensure(room * kSrcStride, "source centres") != B12G_OK)
+        room = std::min<uint64_t>(t->cand.n, t->srcc.n / kSrcStride);   // that much is not free: what there is
+      ST(next_sources());
+      CK(cudaEventSynchronize(t->sweep_read));
       ST(prof_collect(t));
       if (t->h_ctr[C_ERROR]) {
+        const uint32_t e = t->h_ctr[C_ERROR];
         set_ctr(t, C_ERROR, 0);
-        return fail(B12G_ERR_CAPACITY, "continuation: device error bits %u", t->h_ctr[C_ERROR]);
+        return fail(B12G_ERR_CAPACITY, "continuation: device error bits %u", e);
       }
       u = t->h_ctr[C_CAND];
-      if (u > 0) {
-        // the next sources: the new boxes in code order, their codes and centres
-        // (the centres by a thread per box: inside the compaction's loop over a word's
-        // bits they would serialise, 1.9 ms against 0.95 ms for the run's compactions and
-        // centres apart)
-        ST(t->cand.ensure_room(u, "new boxes", 2));
-        ST(bitmap_codes(t, fresh, words, t->cand.p, true));
-        ST(centres_of(t, t->cand.p, nullptr, t->ctr.p + C_CAND, u));
+      if (u > room) {
+        room = u;
+        ST(t->cand.ensure(room, "new boxes"));
+        ST(t->srcc.ensure(room * kSrcStride, "source centres"));
+        ST(next_sources());
       }
     }
     n += u;
@@ -688,11 +744,13 @@ b12g_status continuation_bitmap(b12g_tree* t, const b12g_scheme* s, uint8_t dept
   ST(reserve(t, n));
   const int o = 1 - t->cur, no = 1 - t->ncur;
   if (u > 0) {
-    set_bits_kernel<<<grid_over(u), kThreads, 0, t->stream>>>(t->cand.p, t->ctr.p + C_CAND, fresh);
+    set_bits_kernel<<<grid_over(u), kThreads, 0, t->stream>>>(t->cand.p, found, fresh);
     CK(cudaGetLastError());
     count_launches(1);
   }
-  ST(bitmap_codes(t, bits, words, t->code[o].p, false, u > 0 ? fresh : nullptr, t->flags[o].p, B12G_INS));
+  BitmapTiles bt;
+  ST(bitmap_counts(t, bits, words, bt));
+  ST(bitmap_scatter(t, bits, words, bt, t->code[o].p, false, u > 0 ? fresh : nullptr, t->flags[o].p, B12G_INS));
   ST(set_ctr(t, no, uint32_t(n)));
   ST(sync(t, "continuation leaves"));
   t->cur = o;

@@ -155,6 +155,7 @@ struct b12g_tree {
   uint32_t hash_tag = 0;       // tag of the last build (1..255; 0 = cleared)
   uint32_t hash_log2 = 0;      // log2 of the table's slots
   uint32_t* h_ctr = nullptr;   // pinned mirror of ctr
+  cudaEvent_t sweep_read = nullptr;   // a continuation sweep's count is in h_ctr
   // graph cache of the fused subdivision loop
   cudaGraphExec_t sub_graph = nullptr;
   std::vector<uint8_t> sub_key;
