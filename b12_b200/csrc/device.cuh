@@ -710,6 +710,13 @@ struct FullGrid {
   }
 };
 
+// 3 + the point of philox_signed without its last bit, in [2, 4): the bits go straight into
+// the fraction (for the screened evaluation, whose start point may differ by a few roundings)
+__device__ __forceinline__ double philox_raised(uint32_t hi, uint32_t lo)
+{
+  return __hiloint2double(int(0x40000000u | (hi >> 12)), int(__funnelshift_r(lo, hi, 12)));
+}
+
 struct PhiloxGrid {
   static constexpr bool kTable = false;
   static __device__ __forceinline__ double table_value(const GridParams&, const double*, uint32_t, int) { return 0.0; }
@@ -724,6 +731,18 @@ struct PhiloxGrid {
       philox4x32_10(c, uint32_t(g.seed), uint32_t(g.seed >> 32));
       res[j] = philox_signed(c[0], c[1]);
       if (j + 1 < D) res[j + 1] = philox_signed(c[2], c[3]);
+    }
+  }
+  // the same points near enough for the screened evaluation, 3 higher
+  template<int D>
+  static __device__ __forceinline__ void raised(const GridParams& g, uint64_t i, double* res)
+  {
+#pragma unroll
+    for (int j = 0; j < D; j += 2) {
+      uint32_t c[4] = {uint32_t(i), uint32_t(i >> 32), uint32_t(j / 2), 0u};
+      philox4x32_10(c, uint32_t(g.seed), uint32_t(g.seed >> 32));
+      res[j] = philox_raised(c[0], c[1]);
+      if (j + 1 < D) res[j + 1] = philox_raised(c[2], c[3]);
     }
   }
 };

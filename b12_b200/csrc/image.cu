@@ -3,6 +3,8 @@
 // GridPointsFunctor (Functors.hpp:476-511) consumed by thrust::lower_bound and
 // ComputeSearchIndexFunctor (ImplicitBoxTree.hpp:2394-2432), evaluated once per point
 // instead of twice and without the point stream ever being stored.
+#include <type_traits>
+
 #include "kernels.h"
 #include "rows.cuh"
 
@@ -102,9 +104,15 @@ struct PointImage {
                                                      uint32_t (&tbits)[D], bool& valid)
   {
     double g[D], x[D];
-    grid_point(a, pts, use_table, i, k, g);
+    if constexpr (std::is_same<Grid, PhiloxGrid>::value) {
+      Grid::template raised<D>(a.grid, i, g);
 #pragma unroll
-    for (int j = 0; j < D; ++j) x[j] = __fma_rn(g[j], a.sc.sR[j], __fma_rn(c[j], a.sc.sC[j], a.sc.sD[j]));
+      for (int j = 0; j < D; ++j) x[j] = __fma_rn(g[j], a.sc.sR[j], __fma_rn(c[j], a.sc.sC[j], a.sc.sP[j]));
+    } else {
+      grid_point(a, pts, use_table, i, k, g);
+#pragma unroll
+      for (int j = 0; j < D; ++j) x[j] = __fma_rn(g[j], a.sc.sR[j], __fma_rn(c[j], a.sc.sC[j], a.sc.sD[j]));
+    }
     const bool kept = Screen<Map>::run(a.sc, a.map, x);
     return screen_locate<D>(a.sc, x, tbits, valid) && kept;
   }
@@ -141,7 +149,9 @@ struct PointImage {
 };
 
 constexpr uint32_t kPointTable = 2048;  // doubles of grid-point table per block (16 KB)
-constexpr int kChunkTrips = 4;          // units (a point a lane) a warp takes at a time from the work queue
+constexpr int kChunkTrips = 4;          // units (a point a lane) a warp takes at a time from the work queue;
+                                        // twice as many in Mark mode, whose points are short and whose
+                                        // launches large (the continuation 9.26 ms, with four 9.46)
 constexpr int kFineUnits = 4;           // units a warp left in the queue when it takes single ones (1: a
                                         // depth-22 forced Duffing job's image launches 1.64 ms, 4: 1.48, 8: 1.45,
                                         // while the continuation's take 11.07, 11.13 and 11.47 ms)
@@ -169,13 +179,27 @@ __device__ __forceinline__ bool load_points(const GridParams& g, uint64_t P, dou
 // other instructions per 32 Lorenz points against 942 and 290 (FMA) or 1,600 (strict); the
 // image launches of a depth-27 job take 5.52 ms against 6.58 (FMA) and 10.21 (strict).  Four
 // blocks an SM, 64 registers: the coefficients stay in registers over the unrolled steps
-// (five blocks with 48: 5.72 ms, three: 5.52).
+// (five blocks with 48: 5.72 ms, three: 5.52).  Mark mode (the continuation, short points):
+// five blocks, 9.46 ms against 9.62 with four.
 template<class Map, class Grid, ImageMode M, bool kScreen>
-__global__ void __launch_bounds__(kThreads, kScreen ? 4 : 6) image_points_kernel(const ImageArgs a)
+__global__ void __launch_bounds__(kThreads, !kScreen ? 6 : M == ImageMode::Mark ? 5 : 4) image_points_kernel(const ImageArgs a)
 {
   using PI = PointImage<Map, Grid>;
   __shared__ double pts[kPointTable];
-  const bool table = load_points<Grid, Map::D>(a.grid, a.points, pts);
+  // Mark mode: an index's place in the box's code, by dimension, where the indices have at
+  // most 8 bits (four reads and two ORs instead of 36 instructions of bit spreading)
+  __shared__ uint32_t spread[M == ImageMode::Mark ? Map::D * 256 : 1];
+  bool spread_ok = false;
+  if constexpr (M == ImageMode::Mark) {
+    spread_ok = a.dc.c32 && a.dc.k[0] <= 8;
+    if (spread_ok)
+      for (uint32_t i = threadIdx.x; i < Map::D * 256; i += blockDim.x) {
+        uint32_t one[Map::D] = {};
+        one[i >> 8] = i & 255u;
+        spread[i] = uint32_t(code_of_bits<Map::D>(a.dc, one, a.depth));
+      }
+  }
+  const bool table = load_points<Grid, Map::D>(a.grid, a.points, pts);   // (ends with a block barrier)
 
   const uint32_t n = *a.n_leaves;
   const uint32_t nboxes = M == ImageMode::Mark ? a.n_src_value : a.n_src ? *a.n_src : (a.children ? 2u * n : n);
@@ -189,6 +213,10 @@ __global__ void __launch_bounds__(kThreads, kScreen ? 4 : 6) image_points_kernel
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(a.error, 1u);
     return;
   }
+  // Mark mode: the warp's new boxes (the same in every lane), added to the launch's count at
+  // the end (an atomic for every warp with a new box held the continuation's image launches
+  // at 10.8 ms; without them 9.6)
+  uint32_t new_boxes = 0;
   // One point of the launch: g = rank * P + k (the source's rank among the sources, the
   // point's index in its box).  Every lane of the warp calls it the same number of times
   // (inactive lanes with active = false), so that the warp collectives stay converged.
@@ -234,12 +262,17 @@ __global__ void __launch_bounds__(kThreads, kScreen ? 4 : 6) image_points_kernel
     } else if constexpr (M == ImageMode::Mark) {
       // the image's box, unless its bit is set already (a stale read only sends the point
       // on to the atomic), deduplicated within the warp: most warps find no new box.  The lane
-      // whose atomic sets the bit marks the box in `fresh`, and the warp counts its new boxes
-      // with one atomic.
+      // whose atomic sets the bit marks the box in `fresh`.
       uint32_t code = 0;
       bool fresh = false;
       if (active && valid) {
-        code = uint32_t(code_of_bits<Map::D>(a.dc, tbits, a.depth));
+        if (spread_ok) {
+          code = 0;
+#pragma unroll
+          for (int j = 0; j < Map::D; ++j) code |= spread[j * 256 + tbits[j]];
+        } else {
+          code = uint32_t(code_of_bits<Map::D>(a.dc, tbits, a.depth));
+        }
         fresh = !((a.bits[code >> 5] >> (code & 31u)) & 1u);
       }
       if (__any_sync(0xFFFFFFFFu, fresh)) {
@@ -251,7 +284,7 @@ __global__ void __launch_bounds__(kThreads, kScreen ? 4 : 6) image_points_kernel
           if (fresh) atomicOr(a.fresh + (code >> 5), m);
         }
         const unsigned lead_mask = __ballot_sync(0xFFFFFFFFu, fresh);
-        if (lane == 0 && lead_mask) atomicAdd(a.cand_count, uint32_t(__popc(lead_mask)));
+        new_boxes += uint32_t(__popc(lead_mask));
       }
     } else {
       // candidates: valid images that are not leaves, as packed keys (the caller turns them
@@ -289,6 +322,7 @@ __global__ void __launch_bounds__(kThreads, kScreen ? 4 : 6) image_points_kernel
   // through its units one after another, so in a small launch, and at the end of a large
   // one, larger pieces would leave the others idle (the small steps of a forced Duffing job
   // took 68 us with four points a lane, 25 us with one).
+  constexpr uint32_t kTake = M == ImageMode::Mark ? 2 * kChunkTrips : kChunkTrips;
   uint32_t shift = 0;
   while (((total + 31) >> (5 + shift)) >= 0x40000000ull) ++shift;
   const uint32_t units = uint32_t((total + (32ull << shift) - 1) >> (5 + shift));
@@ -296,14 +330,14 @@ __global__ void __launch_bounds__(kThreads, kScreen ? 4 : 6) image_points_kernel
   const uint32_t coarse_end = units > fine ? units - fine : 0;
   uint32_t c = 0;
   for (;;) {
-    const uint32_t size = c < coarse_end ? uint32_t(kChunkTrips) : 1u;
+    const uint32_t size = c < coarse_end ? kTake : 1u;
     if (lane == 0) c = atomicAdd(a.work, size);
     c = __shfl_sync(0xFFFFFFFFu, c, 0);
     if (c >= units) break;
     // (sources and points per box both fit 32 bits: the rank and the point index do)
     const uint64_t g = (uint64_t(c) << (5 + shift)) + uint64_t(lane);
     uint32_t rank, k;
-    if (total <= 0xFFFFFFFFull - 64ull * kChunkTrips) {
+    if (total <= 0xFFFFFFFFull - 64ull * kTake) {
       rank = uint32_t(g) / P32;
       k = uint32_t(g) - rank * P32;
     } else {
@@ -317,6 +351,9 @@ __global__ void __launch_bounds__(kThreads, kScreen ? 4 : 6) image_points_kernel
       k += 32;
       while (k >= P32) { k -= P32; ++rank; }
     }
+  }
+  if constexpr (M == ImageMode::Mark) {
+    if (lane == 0 && new_boxes) atomicAdd(a.cand_count, new_boxes);
   }
 }
 

@@ -400,6 +400,7 @@ void screen_at(ScreenPlan& plan, int depth, ScreenArgs& s)
       s.sC[j] = S;
       s.sD[j] = -S * b.shift[j];
       s.sR[j] = S * rk;
+      s.sP[j] = s.sD[j] - 3.0 * s.sR[j];
       s.tA[j] = half / (r * S);
       s.tB[j] = 0x1.8p20 + (half + half * (b.shift[j] - dom.c[j]) / r);
       s.bits[j] = uint32_t(dc.k[j]);

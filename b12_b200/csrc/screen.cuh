@@ -39,8 +39,10 @@ struct ScreenArgs {
   float lim[B12G_MAX_DIM];     // limits on |X_j| as the high words of doubles, see screen_track
   double k[kScreenCoef];       // the map's coefficients
   // the start point: fma(g, sR, fma(v, sA, sB)) from the box's index (v = 1 + index 2^-k),
-  // or fma(g, sR, fma(centre, sC, sD)) from the box's centre
+  // or fma(g, sR, fma(centre, sC, sD)) from the box's centre; sP = sD - 3 sR for points
+  // given 3 too high
   double sA[B12G_MAX_DIM], sB[B12G_MAX_DIM], sC[B12G_MAX_DIM], sD[B12G_MAX_DIM], sR[B12G_MAX_DIM];
+  double sP[B12G_MAX_DIM];
   // the image's box: fma(X, tA, tB) is 1.5 2^20 + (position in boxes), so its high word
   // counts boxes and its low word is the fraction in units of 2^-32
   double tA[B12G_MAX_DIM], tB[B12G_MAX_DIM];
