@@ -56,9 +56,18 @@ b12g_status sync(b12g_tree* t, const char* where)
   return B12G_OK;
 }
 
+// The counters are written to the pinned block by a kernel: its launch and its store take
+// less time than a copy's submission and the copy engine's turn.
+__global__ void publish_words_kernel(const uint32_t* p, volatile uint32_t* host, int count)
+{
+  if (int(threadIdx.x) < count) host[threadIdx.x] = p[threadIdx.x];
+}
+
 b12g_status read_ctr(b12g_tree* t, int first, int count)
 {
-  CK(cudaMemcpyAsync(t->h_ctr + first, t->ctr.p + first, count * sizeof(uint32_t), cudaMemcpyDeviceToHost, t->stream));
+  publish_words_kernel<<<1, 96, 0, t->stream>>>(t->ctr.p + first, t->h_ctr + first, count);
+  CK(cudaGetLastError());
+  count_launches(1);
   return sync(t, "read counters");
 }
 
@@ -298,7 +307,7 @@ b12g_status flag_call(b12g_tree* t, int op, uint8_t u, uint8_t f, uint8_t depth,
     if (depth > 64) return fail(B12G_ERR_INVALID, "depth %u above the maximal depth 64", depth);
     return mixed_flags_at_depth(t, op, u, f, depth, n_changed);
   }
-  ST(set_ctr(t, C_CHANGED, 0));
+  if (!counts_alone(t->n)) ST(set_ctr(t, C_CHANGED, 0));
   CK(flag_op(t->flg(), t->dn(), op, u, f, t->ctr.p + C_CHANGED, t->n, t->stream));
   count_launches(1);
   if (!n_changed) return B12G_OK;   // nobody reads the count: no round trip (the stream keeps the order)
@@ -561,7 +570,7 @@ b12g_status b12g_subdivide(b12g_tree* t, uint8_t flags, uint32_t* n_subdivided)
   // subdivide (ImplicitBoxTree.hpp:2884-2929) returns the number of leaves with all
   // flags set; IsSubdividableFunctor (Functors.hpp:332-335) splits those below depth 64
   uint32_t m = 0;
-  ST(set_ctr(t, C_TMP, 0));
+  if (!counts_alone(t->n)) ST(set_ctr(t, C_TMP, 0));
   CK(count_flags(t->flg(), t->dn(), flags, t->ctr.p + C_TMP, t->n, t->stream));
   count_launches(1);
   ST(read_ctr(t, C_TMP, 1));
@@ -652,7 +661,7 @@ b12g_status b12g_set_flags_by_image(b12g_tree* t, const b12g_scheme* sc, uint8_t
   uint32_t n_src = 0;
   ST(select_sources(t, sc, pr, n_src));
   ST(build_current_hash(t, pr));
-  ST(set_ctr(t, C_CHANGED, 0));
+  if (!counts_alone(t->n)) ST(set_ctr(t, C_CHANGED, 0));
   pr.a.hit_cap = uint32_t(std::min<size_t>(t->hit.n, 0xFFFFFFFFu));
   prof_mark(t, 0);
   CK(launch_image(sc->map.kind, sc->map.arith, sc->grid.kind, t->domain.dim, ImageMode::Hit, pr.a,

@@ -111,6 +111,9 @@ int device_sm_count();
 cudaError_t build_leaf_hash(const uint64_t* codes, const uint32_t* n, int depth, int dim, LeafHash h, uint32_t* error,
                             uint32_t max_n, cudaStream_t s);
 
+// whether the three counts below, over at most max_n leaves, store their count instead of
+// adding it (the counter may then hold anything before)
+bool counts_alone(uint32_t max_n);
 // flags |= f on hit leaves (hit cleared); *changed += leaves that lacked f
 cudaError_t apply_hits(uint8_t* flags, uint8_t* hit, const uint32_t* n, uint8_t f, uint32_t* changed,
                        uint32_t max_n, cudaStream_t s);

@@ -59,6 +59,19 @@ int grid_for(uint64_t work, int per_block, int blocks_per_sm)
   return int(std::max<uint64_t>(1, std::min(want, cap)));
 }
 
+// A count over at most kSingleBlock elements is made by one block, which stores it: the
+// counter need not be zero before (a memset is as much work for the host as the kernel).
+constexpr uint32_t kSingleBlock = 2048;
+
+int count_grid(uint32_t max_n) { return max_n <= kSingleBlock ? 1 : grid_for(max_n, kThreads, 8); }
+
+__device__ __forceinline__ void add_count(uint32_t* count, uint32_t c)
+{
+  if (threadIdx.x != 0 || !count) return;
+  if (gridDim.x == 1) *count = c;
+  else if (c) atomicAdd(count, c);
+}
+
 // ---------------------------------------------------------------------------------
 __global__ void apply_hits_kernel(uint8_t* flags, uint8_t* hit, const uint32_t* n_ptr, uint8_t f, uint32_t* changed)
 {
@@ -76,7 +89,7 @@ __global__ void apply_hits_kernel(uint8_t* flags, uint8_t* hit, const uint32_t* 
     }
   }
   c = block_sum(c, red);
-  if (threadIdx.x == 0 && c) atomicAdd(changed, c);
+  add_count(changed, c);
 }
 
 // op 0: set f (count boxes lacking f); 1: unset f (count boxes having any of f);
@@ -96,7 +109,7 @@ __global__ void flag_op_kernel(uint8_t* flags, const uint32_t* n_ptr, int op, ui
     else if (has_all(old, u)) { ++c; flags[i] = uint8_t((old & ~u) | f); }
   }
   c = block_sum(c, red);
-  if (threadIdx.x == 0 && c && changed) atomicAdd(changed, c);
+  add_count(changed, c);
 }
 
 __global__ void count_flags_kernel(const uint8_t* flags, const uint32_t* n_ptr, uint8_t f, uint32_t* count)
@@ -109,7 +122,7 @@ __global__ void count_flags_kernel(const uint8_t* flags, const uint32_t* n_ptr, 
   for (uint32_t it = 0, i = blockIdx.x * blockDim.x + threadIdx.x; it < iters; ++it, i += stride)
     if (i < n && has_all(flags[i], f)) ++c;
   c = block_sum(c, red);
-  if (threadIdx.x == 0 && c) atomicAdd(count, c);
+  add_count(count, c);
 }
 
 // subdivide: incrementDepthBy(1) + computeOtherHalf (Box.hpp:140-147, 234-239); the
@@ -464,24 +477,26 @@ int device_sm_count()
   return sms[dev];
 }
 
+bool counts_alone(uint32_t max_n) { return max_n <= kSingleBlock; }
+
 cudaError_t apply_hits(uint8_t* flags, uint8_t* hit, const uint32_t* n, uint8_t f, uint32_t* changed, uint32_t max_n,
                        cudaStream_t s)
 {
-  apply_hits_kernel<<<grid_for(max_n, kThreads, 8), kThreads, 0, s>>>(flags, hit, n, f, changed);
+  apply_hits_kernel<<<count_grid(max_n), kThreads, 0, s>>>(flags, hit, n, f, changed);
   return cudaGetLastError();
 }
 
 cudaError_t flag_op(uint8_t* flags, const uint32_t* n, int op, uint8_t u, uint8_t f, uint32_t* changed,
                     uint32_t max_n, cudaStream_t s)
 {
-  flag_op_kernel<<<grid_for(max_n, kThreads, 8), kThreads, 0, s>>>(flags, n, op, u, f, changed);
+  flag_op_kernel<<<count_grid(max_n), kThreads, 0, s>>>(flags, n, op, u, f, changed);
   return cudaGetLastError();
 }
 
 cudaError_t count_flags(const uint8_t* flags, const uint32_t* n, uint8_t f, uint32_t* count, uint32_t max_n,
                         cudaStream_t s)
 {
-  count_flags_kernel<<<grid_for(max_n, kThreads, 8), kThreads, 0, s>>>(flags, n, f, count);
+  count_flags_kernel<<<count_grid(max_n), kThreads, 0, s>>>(flags, n, f, count);
   return cudaGetLastError();
 }
 
