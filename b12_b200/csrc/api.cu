@@ -904,12 +904,13 @@ b12g_status ensure_transpose(b12g_csr* m)
     count_launches(7);
     // a matrix of counts of a size that fits: its packed form, whose outcome comes back with
     // the longest row (ctr words 6, and 7 to 9)
+    // (without memory for it, the iteration takes the matrix as it is)
     const bool pack = m->count_points > 0 && m->count_points <= 255 &&
-                      count_plan_possible(m->nnz, n, uint32_t(measure_partial_slots()));
+                      count_plan_possible(m->nnz, n, uint32_t(measure_partial_slots())) &&
+                      m->pack.ensure(m->nnz, "packed matrix") == B12G_OK &&
+                      m->dlist.ensure(size_t(device_sm_count()) * count_distinct_cap(m->nnz), "packed matrix") == B12G_OK &&
+                      m->dcount.ensure(device_sm_count(), "packed matrix") == B12G_OK;
     if (pack) {
-      ST(m->pack.ensure(m->nnz, "packed matrix"));
-      ST(m->dlist.ensure(size_t(device_sm_count()) * count_distinct_cap(m->nnz), "packed matrix"));
-      ST(m->dcount.ensure(device_sm_count(), "packed matrix"));
       CK(count_plan(m->tptr.p, m->trows.p, m->tvals.p, n, m->nnz, m->count_points, m->pack.p, m->dlist.p,
                     m->dcount.p, m->ctr.p + 7, s));
       count_launches(1);
@@ -1061,10 +1062,18 @@ b12g_status b12g_subdivision_run(b12g_tree* t, const b12g_scheme* sc, uint32_t s
   // keep the initial state so that a capacity overflow can be retried with more room
   const uint32_t n0 = t->n;
   const uint8_t d0 = t->depth;
-  ST(t->snap_code.ensure(n0, "initial leaves"));
-  ST(t->snap_flags.ensure(n0, "initial leaves"));
-  CK(cudaMemcpyAsync(t->snap_code.p, t->codes(), size_t(n0) * 8, cudaMemcpyDeviceToDevice, t->stream));
-  CK(cudaMemcpyAsync(t->snap_flags.p, t->flg(), n0, cudaMemcpyDeviceToDevice, t->stream));
+  // (on the device, or on the host when the device has no room for it)
+  std::vector<uint64_t> host_code;
+  std::vector<uint8_t> host_flags;
+  if (t->snap_code.ensure(n0, "initial leaves") != B12G_OK || t->snap_flags.ensure(n0, "initial leaves") != B12G_OK) {
+    host_code.resize(n0);
+    host_flags.resize(n0);
+  }
+  const bool on_host = !host_code.empty();
+  uint64_t* const snap_code = on_host ? host_code.data() : t->snap_code.p;
+  uint8_t* const snap_flags = on_host ? host_flags.data() : t->snap_flags.p;
+  CK(cudaMemcpyAsync(snap_code, t->codes(), size_t(n0) * 8, cudaMemcpyDefault, t->stream));
+  CK(cudaMemcpyAsync(snap_flags, t->flg(), n0, cudaMemcpyDefault, t->stream));
   // the steps' counts follow the counters, so that one read-back brings both
   uint32_t* const step_counts = t->ctr.p + C_COUNT;
 
@@ -1189,8 +1198,8 @@ b12g_status b12g_subdivision_run(b12g_tree* t, const b12g_scheme* sc, uint32_t s
       cap *= 4;
       ST(reserve(t, cap));
       CK(cudaMemsetAsync(t->hit.p, 0, t->hit.n, t->stream));
-      CK(cudaMemcpyAsync(t->codes(), t->snap_code.p, size_t(n0) * 8, cudaMemcpyDeviceToDevice, t->stream));
-      CK(cudaMemcpyAsync(t->flg(), t->snap_flags.p, n0, cudaMemcpyDeviceToDevice, t->stream));
+      CK(cudaMemcpyAsync(t->codes(), snap_code, size_t(n0) * 8, cudaMemcpyDefault, t->stream));
+      CK(cudaMemcpyAsync(t->flg(), snap_flags, n0, cudaMemcpyDefault, t->stream));
       ST(set_ctr(t, t->ncur, n0));
       ST(sync(t, "restore"));
       t->n = n0;

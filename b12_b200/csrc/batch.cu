@@ -7,14 +7,15 @@
 // subdividing at step k are a prefix of the order.  Their leaves are concatenated in
 // one code array with per-instance offsets.  A step runs:
 //   1. a lookup table over (instance, parent code);
-//   2. the box-image kernel: a device work queue of fixed-size point chunks over all
-//      instances' (implicit) children, claimed by the persistent blocks with one atomic
-//      per chunk; a chunk's points find their instance by binary search in shared memory;
+//   2. the box-image kernel: a device work queue of points over all instances' (implicit)
+//      children, claimed by the persistent blocks (batch_screen_kernel: a warp at a time,
+//      in units of 32; batch_image_kernel: a block at a time, in fixed-size chunks); a
+//      piece's points find their instance by binary search in shared memory;
 //   3. per-instance survivor counts, then one ordered compaction of all children;
 //   4. new offsets; instances whose depth is reached move to the final arena.
 // All launches read their sizes from device memory: the whole run is one CUDA graph.
-// The image kernel's block size, points per thread and chunk size are chosen by timing
-// the candidates on the first run (autotuner).
+// batch_image_kernel's block size, points per thread and chunk size are chosen by timing
+// the candidates on the first run (autotuner); batch_screen_kernel has one shape.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -835,7 +836,8 @@ b12g_status batch_screen_records(b12g_batch* b, const std::vector<double>& param
     }
   }
   if (!common.on) return B12G_OK;
-  ST(b->screen.ensure(rec.size(), "batch screen records"));
+  // (without memory for them, too)
+  if (b->screen.ensure(rec.size(), "batch screen records") != B12G_OK) return B12G_OK;
   CK(cudaMemcpy(b->screen.p, rec.data(), rec.size() * sizeof(ScreenRec), cudaMemcpyHostToDevice));
   b->screen_common = common;
   return B12G_OK;

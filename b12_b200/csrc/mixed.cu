@@ -1173,7 +1173,11 @@ b12g_status mixed_screen(b12g_tree* t, const b12g_scheme* sc, MixedArgs& a)
   a.depth = int(t->depth);
   fill_screen(sc->map.kind, a.map, a.dom, int(t->domain.dim), a.depth, grid_reach(sc->grid.kind, a.grid), a.sc);
   if (!a.sc.on) return B12G_OK;
-  ST(t->srcc.ensure_room(uint64_t(std::max<uint32_t>(t->n, 1)) * kSrcStride, "leaf centres", 2));
+  const size_t need = size_t(std::max<uint32_t>(t->n, 1)) * kSrcStride;
+  if (t->srcc.ensure_room(need, "leaf centres", 2) != B12G_OK && t->srcc.ensure(need, "leaf centres") != B12G_OK) {
+    a.sc.on = 0;   // no memory for the centres: the map's own arithmetic needs none
+    return B12G_OK;
+  }
   a.src_c = t->srcc.p;
   const int g = grid_for_n(t->n);
   switch (t->domain.dim) {

@@ -11,7 +11,8 @@
 // step's inputs.  Iterated over the map's steps from the start points' distance this gives
 // E; eta is checked at the end.  Only |x^ - x~| <= E matters, not the integrator's own
 // error, so E stays near the roundings times the flow's growth: for the benchmark's Lorenz
-// map over twice its domain 4e-6 of a box of width 0.12, where the distances seen are 3e-14.
+// map over twice its domain 4e-6, against boxes 0.12 wide at depth 27 and distances seen of
+// 3e-14.
 #include <algorithm>
 #include <cmath>
 #include <cstring>

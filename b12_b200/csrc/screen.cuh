@@ -122,7 +122,8 @@ __host__ __device__ __forceinline__ void lorenz_screen_step(const K* k, T (&x)[3
 // Q1 = h q1, Q2 = sqrt(0.2) h q2, P1 = h^2 p1, P2 = sqrt(0.2) h^2 p2: a drift is Q + P and a
 // kick P1 += Q1 (h^2 - Q1^2 - Q2^2), P2 += Q2 (-1.69 h^2 - 0.2 Q1^2).  The half drifts of
 // consecutive steps join: 7 operations a step.  The image launches of the depth-24
-// continuation take 11.0 ms against 15.5 (now the Philox points and the marking dominate).
+// continuation take 11.0 ms against 15.5 with these steps alone (9.26 with the counting and
+// the codes of the Mark launches made cheaper: the Philox points and the marking dominate).
 // k: h^2, 0.2, -(1.69 + 0.2) h^2
 template<class T, class K>
 __host__ __device__ __forceinline__ void duffing_screen_kick(const K* k, T (&x)[4])
@@ -152,7 +153,8 @@ __host__ __device__ __forceinline__ void duffing_screen_half_drift(T (&x)[4])
 //   c V' = -c delta V - X (c^2 alpha + X^2) + F(t),
 // RK4 put together as for Lorenz: 25 operations a step and the two of F = k[3] cos at the
 // middle and the end.  f0, f1, f2: F at the stages' times.  The image launches of a
-// depth-19 job take 2.03 ms against 3.85, of a depth-22 one 2.72 against 5.44.
+// depth-19 job take 2.03 ms against 3.85, of a depth-22 one 2.72 against 5.44, with these
+// steps alone (0.86 and 1.47 with the work queue of 32-point units: small launches).
 // k: -c^2 alpha, -c delta, 1 - c delta, c^3 sqrt(beta) gamma, 1 / 3
 template<class T, class K>
 __host__ __device__ __forceinline__ void forced_screen_step(const K* k, const T& f0, const T& f1, const T& f2,

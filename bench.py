@@ -554,9 +554,10 @@ def configs_mode(args, peak_tflops: float):
                      "achieved": img_tflops, "peak": peak_tflops, "unit": "TFLOP/s",
                      "frac": img_tflops / peak_tflops if img_tflops else None,
                      "strict_cap": 0.5, "kernel_ms": img_ms, "launches": img_n,
-                     "note": "strict arithmetic (one rounding per operation, the reference's own "
-                             "SymplecticIntegratorAuto order): at most half the FMA peak; the rest of the run is "
-                             "the candidate sort, unique, merge and flag updates (launch list in profiles/)"},
+                     "note": "FLOP counted as strict arithmetic (one rounding per operation, the reference's own "
+                             "SymplecticIntegratorAuto order; at most half the FMA peak); most images are decided by "
+                             "a screened evaluation of fewer operations; the rest of the run is the bitmaps' "
+                             "compactions and the centres (launch list in profiles/)"},
         "note": "every box is imaged once, in the sweep after it was inserted"}
     if cpu:
         sweeps_ref = 20
