@@ -276,6 +276,41 @@ __global__ void __launch_bounds__(512) batch_image_kernel(const BatchArgs a)
 // 32.3 (the shape with four points a thread).
 constexpr uint32_t kScreenTrips = 4, kScreenFine = 4;
 
+// test point k of the box with indices sb, by an instance's record and the launch's
+// coefficients: the image's indices and whether it lies in the domain; returns whether both
+// are certain
+template<class Map>
+__device__ __forceinline__ bool screened_point(const ScreenRec* r, const double* sk, const double* sA,
+                                               const MapParams& map, const double* pts, uint32_t P, uint32_t k,
+                                               const uint32_t (&sb)[Map::D], uint32_t (&tb)[Map::D], bool& inside)
+{
+  constexpr int D = Map::D;
+  const uint32_t kb = __ldg(&r->k);
+  double x[D], kk[kScreenCoef];
+  float lim[D];
+#pragma unroll
+  for (int j = 0; j < D; ++j) {
+    lim[j] = __ldg(&r->lim[j]);
+    x[j] = __fma_rn(pts[j * P + k], __ldg(&r->sR[j]),
+                    __fma_rn(screen_index(sb[j], (kb >> (8 * j)) & 0xFFu), sA[j], __ldg(&r->sB[j])));
+  }
+#pragma unroll
+  for (int i = 0; i < kScreenCoef; ++i) kk[i] = sk[i];
+#pragma unroll
+  for (int i = 0; i < Screen<Map>::kOwnCount; ++i) kk[Screen<Map>::own(i)] = __ldg(&r->own[i]);
+  bool sure = Screen<Map>::run(kk, lim, map, x) && __ldg(&r->on) != 0u;
+  inside = true;
+#pragma unroll
+  for (int j = 0; j < D; ++j) {
+    const double p = __fma_rn(x[j], __ldg(&r->tA[j]), __ldg(&r->tB[j]));
+    const uint32_t b = uint32_t(__double2hiint(p)) - 0x41380000u, gd = __ldg(&r->guard[j]);
+    sure = sure && uint32_t(__double2loint(p)) - gd <= ~(2u * gd);
+    inside = inside && (b >> ((kb >> (8 * j)) & 0xFFu)) == 0u;
+    tb[j] = b;
+  }
+  return sure;
+}
+
 template<class Map, class Grid>
 __global__ void __launch_bounds__(256, 4) batch_screen_kernel(const BatchArgs a)
 {
@@ -325,32 +360,10 @@ __global__ void __launch_bounds__(256, 4) batch_screen_kernel(const BatchArgs a)
       if (active) {
         const uint64_t code = (__ldg(a.codes + (child >> 1)) << 1) | (child & 1u);
         const int depth = uni ? a.depth : int(__ldg(a.inst_depth + inst));
-        const ScreenRec* r = a.screen + inst;
-        const uint32_t kb = __ldg(&r->k);
         uint32_t sb[D], tb[D];
         split_code<D>(code, depth, sb);
-        double x[D], kk[kScreenCoef];
-        float lim[D];
-#pragma unroll
-        for (int j = 0; j < D; ++j) {
-          lim[j] = __ldg(&r->lim[j]);
-          x[j] = __fma_rn(pts[j * P + k], __ldg(&r->sR[j]),
-                          __fma_rn(screen_index(sb[j], (kb >> (8 * j)) & 0xFFu), a.sA[j], __ldg(&r->sB[j])));
-        }
-#pragma unroll
-        for (int i = 0; i < kScreenCoef; ++i) kk[i] = a.sk[i];
-#pragma unroll
-        for (int i = 0; i < Screen<Map>::kOwnCount; ++i) kk[Screen<Map>::own(i)] = __ldg(&r->own[i]);
-        bool sure = Screen<Map>::run(kk, lim, a.map, x) && __ldg(&r->on) != 0u, inside = true;
-#pragma unroll
-        for (int j = 0; j < D; ++j) {
-          const double p = __fma_rn(x[j], __ldg(&r->tA[j]), __ldg(&r->tB[j]));
-          const uint32_t b = uint32_t(__double2hiint(p)) - 0x41380000u, gd = __ldg(&r->guard[j]);
-          sure = sure && uint32_t(__double2loint(p)) - gd <= ~(2u * gd);
-          inside = inside && (b >> ((kb >> (8 * j)) & 0xFFu)) == 0u;
-          tb[j] = b;
-        }
-        if (!sure) {
+        bool inside;
+        if (!screened_point<Map>(a.screen + inst, a.sk, a.sA, a.map, pts, P, k, sb, tb, inside)) {
           const uint64_t cc[1] = {child};
           const uint32_t ck[1] = {k}, ci[1] = {inst};
           const bool ca[1] = {true};
@@ -452,8 +465,12 @@ __global__ void copy_finished_kernel(const uint64_t* code, const uint8_t* flags,
   }
 }
 
-template<class Map, class Grid>
-__global__ void __launch_bounds__(256) batch_rows_kernel(const BatchRowArgs a)
+// Bound by FP64 issue.  kScreen: with the screened evaluation of the instance's last step;
+// the matrices of 32 Lorenz instances of depths 18 to 22 (5^3 points a box) take 3.35 ms
+// against 3.86 (FMA) and 5.57 (strict), of 16 forced Duffing ones of depths 15 to 18 0.82
+// against 1.32.  A record serves a whole row, so its fields are read from L1 per point.
+template<class Map, class Grid, bool kScreen>
+__global__ void __launch_bounds__(256, kScreen ? 4 : 1) batch_rows_kernel(const BatchRowArgs a)
 {
   constexpr int D = Map::D;
   __shared__ uint32_t off_s[kMaxInstances + 1];
@@ -473,23 +490,46 @@ __global__ void __launch_bounds__(256) batch_rows_kernel(const BatchRowArgs a)
     const int depth = a.depths[sp];
     const uint64_t code = a.codes[row];
     const uint32_t n_i = off_s[inst + 1] - off_s[inst];
+    // the image's code by the map's own arithmetic; whether it lies in the domain
     MapParams mp = a.map;
-#pragma unroll
-    for (int q = 0; q < 6; ++q) mp.p[q] = a.params[size_t(sp) * 6 + q];
     double cc[D], r[D];
-    box_coordinates<D>(a.dom, code, depth, cc, r);
+    auto own = [&]() {
+#pragma unroll
+      for (int q = 0; q < 6; ++q) mp.p[q] = a.params[size_t(sp) * 6 + q];
+      box_coordinates<D>(a.dom, code, depth, cc, r);
+    };
+    auto own_code = [&](uint32_t k, uint64_t& tcode) {
+      double x[D], y[D];
+#pragma unroll
+      for (int j = 0; j < D; ++j) x[j] = __dadd_rn(cc[j], __dmul_rn(pts[j * P + k], r[j]));
+      if constexpr (kScreen) Map::apply_cold(mp, x, y);
+      else Map::apply(mp, x, y);
+      return point_code<D>(a.dom, y, depth, tcode);
+    };
+    uint32_t sb[D];
+    if constexpr (kScreen) split_code<D>(code, depth, sb);
+    else own();
 #pragma unroll 1
     for (int q = 0; q < 4; ++q) {
       const uint32_t k = uint32_t(lane) + 32u * q;
       uint32_t key = kPadKey;
       if (k < P) {
-        double x[D], y[D];
-#pragma unroll
-        for (int j = 0; j < D; ++j) x[j] = __dadd_rn(cc[j], __dmul_rn(pts[j * P + k], r[j]));
-        Map::apply(mp, x, y);
         uint64_t tcode = 0;
         uint32_t t = kInvalidIndex;
-        if (point_code<D>(a.dom, y, depth, tcode)) {
+        bool inside;
+        if constexpr (kScreen) {
+          uint32_t tb[D];
+          if (screened_point<Map>(a.screen + (size_t(depth - 1) * a.screen_stride + sp), a.sk, a.sA, a.map, pts, P, k,
+                                  sb, tb, inside)) {
+            if (inside) tcode = join_code<D>(tb, depth);
+          } else {
+            own();
+            inside = own_code(k, tcode);
+          }
+        } else {
+          inside = own_code(k, tcode);
+        }
+        if (inside) {
           const uint32_t g = hash_locate(a.hash, nrows, inst_key(inst, tcode));
           if (g != kInvalidIndex) t = g - off_s[inst];
         } else if (a.codes[off_s[inst] + n_i - 1] == 0) {
@@ -640,10 +680,16 @@ cudaError_t launch_batch_rows(uint32_t map_kind, uint32_t arith, uint32_t grid_k
   return batch_dispatch(map_kind, arith, grid_kind, [&](auto map, auto grid) -> cudaError_t {
     using Map = decltype(map);
     using Grid = decltype(grid);
-    const void* k = (const void*)batch_rows_kernel<Map, Grid>;
-    const int g = std::max(1, std::min<int>(batch_grid(k, 256), int((uint64_t(max_rows) + 7) / 8)));
-    batch_rows_kernel<Map, Grid><<<g, 256, 0, s>>>(a);
-    return cudaGetLastError();
+    auto launch = [&](auto screened) -> cudaError_t {
+      constexpr bool kScreen = decltype(screened)::value;
+      const void* k = (const void*)batch_rows_kernel<Map, Grid, kScreen>;
+      const int g = std::max(1, std::min<int>(batch_grid(k, 256), int((uint64_t(max_rows) + 7) / 8)));
+      batch_rows_kernel<Map, Grid, kScreen><<<g, 256, 0, s>>>(a);
+      return cudaGetLastError();
+    };
+    if constexpr (Screen<Map>::kOk)
+      if (a.screen) return launch(std::true_type{});
+    return launch(std::false_type{});
   });
 }
 
@@ -1271,6 +1317,12 @@ b12g_status b12g_batch_transition_matrices(b12g_batch* b, int absolute, int inva
   ra.stage_col = b->stage_col.p;
   ra.stage_cnt = b->stage_cnt.p;
   ra.row_count = b->row_count.p;
+  if (b->screen_common.on) {
+    ra.screen = b->screen.p;
+    ra.screen_stride = b->N;
+    for (int i = 0; i < kScreenCoef; ++i) ra.sk[i] = b->screen_common.k[i];
+    for (int j = 0; j < 3; ++j) ra.sA[j] = b->screen_common.sA[j];
+  }
   CK(launch_batch_rows(b->scheme.map.kind, b->scheme.map.arith, b->scheme.grid.kind, ra, rows, b->stream));
   CK(exclusive_scan_u32(b->row_count.p, b->rowptr.p, b->arena_off.p + b->N, b->tiles_a.p, rows, b->stream));
   uint32_t nnz = 0;

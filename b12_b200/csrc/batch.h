@@ -84,6 +84,11 @@ struct BatchRowArgs {
   uint32_t* stage_col;
   uint32_t* stage_cnt;
   uint32_t* row_count;
+  // the screened evaluation (null: the map's own arithmetic): a record per depth and sorted
+  // position, screen_stride a depth, with the launch's coefficients as in BatchArgs
+  const ScreenRec* screen;
+  uint32_t screen_stride;
+  double sk[kScreenCoef], sA[3];
 };
 
 // the image kernel's launch shape for a map family: the autotuned one when a batch of

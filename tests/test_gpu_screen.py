@@ -165,6 +165,35 @@ def test_batches_and_served_jobs_equal_single_trees(which):
     b.close()
 
 
+@pytest.mark.parametrize("name,n,full", [("lorenz", 1, False), ("lorenz", 2, True), ("lorenz", 3, False),
+                                         ("lorenz", 5, False), ("forced", 6, False), ("forced", 11, True)])
+def test_batch_matrices_keep_lost_points(name, n, full):
+    """Rows of 1 to 125 points, counts or shares, with the lost column, against the oracle."""
+    import b12_b200 as B
+    depths = [11, 4, 8]
+    if name == "lorenz":
+        params = [(10.0, r, 8.0 / 3.0) for r in (28.0, 33.0, 24.5)]
+        specs, maps = [lorenz(rho=p[1], fma=1) for p in params], [B.lorenz(*p, fma=True) for p in params]
+    else:
+        params = [(0.25, -1.0, 1.0, g) for g in (0.3, 0.1, 0.4)]
+        specs, maps = [forced(p=p) for p in params], [B.forced_duffing(200, *p) for p in params]
+    grid = B.full_grid(n, 0.1) if full else B.inner_grid(n)
+    spec_grid = dict(kind=O.GRID_FULL if full else O.GRID_INNER, n=n, eps=0.1 if full else 0.0)
+    b = B.Batch(specs[0]["center"], specs[0]["radius"], B.Scheme(maps[0], grid), params, depths)
+    b.run()
+    for absolute in (False, True):
+        b.transition_matrices(absolute, True)
+        for i, d in enumerate(depths):
+            o = O.Oracle(dict(specs[i], grid=spec_grid))
+            want, _ = o.subdivision(d)
+            assert list(b.counts(i)) == list(want)
+            if want.min() == 0 or o.n == 1:
+                continue               # every box was lost: no rows are kept
+            for x, y in zip(b.csr(i), o.transition_matrix(absolute, True)):
+                assert np.array_equal(x, y)
+    b.close()
+
+
 @pytest.mark.parametrize("case,depth", [(0, 4), (0, 24), (0, 50), (1, 21), (2, 17), (3, 20), (4, 13), (4, 25), (5, 16),
                                         (6, 23), (6, 60), (7, 18)])
 def test_leaves_of_several_depths(case, depth):
