@@ -186,6 +186,27 @@ __global__ void __launch_bounds__(kThreads, !kScreen ? 6 : M == ImageMode::Mark 
 {
   using PI = PointImage<Map, Grid>;
   __shared__ double pts[kPointTable];
+  const uint32_t n = *a.n_leaves;
+  const uint32_t nboxes = M == ImageMode::Mark ? a.n_src_value : a.n_src ? *a.n_src : (a.children ? 2u * n : n);
+  const uint64_t P = a.points;
+  const uint32_t P32 = uint32_t(P);
+  const uint64_t total = uint64_t(nboxes) * P;
+  const int lane = threadIdx.x & 31;
+  // the queue of the next launch on the tree's stream starts empty
+  if (blockIdx.x == 0 && threadIdx.x == 0) *a.work_next = 0u;
+  if (M == ImageMode::Hit && a.children && 2ull * n > a.hit_cap) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(a.error, 1u);
+    return;
+  }
+  // A device work queue (UnitQueue) of 32-point units (of 2^shift times as many where that
+  // many units would not fit 32 bits): every warp takes the next points until none is left,
+  // so that warps that run faster do more (a static grid-stride split left the slower warps
+  // alone at the end: 47 % of the warp slots were active on average, of 75 % possible).
+  constexpr uint32_t kTake = M == ImageMode::Mark ? 2 * kChunkTrips : kChunkTrips;
+  uint32_t shift = 0;
+  while (((total + 31) >> (5 + shift)) >= 0x40000000ull) ++shift;
+  UnitQueue<kTake, kFineUnits, M != ImageMode::Mark> q(a.work, uint32_t((total + (32ull << shift) - 1) >> (5 + shift)));
+  if (q.idle_block()) return;
   // Mark mode: an index's place in the box's code, by dimension, where the indices have at
   // most 8 bits (four reads and two ORs instead of 36 instructions of bit spreading)
   __shared__ uint32_t spread[M == ImageMode::Mark ? Map::D * 256 : 1];
@@ -201,18 +222,6 @@ __global__ void __launch_bounds__(kThreads, !kScreen ? 6 : M == ImageMode::Mark 
   }
   const bool table = load_points<Grid, Map::D>(a.grid, a.points, pts);   // (ends with a block barrier)
 
-  const uint32_t n = *a.n_leaves;
-  const uint32_t nboxes = M == ImageMode::Mark ? a.n_src_value : a.n_src ? *a.n_src : (a.children ? 2u * n : n);
-  const uint64_t P = a.points;
-  const uint32_t P32 = uint32_t(P);
-  const uint64_t total = uint64_t(nboxes) * P;
-  const int lane = threadIdx.x & 31;
-  // the queue of the next launch on the tree's stream starts empty
-  if (blockIdx.x == 0 && threadIdx.x == 0) *a.work_next = 0u;
-  if (M == ImageMode::Hit && a.children && 2ull * n > a.hit_cap) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(a.error, 1u);
-    return;
-  }
   // Mark mode: the warp's new boxes (the same in every lane), added to the launch's count at
   // the end (an atomic for every warp with a new box held the continuation's image launches
   // at 10.8 ms; without them 9.6)
@@ -313,27 +322,8 @@ __global__ void __launch_bounds__(kThreads, !kScreen ? 6 : M == ImageMode::Mark 
     }
   };
 
-  // A device work queue: every warp takes the next points until none is left, so that warps
-  // that run ahead take more work and the SM stays full to the end (a static split leaves
-  // the slower warps alone at the end: 47 % of the warp slots were active on average, of
-  // 75 % possible).  The queue counts units of 32 points (of 2^shift times as many where
-  // that many units would not fit 32 bits); a warp takes kChunkTrips units at a time while
-  // at least kFineUnits units a warp are left, and single ones after that: a warp works
-  // through its units one after another, so in a small launch, and at the end of a large
-  // one, larger pieces would leave the others idle (the small steps of a forced Duffing job
-  // took 68 us with four points a lane, 25 us with one).
-  constexpr uint32_t kTake = M == ImageMode::Mark ? 2 * kChunkTrips : kChunkTrips;
-  uint32_t shift = 0;
-  while (((total + 31) >> (5 + shift)) >= 0x40000000ull) ++shift;
-  const uint32_t units = uint32_t((total + (32ull << shift) - 1) >> (5 + shift));
-  const uint32_t fine = gridDim.x * (kThreads / 32) * kFineUnits;
-  const uint32_t coarse_end = units > fine ? units - fine : 0;
-  uint32_t c = 0;
-  for (;;) {
-    const uint32_t size = c < coarse_end ? kTake : 1u;
-    if (lane == 0) c = atomicAdd(a.work, size);
-    c = __shfl_sync(0xFFFFFFFFu, c, 0);
-    if (c >= units) break;
+  for (bool more = q.any(); more; more = q.next()) {
+    const uint32_t c = q.at, size = q.size;
     // (sources and points per box both fit 32 bits: the rank and the point index do)
     const uint64_t g = (uint64_t(c) << (5 + shift)) + uint64_t(lane);
     uint32_t rank, k;

@@ -92,6 +92,13 @@ def test_work_queue_sizes(n):
     t.close()
 
 
+@pytest.mark.parametrize("n", [14207, 14208, 14209, 14300, 113663, 113664, 113665, 130000])
+def test_work_queue_first_pieces(n):
+    """7,104 warps: as many units of 32 points as warps (14,208 boxes of 16 points) need no
+    counter, 8 times as many start with larger first pieces."""
+    test_work_queue_sizes(n)
+
+
 def test_queue_turns_through_graphs_and_single_launches():
     """Fused runs (an odd and an even number of launches) between single launches."""
     spec = O.henon_spec()
