@@ -1037,6 +1037,22 @@ b12g_status b12g_csr_measure(const b12g_csr* m, double* v)
 }
 
 // ---- fused subdivision loop --------------------------------------------------------------
+}  // extern "C"
+
+namespace {
+
+// whether b12g_tree_refuse_graph asked for this stage to fail (once)
+bool refused(b12g_tree* t, int stage)
+{
+  if (t->refuse_graph != stage) return false;
+  t->refuse_graph = 0;
+  return true;
+}
+
+}  // namespace
+
+extern "C" {
+
 b12g_status b12g_subdivision_run(b12g_tree* t, const b12g_scheme* sc, uint32_t steps, uint32_t* counts)
 {
   if (!t || !sc) return fail(B12G_ERR_INVALID, "NULL argument");
@@ -1119,9 +1135,12 @@ b12g_status b12g_subdivision_run(b12g_tree* t, const b12g_scheme* sc, uint32_t s
       int cur = t->cur, ncur = t->ncur;
       cudaError_t err = cudaSuccess;
       // both work-queue counters start empty at every replay, whose first launch takes the
-      // first of them
+      // first of them.  The capture counts its launches' turns in a word of its own: the
+      // tree's turn belongs to the launches that ran, and stays as it is when the graph
+      // cannot be made or launched.
       err = cudaMemsetAsync(t->ctr.p + C_WORK, 0, 2 * sizeof(uint32_t), t->stream);
-      t->work_turn = 0;
+      unsigned turn = 0;
+      pr.a.work_turn = &turn;
       // the lookup table starts clean at every replay; step s builds with tag s + 1
       if (use_hash && err == cudaSuccess) err = cudaMemsetAsync(t->hash.p, 0, t->hash.n * sizeof(ulonglong2), t->stream);
       for (uint32_t s = 0; s < steps && err == cudaSuccess; ++s) {
@@ -1169,7 +1188,7 @@ b12g_status b12g_subdivision_run(b12g_tree* t, const b12g_scheme* sc, uint32_t s
       cudaError_t e2 = cudaStreamEndCapture(t->stream, &g);
       if (err != cudaSuccess) { if (g) cudaGraphDestroy(g); return cuda_fail(err, "capture subdivision"); }
       if (e2 != cudaSuccess) return cuda_fail(e2, "end capture");
-      cudaError_t e3 = cudaGraphInstantiate(&t->sub_graph, g, 0);
+      cudaError_t e3 = refused(t, 1) ? cudaErrorMemoryAllocation : cudaGraphInstantiate(&t->sub_graph, g, 0);
       cudaGraphDestroy(g);
       if (e3 != cudaSuccess) { t->sub_graph = nullptr; return cuda_fail(e3, "instantiate"); }
       t->sub_key = key;
@@ -1183,7 +1202,7 @@ b12g_status b12g_subdivision_run(b12g_tree* t, const b12g_scheme* sc, uint32_t s
       }
     }
     ST(set_ctr(t, C_TGT, 0));
-    CK(cudaGraphLaunch(t->sub_graph, t->stream));
+    CK(refused(t, 2) ? cudaErrorMemoryAllocation : cudaGraphLaunch(t->sub_graph, t->stream));
     count_launches(t->sub_graph_kernels);
     t->work_turn = steps & 1u;
     if (use_hash) t->hash_tag = steps;
@@ -1239,6 +1258,13 @@ b12g_status b12g_subdivision_run(b12g_tree* t, const b12g_scheme* sc, uint32_t s
     return B12G_OK;
   }
   return fail(B12G_ERR_CAPACITY, "subdivision run: capacity retries exhausted");
+}
+
+b12g_status b12g_tree_refuse_graph(b12g_tree* t, int stage)
+{
+  if (!t || stage < 0 || stage > 2) return fail(B12G_ERR_INVALID, "NULL tree, or stage not 0, 1 or 2");
+  t->refuse_graph = stage;
+  return B12G_OK;
 }
 
 // ---- measurement hooks --------------------------------------------------------------------

@@ -160,6 +160,7 @@ struct b12g_tree {
   cudaGraphExec_t sub_graph = nullptr;
   std::vector<uint8_t> sub_key;
   uint64_t sub_graph_kernels = 0;
+  int refuse_graph = 0;        // b12g_tree_refuse_graph: the stage of the next run that fails
   // optional per-kernel timing: event pairs around image / transition-row launches
   bool profile = false;
   std::vector<cudaEvent_t> prof_events[2];   // [kind] start/stop pairs, reused

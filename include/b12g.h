@@ -441,6 +441,11 @@ b12g_status b12g_server_stats(b12g_server* server, uint64_t* ticks, uint64_t* bo
 b12g_status b12g_server_engine_stats(b12g_server* server, uint32_t i, uint32_t* map_kind, uint64_t* ticks,
                                      uint64_t* jobs_done, double* tick_seconds, double* finish_seconds);
 
+/* for tests of the error path: the next b12g_subdivision_run of this tree that makes a CUDA
+ * graph (stage 1) or launches one (stage 2) fails there with B12G_ERR_OOM, as on a device
+ * without memory, and no step runs; 0 takes the request back */
+b12g_status b12g_tree_refuse_graph(b12g_tree* tree, int stage);
+
 /* ---- measurement hooks (no counterpart in the reference) ---------------------------------- */
 /* the CUDA stream (cudaStream_t) every kernel of this tree runs on */
 b12g_status b12g_tree_stream(b12g_tree* tree, void** stream);
