@@ -884,7 +884,8 @@ b12g_status batch_screen_records(b12g_batch* b, const std::vector<double>& param
   if (!common.on) return B12G_OK;
   // (without memory for them, too)
   if (b->screen.ensure(rec.size(), "batch screen records") != B12G_OK) return B12G_OK;
-  CK(cudaMemcpy(b->screen.p, rec.data(), rec.size() * sizeof(ScreenRec), cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(b->screen.p, rec.data(), rec.size() * sizeof(ScreenRec), cudaMemcpyHostToDevice, b->stream));
+  CK(cudaStreamSynchronize(b->stream));
   b->screen_common = common;
   return B12G_OK;
 }
@@ -1109,17 +1110,18 @@ b12g_status b12g_batch_create(const b12g_domain* domain, const b12g_scheme* sche
   b->dom = probe->dom;
   b->scheme = *scheme;
   b->mp = pr.a.map;
+  b->mp.table = nullptr;           // a copy of its own, below
   b->gp = pr.a.grid;
   b->P = pr.P;
   b->N = n;
   std::vector<double> table;
   if (scheme->map.kind == B12G_MAP_FORCED_DUFFING) {
     table.resize(2 * size_t(scheme->map.steps) + 1);
-    cudaMemcpy(table.data(), probe->table.p, table.size() * 8, cudaMemcpyDeviceToHost);
+    const cudaError_t e = cudaMemcpy(table.data(), probe->table.p, table.size() * 8, cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) st = cuda_fail(e, "forcing table");
   }
   b12g_tree_destroy(probe);
-  st = B12G_OK;
-  if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess)
+  if (st == B12G_OK && cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess)
     st = cuda_fail(cudaGetLastError(), "stream");
   // deepest first, stable by instance index
   b->order.resize(n);
@@ -1147,18 +1149,23 @@ b12g_status b12g_batch_create(const b12g_domain* domain, const b12g_scheme* sche
   if (st == B12G_OK) st = b->fin_lo.ensure(n, "batch final offsets");
   if (st == B12G_OK) st = b->fin_len.ensure(n, "batch final offsets");
   if (st == B12G_OK) st = b->ctr.ensure(B_COUNT, "batch counters");
-  if (st == B12G_OK) {
-    cudaMemcpy(b->params.p, ps.data(), ps.size() * 8, cudaMemcpyHostToDevice);
-    cudaMemcpy(b->depths.p, b->depth_sorted.data(), n, cudaMemcpyHostToDevice);
-    cudaMemset(b->step_counts.p, 0, size_t(b->max_depth) * n * 4);
-  }
+  // (uploads go through the stream that reads them: a copy on the default stream is not
+  // ordered before the launches of this one, which does not wait for that stream)
   if (st == B12G_OK && !table.empty()) {
     double* tp = nullptr;
     if (cudaMalloc(&tp, table.size() * 8) != cudaSuccess) st = cuda_fail(cudaGetLastError(), "table");
-    else {
-      cudaMemcpy(tp, table.data(), table.size() * 8, cudaMemcpyHostToDevice);
-      b->mp.table = tp;
-    }
+    else b->mp.table = tp;
+  }
+  if (st == B12G_OK) {
+    cudaError_t e = cudaMemcpyAsync(b->params.p, ps.data(), ps.size() * 8, cudaMemcpyHostToDevice, b->stream);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(b->depths.p, b->depth_sorted.data(), n, cudaMemcpyHostToDevice, b->stream);
+    if (e == cudaSuccess && !table.empty())
+      e = cudaMemcpyAsync(const_cast<double*>(b->mp.table), table.data(), table.size() * 8, cudaMemcpyHostToDevice,
+                          b->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(b->step_counts.p, 0, size_t(b->max_depth) * n * 4, b->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
+    if (e != cudaSuccess) st = cuda_fail(e, "batch parameters");
   }
   if (st == B12G_OK) st = batch_reserve(b, std::max<uint64_t>(1ull << 22, 4ull * n));
   if (st == B12G_OK) st = batch_screen_records(b, ps);

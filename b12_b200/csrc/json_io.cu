@@ -402,9 +402,14 @@ b12g_status b12g_csr_load_json(const char* path, b12g_csr** out)
   if (st == B12G_OK) st = m->vals.ensure(std::max<uint64_t>(m->nnz, 1), "vals");
   if (st == B12G_OK) st = m->ctr.ensure(256, "csr counters");
   if (st == B12G_OK) {
-    cudaError_t e = cudaMemcpy(m->rowptr.p, f.rowptr.data(), f.rowptr.size() * 4, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && m->nnz) e = cudaMemcpy(m->cols.p, f.cols.data(), m->nnz * 4, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && m->nnz) e = cudaMemcpy(m->vals.p, f.vals.data(), m->nnz * 8, cudaMemcpyHostToDevice);
+    // (through the stream that reads them, which does not wait for the default stream)
+    cudaStream_t s = m->stream;
+    cudaError_t e = cudaMemcpyAsync(m->rowptr.p, f.rowptr.data(), f.rowptr.size() * 4, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess && m->nnz)
+      e = cudaMemcpyAsync(m->cols.p, f.cols.data(), m->nnz * 4, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess && m->nnz)
+      e = cudaMemcpyAsync(m->vals.p, f.vals.data(), m->nnz * 8, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) st = cuda_fail(e, "csr upload");
   }
   if (st != B12G_OK) {

@@ -319,6 +319,7 @@ b12g_status engine_reserve(Engine* e, uint64_t parents);
 b12g_status engine_init(Engine* e, const b12g_job& key)
 {
   e->key = key;
+  CK(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
   b12g_tree* probe = nullptr;
   ST(b12g_tree_create(&key.domain, &probe));
   b12g_scheme sc{};
@@ -333,10 +334,13 @@ b12g_status engine_init(Engine* e, const b12g_job& key)
     e->gp = pr.a.grid;
     e->P = pr.P;
     if (key.map.kind == B12G_MAP_FORCED_DUFFING) {
-      // the engine keeps its own copy of the forcing table
+      // the engine keeps its own copy of the forcing table (made on the engine's stream, which
+      // does not wait for the default one)
       const size_t n = 2 * size_t(key.map.steps) + 1;
       if (cudaMalloc(&e->table, n * sizeof(double)) != cudaSuccess ||
-          cudaMemcpy(e->table, probe->table.p, n * sizeof(double), cudaMemcpyDeviceToDevice) != cudaSuccess)
+          cudaMemcpyAsync(e->table, probe->table.p, n * sizeof(double), cudaMemcpyDeviceToDevice, e->stream) !=
+              cudaSuccess ||
+          cudaStreamSynchronize(e->stream) != cudaSuccess)
         st = cuda_fail(cudaGetLastError(), "forcing table");
       e->mp.table = e->table;
     }
@@ -346,7 +350,6 @@ b12g_status engine_init(Engine* e, const b12g_job& key)
   if (e->P > kMaxRowPoints)
     return fail(B12G_ERR_CAPACITY, "served jobs take up to %u grid points per box", kMaxRowPoints);
   e->tuning = batch_tuning(e->srv->device, key.map.kind, key.map.arith, key.grid.kind, key.domain.dim);
-  CK(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
   CK(cudaMallocHost(&e->h, kHostWords * 4));
   CK(cudaMallocHost(&e->hp, size_t(kMaxSlots) * 6 * 8));
   CK(cudaMallocHost(&e->hd, 2 * size_t(kMaxSlots)));
