@@ -15,7 +15,8 @@
 //   4. new offsets; instances whose depth is reached move to the final arena.
 // All launches read their sizes from device memory: the whole run is one CUDA graph.
 // batch_image_kernel's block size, points per thread and chunk size are chosen by timing
-// the candidates on the first run (autotuner); batch_screen_kernel has one shape.
+// the candidates on the first run (autotuner) of a batch with steps it runs;
+// batch_screen_kernel has one shape.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -278,13 +279,15 @@ constexpr uint32_t kScreenTrips = 4, kScreenFine = 4;
 
 // test point k of the box with indices sb, by an instance's record and the launch's
 // coefficients: the image's indices and whether it lies in the domain; returns whether both
-// are certain
+// are certain (never for an instance that the bound does not cover at its depth: nothing is
+// evaluated for it here)
 template<class Map>
 __device__ __forceinline__ bool screened_point(const ScreenRec* r, const double* sk, const double* sA,
                                                const MapParams& map, const double* pts, uint32_t P, uint32_t k,
                                                const uint32_t (&sb)[Map::D], uint32_t (&tb)[Map::D], bool& inside)
 {
   constexpr int D = Map::D;
+  if (__ldg(&r->on) == 0u) return false;
   const uint32_t kb = __ldg(&r->k);
   double x[D], kk[kScreenCoef];
   float lim[D];
@@ -298,7 +301,7 @@ __device__ __forceinline__ bool screened_point(const ScreenRec* r, const double*
   for (int i = 0; i < kScreenCoef; ++i) kk[i] = sk[i];
 #pragma unroll
   for (int i = 0; i < Screen<Map>::kOwnCount; ++i) kk[Screen<Map>::own(i)] = __ldg(&r->own[i]);
-  bool sure = Screen<Map>::run(kk, lim, map, x) && __ldg(&r->on) != 0u;
+  bool sure = Screen<Map>::run(kk, lim, map, x);
   inside = true;
 #pragma unroll
   for (int j = 0; j < D; ++j) {
@@ -778,6 +781,8 @@ struct b12g_batch {
   Buf<double> params;                  // sorted order
   Buf<ScreenRec> screen;               // a record an instance and step (max_depth x N), when screened
   ScreenArgs screen_common{};
+  std::vector<uint8_t> screen_step;    // whether step k runs screened (k = 0..max_depth)
+  std::vector<uint8_t> screen_last;    // whether the bound covers an instance's last step (sorted order)
   Buf<uint8_t> depths;                 // sorted order
   Buf<uint64_t> code[2];
   Buf<uint8_t> flags[2];
@@ -864,10 +869,18 @@ b12g_status batch_reset(b12g_batch* b)
 }
 
 // the records of every step: all instances share their map's coefficients but for their own
-// (rho of Lorenz, gamma of forced Duffing), else the batch runs the maps' own arithmetic
+// (rho of Lorenz, gamma of forced Duffing), else the batch runs the maps' own arithmetic.
+// A step runs screened where the bound covers at least half of its instances
+// (screen_covers): the bound ends at a depth (26 for the usual forced Duffing map), and the
+// steps past it keep the tuned shape of batch_image_kernel (8 forced instances of depth 29:
+// 190 ms, 235 with all steps in it).  An instance past the bound costs a screened launch its
+// own arithmetic only, so half is on the safe side: 16 Lorenz instances of depth 22, 8 of
+// them past it, run in 5.8 ms against 13.6 (strict) and 9.6 (FMA).
 b12g_status batch_screen_records(b12g_batch* b, const std::vector<double>& params)
 {
   std::vector<ScreenRec> rec(size_t(b->max_depth) * b->N);
+  std::vector<uint32_t> on(size_t(b->max_depth) + 1, 0);
+  std::vector<uint8_t> last(b->N, 0);
   ScreenArgs common{};
   for (uint32_t q = 0; q < b->N; ++q) {
     MapParams mp = b->mp;
@@ -879,6 +892,8 @@ b12g_status batch_screen_records(b12g_batch* b, const std::vector<double>& param
       screen_at(plan, int(k), s);
       if (!screen_record(b->scheme.map.kind, int(b->domain.dim), s, common, rec[size_t(k - 1) * b->N + q]))
         return B12G_OK;
+      on[k] += s.on ? 1u : 0u;
+      last[q] = s.on ? 1 : 0;
     }
   }
   if (!common.on) return B12G_OK;
@@ -887,12 +902,17 @@ b12g_status batch_screen_records(b12g_batch* b, const std::vector<double>& param
   CK(cudaMemcpyAsync(b->screen.p, rec.data(), rec.size() * sizeof(ScreenRec), cudaMemcpyHostToDevice, b->stream));
   CK(cudaStreamSynchronize(b->stream));
   b->screen_common = common;
+  b->screen_step.assign(size_t(b->max_depth) + 1, 0);
+  for (uint32_t k = 1; k <= b->max_depth; ++k) b->screen_step[k] = screen_covers(on[k], b->active[k]) ? 1 : 0;
+  b->screen_last = std::move(last);
   return B12G_OK;
 }
 
+bool step_screened(const b12g_batch* b, uint32_t k) { return !b->screen_step.empty() && b->screen_step[k] != 0; }
+
 void batch_screen(const b12g_batch* b, uint32_t k, BatchArgs& a)
 {
-  if (!b->screen_common.on) return;
+  if (!step_screened(b, k)) return;
   a.screen = b->screen.p + size_t(k - 1) * b->N;
   for (int i = 0; i < kScreenCoef; ++i) a.sk[i] = b->screen_common.k[i];
   for (int j = 0; j < 3; ++j) a.sA[j] = b->screen_common.sA[j];
@@ -975,7 +995,8 @@ uint64_t step_kernels(const b12g_batch* b, uint32_t k)
   return 4 + compact_launches(true, capu) + (b->active[k + 1] < b->active[k] ? 1 : 0);
 }
 
-// time every candidate shape on the batch's own steps (first run) and keep the fastest
+// time every candidate shape on the batch's own steps (first run; those that
+// batch_image_kernel runs) and keep the fastest
 b12g_status autotune(b12g_batch* b)
 {
   const Tuning all[] = {{256, 1, 8192}, {256, 2, 8192}, {128, 1, 8192}, {512, 1, 16384}, {256, 1, 32768},
@@ -995,7 +1016,8 @@ b12g_status autotune(b12g_batch* b)
     uint32_t parents = 0;
     CK(cudaMemcpyAsync(&parents, b->off[in].p + A, 4, cudaMemcpyDeviceToHost, b->stream));
     CK(cudaStreamSynchronize(b->stream));
-    if (2ull * parents * b->P >= (1ull << 22)) {
+    const bool timed = 2ull * parents * b->P >= (1ull << 22) && !step_screened(b, k);
+    if (timed) {
       for (size_t c = 0; c < total.size(); ++c) {
         BatchArgs a{};
         a.dom = b->dom; a.map = b->mp; a.grid = b->gp; a.points = b->P; a.params = b->params.p;
@@ -1016,7 +1038,7 @@ b12g_status autotune(b12g_batch* b)
       }
     }
     // the real step (with the default shape; the hit marks of the trials are the same)
-    CK(enqueue_step(b, k, b->tuning, /*with_hash=*/!(2ull * parents * b->P >= (1ull << 22))));
+    CK(enqueue_step(b, k, b->tuning, /*with_hash=*/!timed));
     CK(cudaStreamSynchronize(b->stream));
   }
   cudaEventDestroy(e0);
@@ -1176,7 +1198,9 @@ b12g_status b12g_batch_create(const b12g_domain* domain, const b12g_scheme* sche
     auto it = g_tuned.find(tune_key(b->device, scheme->map.kind, scheme->map.arith, scheme->grid.kind));
     if (it != g_tuned.end()) { b->tuning = it->second; b->tuned = true; }
   }
-  if (b->screen_common.on) {       // the screened kernel has one shape
+  bool all_screened = !b->screen_step.empty();
+  for (uint32_t k = 1; k <= b->max_depth; ++k) all_screened = all_screened && step_screened(b, k);
+  if (all_screened) {              // the screened kernel has one shape
     b->tuning = Tuning{256, 1, 32 * kScreenTrips};
     b->tuned = true;
   }
@@ -1324,7 +1348,9 @@ b12g_status b12g_batch_transition_matrices(b12g_batch* b, int absolute, int inva
   ra.stage_col = b->stage_col.p;
   ra.stage_cnt = b->stage_cnt.p;
   ra.row_count = b->row_count.p;
-  if (b->screen_common.on) {
+  uint64_t rows_on = 0;
+  for (uint32_t q = 0; q < b->N && !b->screen_last.empty(); ++q) rows_on += b->screen_last[q] ? b->h_fin_len[q] : 0u;
+  if (screen_covers(rows_on, rows)) {
     ra.screen = b->screen.p;
     ra.screen_stride = b->N;
     for (int i = 0; i < kScreenCoef; ++i) ra.sk[i] = b->screen_common.k[i];

@@ -362,5 +362,8 @@ double grid_reach(uint32_t grid_kind, const GridParams& g);
 // the record of a batched instance; false where it cannot share `common`'s coefficients and
 // scales (common.on == 0: the first one, which sets them)
 bool screen_record(uint32_t map_kind, int dim, const ScreenArgs& s, ScreenArgs& common, ScreenRec& rec);
+// whether a batched launch of `all` instances (or boxes) runs screened when the bound covers
+// `on` of them
+inline bool screen_covers(uint64_t on, uint64_t all) { return on > 0 && 2 * on >= all; }
 
 }  // namespace b12g

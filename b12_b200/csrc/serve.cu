@@ -673,15 +673,21 @@ b12g_status engine_tick(Engine* e, const std::vector<Job*>& joining)
   a.targets = store ? e->targets.p : nullptr;
   a.tgt_base = store ? e->tgt_base.p : nullptr;
   // the jobs' records at their children's depths; jobs that do not share their coefficients
-  // run the map's own arithmetic
+  // run the map's own arithmetic, and so does a tick whose boxes belong mostly to jobs past
+  // the bound
   ScreenArgs common{};
   bool shared = true;
+  uint64_t boxes_on = 0, boxes_all = 0;
   for (uint32_t i = 0; i < A && shared; ++i) {
+    const Job* j = e->slots[i];
+    const uint64_t boxes = j->counts.empty() ? 1u : j->counts.back();
     ScreenArgs sa{};
     screen_at(e->slots[i]->plan, int(e->hd[i]), sa);
     shared = screen_record(e->key.map.kind, int(e->key.domain.dim), sa, common, e->hs[i]);
+    boxes_all += boxes;
+    if (sa.on) boxes_on += boxes;
   }
-  if (shared && common.on) {
+  if (shared && screen_covers(boxes_on, boxes_all)) {
     CK(cudaMemcpyAsync(e->screen.p, e->hs, size_t(A) * sizeof(ScreenRec), cudaMemcpyHostToDevice, e->stream));
     a.screen = e->screen.p;
     for (int i = 0; i < kScreenCoef; ++i) a.sk[i] = common.k[i];

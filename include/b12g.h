@@ -365,8 +365,9 @@ b12g_status b12g_json_read_coo(const char* path, uint32_t* n_rows, uint32_t* n_c
  * kind, grid and arithmetic but per-instance map parameters and depths, advanced in
  * lockstep on one GPU: one persistent launch per subdivision step serves every
  * instance still subdividing, fed by a device work queue of points; the steps
- * run as one CUDA graph; the launch shape of maps that run their own arithmetic alone is
- * autotuned on the first run.  The reference runs such scans one ImplicitBoxTree at a time.  Inner and full grids only. */
+ * run as one CUDA graph; the launch shape of the steps that run the map's own arithmetic
+ * alone is autotuned on the first run.  The reference runs such scans one ImplicitBoxTree at
+ * a time.  Inner and full grids only. */
 typedef struct b12g_batch b12g_batch;
 /* params: n x 6 map parameters (b12g_map.p per instance); depths: n target depths 1..32 */
 b12g_status b12g_batch_create(const b12g_domain* domain, const b12g_scheme* scheme, uint32_t n,
