@@ -231,6 +231,7 @@ b12g_status prepare(b12g_tree* t, const b12g_scheme* sc, Prepared& pr)
   a.cand_count = t->ctr.p + C_CAND;
   a.work = t->ctr.p + C_WORK;
   a.work_turn = &t->work_turn;
+  a.plan = &t->plan;
   return B12G_OK;
 }
 

@@ -539,7 +539,7 @@ cudaError_t launch_image(uint32_t map_kind, uint32_t arith, uint32_t grid_kind, 
   b.work = a.work + (*a.work_turn & 1u);
   b.work_next = a.work + ((*a.work_turn & 1u) ^ 1u);
   fill_depth_const(b.dom, int(dim), b.depth, b.dc);
-  fill_screen(map_kind, b.map, b.dom, int(dim), b.depth, grid_reach(grid_kind, b.grid), b.sc);
+  fill_screen(map_kind, b.map, b.dom, int(dim), b.depth, grid_reach(grid_kind, b.grid), b.plan, b.sc);
   return dispatch(map_kind, arith, grid_kind, dim, [&](auto map, auto grid) {
     using Map = decltype(map);
     using Grid = decltype(grid);
@@ -558,7 +558,8 @@ cudaError_t launch_rows(uint32_t map_kind, uint32_t arith, uint32_t grid_kind, u
 {
   RowArgs b = a;
   fill_depth_const(b.img.dom, int(dim), b.img.depth, b.img.dc);
-  fill_screen(map_kind, b.img.map, b.img.dom, int(dim), b.img.depth, grid_reach(grid_kind, b.img.grid), b.img.sc);
+  fill_screen(map_kind, b.img.map, b.img.dom, int(dim), b.img.depth, grid_reach(grid_kind, b.img.grid), b.img.plan,
+              b.img.sc);
   return dispatch(map_kind, arith, grid_kind, dim, [&](auto map, auto grid) {
     using Map = decltype(map);
     using Grid = decltype(grid);

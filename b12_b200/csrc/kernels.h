@@ -30,6 +30,7 @@ struct ImageArgs {
   int depth;                 // depth of the imaged boxes (children depth in children mode)
   DepthConst dc;             // constants of `depth` (launch_image / launch_rows fill them in)
   ScreenArgs sc;             // the screened evaluation's (filled in by the same)
+  ScreenPlan* plan;          // null, or the plan the stream's owner keeps for it (host use)
   int children;              // 1: boxes are the 2n children of `codes`, never materialised
   const uint32_t* src;       // source leaf ranks -> leaf index (nullptr: all leaves)
   const uint32_t* n_src;     // device count of sources (nullptr: all leaves / children)

@@ -1171,7 +1171,8 @@ b12g_status mixed_screen(b12g_tree* t, const b12g_scheme* sc, MixedArgs& a)
 {
   if (a.src_depth || t->depth == 0) return B12G_OK;
   a.depth = int(t->depth);
-  fill_screen(sc->map.kind, a.map, a.dom, int(t->domain.dim), a.depth, grid_reach(sc->grid.kind, a.grid), a.sc);
+  fill_screen(sc->map.kind, a.map, a.dom, int(t->domain.dim), a.depth, grid_reach(sc->grid.kind, a.grid), &t->plan,
+              a.sc);
   if (!a.sc.on) return B12G_OK;
   const size_t need = size_t(std::max<uint32_t>(t->n, 1)) * kSrcStride;
   if (t->srcc.ensure_room(need, "leaf centres", 2) != B12G_OK && t->srcc.ensure(need, "leaf centres") != B12G_OK) {

@@ -337,7 +337,7 @@ struct MapBound {
 
 // The depth-independent part of a screen: a map's bounds over multiples of the domain (found
 // when a depth first asks for them) and its coefficients.
-constexpr int kScreenBoxes = 6;
+constexpr int kScreenBoxes = 7;
 struct ScreenPlan {
   uint32_t kind = 0;
   MapParams map{};
@@ -345,6 +345,7 @@ struct ScreenPlan {
   int dim = 0;
   double gmax = 0.0;
   bool possible = false;
+  bool wide = false;           // box 0 goes beyond the others
   bool found[kScreenBoxes] = {};
   MapBound bound[kScreenBoxes];
   double k[kScreenCoef] = {};
@@ -354,9 +355,10 @@ ScreenPlan screen_plan(uint32_t map_kind, const MapParams& map, const Domain& do
 // fills `s` for launches over boxes of `depth`; s.on tells whether the screened evaluation
 // applies (screen.cu states when)
 void screen_at(ScreenPlan& plan, int depth, ScreenArgs& s);
-// both at once
+// both at once; plan: null, or one kept for launches in this domain, made again when the map
+// or the reach is another (a tree's: its launches are not called from several threads)
 void fill_screen(uint32_t map_kind, const MapParams& map, const Domain& dom, int dim, int depth, double gmax,
-                 ScreenArgs& s);
+                 ScreenPlan* plan, ScreenArgs& s);
 // the largest |coordinate| of a grid's points
 double grid_reach(uint32_t grid_kind, const GridParams& g);
 // the record of a batched instance; false where it cannot share `common`'s coefficients and

@@ -126,6 +126,7 @@ struct b12g_tree {
   Buf<uint8_t> flags[2];
   Buf<uint8_t> hit;
   Buf<uint32_t> ctr;
+  b12g::ScreenPlan plan;       // of the last screened map (depth-independent part)
   unsigned work_turn = 0;      // which of the work-queue counters the next image launch takes
   Buf<uint32_t> tiles_a, tiles_b;
   Buf<uint32_t> src, out, stage_col, stage_cnt, row_count, rowptr;
