@@ -279,15 +279,13 @@ constexpr uint32_t kScreenTrips = 4, kScreenFine = 4;
 
 // test point k of the box with indices sb, by an instance's record and the launch's
 // coefficients: the image's indices and whether it lies in the domain; returns whether both
-// are certain (never for an instance that the bound does not cover at its depth: nothing is
-// evaluated for it here)
+// are certain (an instance that the bound does not cover at its depth has no record: `on` is 0)
 template<class Map>
 __device__ __forceinline__ bool screened_point(const ScreenRec* r, const double* sk, const double* sA,
                                                const MapParams& map, const double* pts, uint32_t P, uint32_t k,
                                                const uint32_t (&sb)[Map::D], uint32_t (&tb)[Map::D], bool& inside)
 {
   constexpr int D = Map::D;
-  if (__ldg(&r->on) == 0u) return false;
   const uint32_t kb = __ldg(&r->k);
   double x[D], kk[kScreenCoef];
   float lim[D];
@@ -341,6 +339,7 @@ __global__ void __launch_bounds__(256, 4) batch_screen_kernel(const BatchArgs a)
   const uint32_t fine = gridDim.x * (256 / 32) * kScreenFine;
   const uint32_t coarse_end = units > fine ? units - fine : 0;
   uint32_t c = 0;
+  ScreenTrial trial;
   for (;;) {
     const uint32_t size = c < coarse_end ? kScreenTrips : 1u;
     if (lane == 0) c = atomicAdd(a.queue, size);
@@ -356,17 +355,24 @@ __global__ void __launch_bounds__(256, 4) batch_screen_kernel(const BatchArgs a)
       k = uint32_t(g - uint64_t(child) * P);
     }
     uint32_t inst = find_instance(off_s, a.n_inst, child >> 1);
+    uint32_t undecided = 0;
 #pragma unroll 1
     for (uint32_t trip = 0; trip < (size << shift); ++trip) {
       const bool active = g + 32ull * trip < total;
       uint32_t t = kInvalidIndex;
+      bool failed = false;
       if (active) {
         const uint64_t code = (__ldg(a.codes + (child >> 1)) << 1) | (child & 1u);
         const int depth = uni ? a.depth : int(__ldg(a.inst_depth + inst));
         uint32_t sb[D], tb[D];
         split_code<D>(code, depth, sb);
         bool inside;
-        if (!screened_point<Map>(a.screen + inst, a.sk, a.sA, a.map, pts, P, k, sb, tb, inside)) {
+        const ScreenRec* rec = a.screen + inst;
+        const bool tried = trial.on() && __ldg(&rec->on) != 0u;
+        const bool sure = tried && screened_point<Map>(rec, a.sk, a.sA, a.map, pts, P, k, sb, tb, inside);
+        failed = tried && !sure;
+        if (!sure) {
+          undecided += tried ? 1u : 0u;
           const uint64_t cc[1] = {child};
           const uint32_t ck[1] = {k}, ci[1] = {inst};
           const bool ca[1] = {true};
@@ -381,6 +387,7 @@ __global__ void __launch_bounds__(256, 4) batch_screen_kernel(const BatchArgs a)
           if (p != kInvalidIndex) t = 2u * p + uint32_t(tcode & 1u);
         }
       }
+      if constexpr (ScreenTrial::by_unit(D)) trial.note(failed, 1);
       if (t < kOutsideIndex) a.hit[t] = 1;
       if (a.targets && active) {
         const uint64_t base = __ldg(a.tgt_base + inst);
@@ -390,6 +397,7 @@ __global__ void __launch_bounds__(256, 4) batch_screen_kernel(const BatchArgs a)
       while (k >= P) { k -= P; ++child; }
       while (inst + 1 < a.n_inst && (child >> 1) >= off_s[inst + 1]) ++inst;
     }
+    if constexpr (!ScreenTrial::by_unit(D)) trial.note(undecided, size << shift);
   }
 }
 
@@ -487,6 +495,7 @@ __global__ void __launch_bounds__(256, kScreen ? 4 : 1) batch_rows_kernel(const 
   const uint32_t P = uint32_t(a.points);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   uint32_t* s = keys[w];
+  ScreenTrial trial;
   for (uint32_t row = blockIdx.x * 8 + w; row < nrows; row += gridDim.x * 8) {
     const uint32_t inst = find_instance(off_s, a.n_inst, row);   // arena index
     const uint32_t sp = a.inst_of[inst];                          // sorted position
@@ -510,8 +519,10 @@ __global__ void __launch_bounds__(256, kScreen ? 4 : 1) batch_rows_kernel(const 
       return point_code<D>(a.dom, y, depth, tcode);
     };
     uint32_t sb[D];
+    const ScreenRec* rec = kScreen ? a.screen + (size_t(depth - 1) * a.screen_stride + sp) : nullptr;
     if constexpr (kScreen) split_code<D>(code, depth, sb);
     else own();
+    uint32_t undecided = 0;
 #pragma unroll 1
     for (int q = 0; q < 4; ++q) {
       const uint32_t k = uint32_t(lane) + 32u * q;
@@ -522,10 +533,12 @@ __global__ void __launch_bounds__(256, kScreen ? 4 : 1) batch_rows_kernel(const 
         bool inside;
         if constexpr (kScreen) {
           uint32_t tb[D];
-          if (screened_point<Map>(a.screen + (size_t(depth - 1) * a.screen_stride + sp), a.sk, a.sA, a.map, pts, P, k,
-                                  sb, tb, inside)) {
+          const bool tried = trial.on() && __ldg(&rec->on) != 0u;
+          const bool sure = tried && screened_point<Map>(rec, a.sk, a.sA, a.map, pts, P, k, sb, tb, inside);
+          if (sure) {
             if (inside) tcode = join_code<D>(tb, depth);
           } else {
+            undecided += tried ? 1u : 0u;
             own();
             inside = own_code(k, tcode);
           }
@@ -542,6 +555,7 @@ __global__ void __launch_bounds__(256, kScreen ? 4 : 1) batch_rows_kernel(const 
       }
       s[lane + 32 * q] = key;
     }
+    if constexpr (kScreen) trial.note(undecided, (P + 31u) / 32u);
     const uint32_t total = row_emit(s, bounds[w], lane, P, a.keep_lost, n_i + 1, a.stage_col + size_t(row) * P,
                                     a.stage_cnt + size_t(row) * P);
     if (lane == 0) a.row_count[row] = total;

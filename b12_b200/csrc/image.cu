@@ -226,20 +226,28 @@ __global__ void __launch_bounds__(kThreads, !kScreen ? 6 : M == ImageMode::Mark 
   // the end (an atomic for every warp with a new box held the continuation's image launches
   // at 10.8 ms; without them 9.6)
   uint32_t new_boxes = 0;
+  // (Mark mode always tries: its kernel is short of registers, the continuation takes 11.05 ms
+  // with the trial and 10.60 without)
+  constexpr bool kTrial = kScreen && M != ImageMode::Mark;
+  ScreenTrial trial;
+  uint32_t undecided = 0;
   // One point of the launch: g = rank * P + k (the source's rank among the sources, the
   // point's index in its box).  Every lane of the warp calls it the same number of times
   // (inactive lanes with active = false), so that the warp collectives stay converged.
   auto point = [&](uint64_t g, uint32_t rank, uint32_t k, bool active) {
     uint32_t t = kInvalidIndex;
     uint32_t tbits[Map::D];
-    bool valid = false;
+    bool valid = false, sure = true;
     if (active) {
       if constexpr (M == ImageMode::Insert || M == ImageMode::Mark) {   // these carry their source centres
         double c[Map::D];
         PI::source_centre(a, rank, c);
         if constexpr (kScreen) {
-          if (!PI::screened_at(a, pts, table, c, g, k, tbits, valid))
+          sure = (!kTrial || trial.on()) && PI::screened_at(a, pts, table, c, g, k, tbits, valid);
+          if (!sure) {
             valid = PI::template image_at<true>(a, pts, table, c, g, k, tbits);
+            ++undecided;
+          }
         } else {
           valid = PI::image_at(a, pts, table, c, g, k, tbits);
         }
@@ -248,7 +256,9 @@ __global__ void __launch_bounds__(kThreads, !kScreen ? 6 : M == ImageMode::Mark 
         uint32_t sbits[Map::D];
         PI::source_bits(a, leaf, sbits);
         if constexpr (kScreen) {
-          if (!PI::screened(a, pts, table, sbits, g, k, tbits, valid)) {
+          sure = (!kTrial || trial.on()) && PI::screened(a, pts, table, sbits, g, k, tbits, valid);
+          if (!sure) {
+            ++undecided;
             PI::source_bits(a, leaf, sbits);       // (read again: not kept over the evaluation)
             valid = PI::template image<true>(a, pts, table, sbits, g, k, tbits);
           }
@@ -258,6 +268,7 @@ __global__ void __launch_bounds__(kThreads, !kScreen ? 6 : M == ImageMode::Mark 
       }
       if constexpr (M != ImageMode::Mark) t = PI::target(a, n, valid, tbits);
     }
+    if constexpr (kTrial && ScreenTrial::by_unit(Map::D)) trial.note(!sure, 1);
     if constexpr (M == ImageMode::Hit) {
       // (a store of all lanes: the warp's few distinct bytes leave the SM as so many sectors
       // either way, and finding one lane for each cost more than it saved)
@@ -341,6 +352,10 @@ __global__ void __launch_bounds__(kThreads, !kScreen ? 6 : M == ImageMode::Mark 
       k += 32;
       while (k >= P32) { k -= P32; ++rank; }
     }
+    if constexpr (kTrial && !ScreenTrial::by_unit(Map::D)) {
+      trial.note(undecided, size << shift);
+      undecided = 0;
+    }
   }
   if constexpr (M == ImageMode::Mark) {
     if (lane == 0 && new_boxes) atomicAdd(a.cand_count, new_boxes);
@@ -355,8 +370,9 @@ __global__ void __launch_bounds__(kThreads, !kScreen ? 6 : M == ImageMode::Mark 
 // ---------------------------------------------------------------------------------
 constexpr int kRowWarps = kThreads / 32;
 
+// (registers: three blocks an SM for Lorenz, four for the others)
 template<class Map, class Grid, bool kScreen>
-__global__ void __launch_bounds__(kThreads) transition_rows_kernel(const RowArgs ra)
+__global__ void __launch_bounds__(kThreads, !kScreen ? 1 : Map::D == 3 ? 3 : 4) transition_rows_kernel(const RowArgs ra)
 {
   using PI = PointImage<Map, Grid>;
   const ImageArgs& a = ra.img;
@@ -371,30 +387,35 @@ __global__ void __launch_bounds__(kThreads) transition_rows_kernel(const RowArgs
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   uint32_t* s = keys[w];
   const uint32_t warps = gridDim.x * kRowWarps;
+  ScreenTrial trial;
 
   for (uint32_t row = blockIdx.x * kRowWarps + w; row < nrows; row += warps) {
     const uint32_t leaf = a.src ? __ldg(a.src + row) : row;
     uint32_t sbits[Map::D];
     PI::source_bits(a, leaf, sbits);
+    uint32_t undecided = 0;
 #pragma unroll 1
     for (int q = 0; q < 4; ++q) {
       const uint32_t k = uint32_t(lane) + 32u * q;
       uint32_t key = kPadKey;
+      bool sure = true;
       if (k < P) {
         uint32_t tbits[Map::D];
         const uint64_t i = uint64_t(row) * P + k;
         bool valid;
         if constexpr (kScreen) {
-          if (!PI::screened(a, pts, table, sbits, i, k, tbits, valid))
-            valid = PI::template image<true>(a, pts, table, sbits, i, k, tbits);
+          sure = trial.on() && PI::screened(a, pts, table, sbits, i, k, tbits, valid);
+          if (!sure) valid = PI::template image<true>(a, pts, table, sbits, i, k, tbits);
         } else {
           valid = PI::image(a, pts, table, sbits, i, k, tbits);
         }
         const uint32_t t = PI::target(a, n, valid, tbits);
         key = t == kInvalidIndex ? kLostKey : t;
       }
+      if (kScreen && !sure) ++undecided;
       s[lane + 32 * q] = key;
     }
+    if constexpr (kScreen) trial.note(undecided, (P + 31u) / 32u);
     const uint32_t total = row_emit(s, bounds[w], lane, P, ra.keep_lost, ra.lost_col,
                                     ra.stage_col + size_t(row) * P, ra.stage_cnt + size_t(row) * P);
     if (lane == 0) ra.row_count[row] = total;

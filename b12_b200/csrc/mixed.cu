@@ -797,15 +797,16 @@ __device__ __forceinline__ bool screened_code(const MixedArgs& a, const double* 
 }
 
 // the leaf the image of point k of source leaf `leaf` lands in (point index g)
+// (kScreen: `sure`, whether to try the screened evaluation, becomes whether it decided)
 template<class Map, class Grid, bool kScreen = false>
 __device__ __forceinline__ uint32_t image_of(const MixedArgs& a, const double* pts, bool table, uint32_t leaf,
-                                             uint32_t k, uint64_t g)
+                                             uint32_t k, uint64_t g, bool& sure)
 {
   uint64_t p64;
   bool valid;
   if constexpr (kScreen) {
-    if (!screened_code<Map, Grid>(a, pts, table, leaf, k, g, p64, valid))
-      valid = image_code<Map, Grid, true>(a, pts, table, leaf, k, g, p64);
+    sure = sure && screened_code<Map, Grid>(a, pts, table, leaf, k, g, p64, valid);
+    if (!sure) valid = image_code<Map, Grid, true>(a, pts, table, leaf, k, g, p64);
   } else {
     valid = image_code<Map, Grid>(a, pts, table, leaf, k, g, p64);
   }
@@ -879,7 +880,8 @@ __global__ void __launch_bounds__(kThreads) mixed_image_kernel(const MixedArgs a
         if constexpr (kMode == 4) a.out[g] = b;
         else if (b != kInvalidIndex) a.box_hit[b] = 1;
       } else {
-        const uint32_t t = image_of<Map, Grid>(a, pts, table, leaf, k, g);
+        bool sure = false;
+        const uint32_t t = image_of<Map, Grid>(a, pts, table, leaf, k, g, sure);
         if constexpr (kMode == 1) a.out[g] = t;
         else if (t != kInvalidIndex) a.hit[t] = 1;
       }
@@ -908,6 +910,7 @@ __global__ void __launch_bounds__(kThreads, kScreenBlocks) mixed_screen_kernel(c
   const uint32_t fine = gridDim.x * (kThreads / 32) * kFine;
   const uint32_t coarse_end = units > fine ? units - fine : 0;
   uint32_t c = 0;
+  ScreenTrial trial;
   for (;;) {
     const uint32_t size = c < coarse_end ? kTrips : 1u;
     if (lane == 0) c = atomicAdd(a.work, size);
@@ -922,18 +925,24 @@ __global__ void __launch_bounds__(kThreads, kScreenBlocks) mixed_screen_kernel(c
       rank = uint32_t(g / P);
       k = uint32_t(g - uint64_t(rank) * P);
     }
+    uint32_t undecided = 0;
 #pragma unroll 1
     for (uint32_t j = 0; j < (size << shift); ++j) {
       const uint64_t gj = g + 32ull * j;
+      bool sure = true;
       if (gj < total) {
+        sure = trial.on();
         const uint32_t leaf = a.src ? __ldg(a.src + rank) : rank;
-        const uint32_t t = image_of<Map, Grid, true>(a, pts, table, leaf, k, gj);
+        const uint32_t t = image_of<Map, Grid, true>(a, pts, table, leaf, k, gj, sure);
         if constexpr (kMode == 1) a.out[gj] = t;
         else if (t != kInvalidIndex) a.hit[t] = 1;
       }
+      if constexpr (ScreenTrial::by_unit(Map::D)) trial.note(!sure, 1);
+      else if (!sure) ++undecided;
       k += 32;
       while (k >= P32) { k -= P32; ++rank; }
     }
+    if constexpr (!ScreenTrial::by_unit(Map::D)) trial.note(undecided, size << shift);
   }
 }
 
@@ -949,17 +958,23 @@ __global__ void __launch_bounds__(kThreads) mixed_rows_kernel(const MixedArgs a)
   const uint32_t P = uint32_t(a.points);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   uint32_t* s = keys[w];
+  ScreenTrial trial;
   for (uint32_t row = blockIdx.x * kWarps + w; row < a.n; row += gridDim.x * kWarps) {
+    uint32_t undecided = 0;
 #pragma unroll 1
     for (int q = 0; q < 4; ++q) {
       const uint32_t k = uint32_t(lane) + 32u * q;
       uint32_t key = kPadKey;
+      bool sure = true;
       if (k < P) {
-        const uint32_t t = image_of<Map, Grid, kScreen>(a, pts, table, row, k, uint64_t(row) * P + k);
+        sure = trial.on();
+        const uint32_t t = image_of<Map, Grid, kScreen>(a, pts, table, row, k, uint64_t(row) * P + k, sure);
         key = t == kInvalidIndex ? kLostKey : t;
       }
+      if (kScreen && !sure) ++undecided;
       s[lane + 32 * q] = key;
     }
+    if constexpr (kScreen) trial.note(undecided, (P + 31u) / 32u);
     const uint32_t total = row_emit(s, bounds[w], lane, P, a.keep_lost, a.lost_col, a.stage_col + size_t(row) * P,
                                     a.stage_cnt + size_t(row) * P);
     if (lane == 0) a.row_count[row] = total;

@@ -286,6 +286,37 @@ template<> struct Screen<ForcedDuffingMap> {
   }
 };
 
+// Whether a warp tries the screened evaluation on its next piece of work.  A warp with an
+// undecided point runs both evaluations, so where many points stay undecided (trajectories
+// that leave the limits, in domains or maps whose bound leaves no room for wider ones) trying
+// costs more than it saves.  After two pieces in a row in which some lane had half of its
+// points undecided the warp takes the map's own arithmetic for the next 3 pieces, and after
+// another one, or more, for 31.  Two, since 4 % of the points are undecided in the usual
+// forced Duffing jobs, where trying still pays.  Counted by pieces, not by points, since the
+// points' loop is bound by its instructions (a vote for every 32 points cost a Lorenz job of
+// depth 27 1.2 %), but in the two-dimensional image launches, whose points are longer and
+// launches smaller, by units of 32 points (a forced Duffing job of depth 19: 1,142 us, by
+// pieces 1,222, always trying 1,174).
+// Images of 250,000 Lorenz boxes (125 points, h = 0.02, radius 10 around 0; 3 % of the points
+// decided): 2.92 ms (strict) and 1.86 (FMA), always trying 4.21 and 3.17, never 2.82 and 1.75.
+// `undecided`: the lane's undecided points of the piece's `tries`.  Every lane calls note()
+// after every piece.
+struct ScreenTrial {
+  uint32_t skip = 0, failed = 0;
+  static __host__ __device__ constexpr bool by_unit(int dim) { return dim == 2; }
+  __device__ __forceinline__ bool on() const { return skip == 0; }
+  __device__ __forceinline__ void note(uint32_t undecided, uint32_t tries)
+  {
+    if (skip) {
+      --skip;
+      return;
+    }
+    const bool bad = __any_sync(0xFFFFFFFFu, undecided != 0 && 2u * undecided >= tries);
+    failed = bad ? min(failed + 1u, 3u) : 0u;
+    skip = failed < 2u ? 0u : failed == 2u ? 3u : 31u;
+  }
+};
+
 // the double 1 + index 2^-k (exact for k <= 20)
 __device__ __forceinline__ double screen_index(uint32_t index, uint32_t k)
 {
