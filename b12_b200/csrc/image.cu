@@ -226,9 +226,9 @@ __global__ void __launch_bounds__(kThreads, !kScreen ? 6 : M == ImageMode::Mark 
   // the end (an atomic for every warp with a new box held the continuation's image launches
   // at 10.8 ms; without them 9.6)
   uint32_t new_boxes = 0;
-  // (Mark mode always tries: its kernel is short of registers, the continuation takes 11.05 ms
-  // with the trial and 10.60 without)
-  constexpr bool kTrial = kScreen && M != ImageMode::Mark;
+  // (the coupled Duffing continuation always tries: its points are short and few of them stay
+  // undecided; 10.68 ms, with the trial 10.85)
+  constexpr bool kTrial = kScreen && !(M == ImageMode::Mark && Map::D == 4);
   ScreenTrial trial;
   uint32_t undecided = 0;
   // One point of the launch: g = rank * P + k (the source's rank among the sources, the

@@ -76,6 +76,29 @@ def test_leaves_of_two_depths(name):
     t.close()
 
 
+@pytest.mark.parametrize("name", sorted(SPECS))
+def test_continuations_and_insertions(name):
+    """From the boxes of 20,000 random points (a continuation's launches, and an insertion's)."""
+    import b12_b200 as B
+    spec, depth = SPECS[name], 18
+    rng = np.random.default_rng(7)
+    x0 = np.array(spec["center"]) + np.array(spec["radius"]) * rng.uniform(-1, 1, size=(20000, spec["dim"]))
+    t = B.ImplicitBoxTree(spec["center"], spec["radius"])
+    counts = t.continuation_run(scheme(spec), x0, depth, max_sweeps=3)
+    o, want = O.continuation(spec, depth, x0, max_sweeps=3)
+    assert list(counts) == list(want)
+    for x, y in zip(t.leaves(), o.leaves()):
+        assert np.array_equal(x, y)
+    for tree in (t, o):
+        tree.set_flags(4)
+    sc = scheme(spec)
+    sc = B.Scheme(sc.map, sc.grid, depth=depth, flags_to_check=4)
+    assert t.insert_by_image(sc, depth, B.INS, B.NONE) == o.insert_by_image(4, 2, 0)
+    for x, y in zip(t.leaves(), o.leaves()):
+        assert np.array_equal(x, y)
+    t.close()
+
+
 @pytest.mark.parametrize("fma", [False, True])
 def test_batches_and_served_jobs(fma):
     import b12_b200 as B
