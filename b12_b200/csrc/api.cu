@@ -921,10 +921,11 @@ b12g_status ensure_transpose(b12g_csr* m)
     CK(cudaStreamSynchronize(s));
     const uint32_t max_row = got[0];
     m->plan = CountPlan{};
+    const bool on_chip = measure_on_chip(m->nnz, max_row, uint32_t(measure_partial_slots()));
     if (pack)
       m->plan = CountPlan{m->pack.p, m->dlist.p, m->dcount.p, double(m->count_points), got[3], got[2],
-                          count_chunk(m->nnz, max_row, got[1], got[2], got[3])};
-    if (m->plan.chunk || measure_on_chip(m->nnz, max_row, uint32_t(measure_partial_slots()))) {
+                          count_chunk(m->nnz, max_row, got[1], got[2], got[3], !on_chip), !on_chip};
+    if (m->plan.chunk || on_chip) {
       // the power iteration keeps the matrix on chip and reads no row-class lists
       m->n_mid = 0;
       m->n_long = 0;

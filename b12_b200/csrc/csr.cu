@@ -11,6 +11,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "kernels.h"
 #include "csr.h"
@@ -209,7 +210,9 @@ __device__ __forceinline__ double iterate_value(const double* wp, const double* 
 // The result v = the last iterate scaled by 1/|.|_1 (the first iterate when iters == 0)
 // and, when asked for, each block's part of |v - previous normalised iterate|_1 (the
 // change made by the last iteration: the stopping test of a tolerance-driven run).
-__device__ void write_result(const MeasureArgs& a, double inv, double inv_prev)
+// (kPair: 1 / |.|_1 is inv + inv_lo, and the product is rounded once)
+template<bool kPair = false>
+__device__ void write_result(const MeasureArgs& a, double inv, double inv_prev, double inv_lo = 0.0)
 {
   __shared__ double red_c[32];
   const uint32_t n = a.n;
@@ -220,7 +223,11 @@ __device__ void write_result(const MeasureArgs& a, double inv, double inv_prev)
   double c = 0.0;
   for (uint32_t j = tid; j < n; j += nthreads) {
     const double first = a.start ? __ldg(a.start + j) : v0;
-    const double x = a.iters ? __dmul_rn(__ldcg(wl + j), inv) : first;
+    double x = first;
+    if (a.iters) {
+      const double w = __ldcg(wl + j);
+      x = kPair ? __fma_rn(w, inv, __dmul_rn(w, inv_lo)) : __dmul_rn(w, inv);
+    }
     a.out[j] = x;
     if (a.change && a.iters) {
       const double prev = a.iters >= 2 ? __dmul_rn(__ldcg(wq + j), inv_prev) : first;
@@ -715,22 +722,71 @@ __global__ void __launch_bounds__(kMeasureThreads, 1) count_plan_kernel(const ui
   if (lane == 0 && most) atomicMax(flags + 2, most);
 }
 
+// hi + lo += c v: hi is the rounded sum and lo takes the rounding error (TwoSum, Knuth, with
+// the product unrounded in an FMA; the error term itself is rounded, some 2^-53 of it)
+__device__ __forceinline__ void two_fma(double c, double v, double& hi, double& lo)
+{
+  const double s = __fma_rn(c, v, hi), z = __dsub_rn(s, hi);
+  lo = __dadd_rn(lo, __dadd_rn(__dsub_rn(hi, __dsub_rn(s, z)), __fma_rn(c, v, -z)));
+  hi = s;
+}
+
+// hi + lo += x + x_lo
+__device__ __forceinline__ void two_add(double x, double x_lo, double& hi, double& lo)
+{
+  two_fma(1.0, x, hi, lo);
+  lo = __dadd_rn(lo, x_lo);
+}
+
+// barrier_total of partial sums in pairs
+__device__ void barrier_total_pair(const double* part, const double* part_lo, double& hi, double& lo)
+{
+  __shared__ double bcast[2];
+  if (threadIdx.x < 32) {
+    double x = 0.0, x_lo = 0.0;
+    for (uint32_t i = threadIdx.x; i < gridDim.x; i += 32) two_add(__ldcg(part + i), __ldcg(part_lo + i), x, x_lo);
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+      const double y = __shfl_xor_sync(0xFFFFFFFFu, x, d), y_lo = __shfl_xor_sync(0xFFFFFFFFu, x_lo, d);
+      two_add(y, y_lo, x, x_lo);
+    }
+    if (threadIdx.x == 0) {
+      bcast[0] = x;
+      bcast[1] = x_lo;
+    }
+  }
+  __syncthreads();
+  hi = bcast[0];
+  lo = bcast[1];
+  __syncthreads();           // bcast is read by every thread before it can be written again
+}
+
 // The same iteration from the packed entries.  Thread t's run is entries [t run, (t + 1) run)
 // of the block, run = entries / threads rounded up, four to a 16-byte word, word g of all
 // threads side by side (conflict-free reads); the places past a run's entries are zero: a
 // count of 0, value 0, of the first source.
 // Everything else - the rows split over runs, the normalising iterations, the waits - is
-// invariant_measure_smem_kernel's.  Bound by the latency of an iteration's chain: the wait
+// invariant_measure_smem_kernel's.
+// kPair: the last two iterations sum a row as an unevaluated pair (two_fma), rounded once at
+// its end, and the norm and its reciprocal are pairs too (a rounding in those shifts every
+// entry alike).  Errors of the iterations before are averaged away by those that follow.
+// It is for the matrices that the kernel above cannot hold, which invariant_measure_kernel
+// takes otherwise: one sum from a row's start to its end rounds more than that kernel's eight.
+// Error in the 2-norm against the iteration in 80 bits, relative, for 300,000 boxes, 4.0 M
+// entries and 40 iterations: 0.65e-16; without pairs 1.9e-16, by that kernel 2.2e-16.
+// Bound by the latency of an iteration's chain: the wait
 // for the blocks it depends on, one gather, the walk over shared memory (a random 8-byte
 // read an entry), the release.  200 iterations of the depth-27 matrix (1.6 M entries): 1.25
 // ms against 1.76; 50 of a matrix of 600,000 boxes and 7.1 M entries, which the kernel above
-// cannot hold: 0.70 ms against 3.44 from HBM and L2.
+// cannot hold: 0.72 ms against 3.44 from HBM and L2.
+template<bool kPair>
 __global__ void __launch_bounds__(kMeasureThreads, 1) invariant_measure_count_kernel(MeasureArgs a, uint32_t nnz,
                                                                                      const uint32_t* pack,
                                                                                      const uint32_t* dlist,
                                                                                      const uint32_t* dcount,
                                                                                      uint32_t cap, uint32_t chunk,
-                                                                                     double points, uint32_t counts)
+                                                                                     double points, uint32_t counts,
+                                                                                     double* partial_lo)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   uint4* s_ent = reinterpret_cast<uint4*>(smem);
@@ -739,8 +795,9 @@ __global__ void __launch_bounds__(kMeasureThreads, 1) invariant_measure_count_ke
   double* s_v = s_val + counts;
   // after an iteration's walk the staged values' place holds the runs' first parts
   double* s_head = s_v;
-  uint32_t* s_head_end = reinterpret_cast<uint32_t*>(s_v + kMeasureThreads);
-  __shared__ double red[kMeasureThreads / 32];
+  double* s_head_lo = s_v + kMeasureThreads;      // kPair only
+  uint32_t* s_head_end = reinterpret_cast<uint32_t*>(s_v + (kPair ? 2 : 1) * kMeasureThreads);
+  __shared__ double red[kMeasureThreads / 32], red_lo[kPair ? kMeasureThreads / 32 : 1];
   __shared__ uint32_t s_bnd[32 * kDepWords + 1];
   __shared__ uint32_t s_dep[kDepWords];
   const uint32_t n = a.n;
@@ -813,12 +870,16 @@ __global__ void __launch_bounds__(kMeasureThreads, 1) invariant_measure_count_ke
   for (uint32_t it = 0; it < a.iters; ++it) {
     const double* wp = (it & 1u) ? a.w0 : a.w1;
     double* wc = (it & 1u) ? a.w1 : a.w0;
-    double local = 0.0;
+    double local = 0.0, local_lo = 0.0;
+    const bool precise = kPair && it + 2 >= a.iters;
     if (!after_barrier && !epoch_wait(a, waits, it)) return;
     // stage the distinct sources (the last iterate, scaled when its norm was summed)
     const bool scale = it > 0 && measure_normalises(it - 1, a.iters);
     if (scale) {
-      const double s_prev = barrier_total(a.partial + ((norms - 1u) & 1u) * gridDim.x);
+      const uint32_t slot = ((norms - 1u) & 1u) * gridDim.x;
+      double s_prev, s_lo = 0.0;
+      if constexpr (kPair) barrier_total_pair(a.partial + slot, partial_lo + slot, s_prev, s_lo);
+      else s_prev = barrier_total(a.partial + slot);
       inv_prev = inv;
       inv = __ddiv_rn(1.0, s_prev);
     }
@@ -842,9 +903,10 @@ __global__ void __launch_bounds__(kMeasureThreads, 1) invariant_measure_count_ke
     __syncthreads();
     // walk the run: a row that ends inside it is written here unless it began earlier
     uint32_t row = row0;
-    double acc = 0.0, head = 0.0;
+    double acc = 0.0, acc_lo = 0.0, head = 0.0, head_lo = 0.0;
     bool first = true;
-    if (any) {
+    auto walk = [&](auto pair) {
+      constexpr bool kP = decltype(pair)::value;
       for (uint32_t g = 0; g < (run + 3) / 4; ++g) {
         const uint4 e4 = s_ent[g * kMeasureThreads + t];
         const uint32_t e[4] = {e4.x, e4.y, e4.z, e4.w};
@@ -856,43 +918,82 @@ __global__ void __launch_bounds__(kMeasureThreads, 1) invariant_measure_count_ke
         }
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          acc = __fma_rn(c[q], v[q], acc);
+          if constexpr (kP) two_fma(c[q], v[q], acc, acc_lo);
+          else acc = __fma_rn(c[q], v[q], acc);
           if (e[q] & kCountEnd) {
-            if (first && head_open) head = acc;
-            else { __stcg(wc + row, acc); local = __dadd_rn(local, fabs(acc)); }
+            if (first && head_open) {
+              head = acc;
+              if constexpr (kP) head_lo = acc_lo;
+            } else if constexpr (kP) {
+              const double x = __dadd_rn(acc, acc_lo);
+              __stcg(wc + row, x);
+              two_add(fabs(x), 0.0, local, local_lo);
+            } else {
+              __stcg(wc + row, acc);
+              local = __dadd_rn(local, fabs(acc));
+            }
             first = false;
             row += 1u + (e[q] >> 25);
             acc = 0.0;
+            if constexpr (kP) acc_lo = 0.0;
           }
         }
+      }
+    };
+    if (any) {
+      if constexpr (kPair) {
+        if (precise) walk(std::true_type{});
+        else walk(std::false_type{});
+      } else {
+        walk(std::false_type{});
       }
     }
     __syncthreads();
     if (any && head_open) {
       // (a run inside one row has its whole sum in acc and leaves the row open)
       s_head[t] = first ? acc : head;
+      if constexpr (kPair) s_head_lo[t] = first ? acc_lo : head_lo;
       s_head_end[t] = first && tail_open ? 0u : 1u;
     }
     __syncthreads();
     if (any && tail_open && !(first && head_open)) {
       // this run holds the row's first entry: add the later runs' parts in order
-      double sum = acc;
+      double sum = acc, sum_lo = acc_lo;
       for (uint32_t j = t + 1; j < blockDim.x; ++j) {
-        sum = __dadd_rn(sum, s_head[j]);
+        if (precise) two_add(s_head[j], s_head_lo[j], sum, sum_lo);
+        else sum = __dadd_rn(sum, s_head[j]);
         if (s_head_end[j]) break;
       }
+      if (precise) sum = __dadd_rn(sum, sum_lo);
       __stcg(wc + row, sum);
-      local = __dadd_rn(local, fabs(sum));
+      if (precise) two_add(fabs(sum), 0.0, local, local_lo);
+      else local = __dadd_rn(local, fabs(sum));
     }
     if (measure_normalises(it, a.iters)) {
 #pragma unroll
-      for (int d = 16; d > 0; d >>= 1) local = __dadd_rn(local, __shfl_xor_sync(0xFFFFFFFFu, local, d));
-      if (lane == 0) red[t >> 5] = local;
+      for (int d = 16; d > 0; d >>= 1) {
+        const double y = __shfl_xor_sync(0xFFFFFFFFu, local, d);
+        if constexpr (kPair) {
+          const double y_lo = __shfl_xor_sync(0xFFFFFFFFu, local_lo, d);
+          two_add(y, y_lo, local, local_lo);
+        } else {
+          local = __dadd_rn(local, y);
+        }
+      }
+      if (lane == 0) {
+        red[t >> 5] = local;
+        if constexpr (kPair) red_lo[t >> 5] = local_lo;
+      }
       __syncthreads();
       if (t == 0) {
-        double sum = 0.0;
-        for (int i = 0; i < kMeasureThreads / 32; ++i) sum = __dadd_rn(sum, red[i]);
-        __stcg(a.partial + (norms & 1u) * gridDim.x + blockIdx.x, sum);
+        double sum = 0.0, sum_lo = 0.0;
+        for (int i = 0; i < kMeasureThreads / 32; ++i) {
+          if constexpr (kPair) two_add(red[i], red_lo[i], sum, sum_lo);
+          else sum = __dadd_rn(sum, red[i]);
+        }
+        const uint32_t at = (norms & 1u) * gridDim.x + blockIdx.x;
+        __stcg(a.partial + at, sum);
+        if constexpr (kPair) __stcg(partial_lo + at, sum_lo);
       }
       if (!barrier_wait(a, bars++)) return;
       ++norms;
@@ -902,12 +1003,18 @@ __global__ void __launch_bounds__(kMeasureThreads, 1) invariant_measure_count_ke
       after_barrier = false;
     }
   }
+  double inv_lo = 0.0;
   if (a.iters) {
-    const double s_last = barrier_total(a.partial + ((norms - 1u) & 1u) * gridDim.x);
+    const uint32_t slot = ((norms - 1u) & 1u) * gridDim.x;
+    double s_last, s_lo = 0.0;
+    if constexpr (kPair) barrier_total_pair(a.partial + slot, partial_lo + slot, s_last, s_lo);
+    else s_last = barrier_total(a.partial + slot);
     inv_prev = inv;
     inv = __ddiv_rn(1.0, s_last);
+    // 1 / (s_last + s_lo) = inv + inv_lo to first order
+    inv_lo = __dmul_rn(__dsub_rn(__fma_rn(-s_last, inv, 1.0), __dmul_rn(s_lo, inv)), inv);
   }
-  write_result(a, inv, inv_prev);
+  write_result<kPair>(a, inv, inv_prev, inv_lo);
 }
 
 // the rows of P^T of one length class (1: medium, 2: long), ascending (flag, scan, scatter)
@@ -1000,11 +1107,15 @@ MeasureLaunch measure_launch()
                                                               kSmemMeasureBytes) == cudaSuccess && b >= 1;
     cudaGetLastError();
     b = 0;
-    c.count_ok = cudaFuncSetAttribute(invariant_measure_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    c.count_ok = cudaFuncSetAttribute(invariant_measure_count_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      int(kCountSmemLimit)) == cudaSuccess &&
+                 cudaFuncSetAttribute(invariant_measure_count_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       int(kCountSmemLimit)) == cudaSuccess &&
                  cudaFuncSetAttribute(count_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       int(kCountSmemLimit)) == cudaSuccess &&
-                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, invariant_measure_count_kernel, kMeasureThreads,
+                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, invariant_measure_count_kernel<false>, kMeasureThreads,
+                                                               kCountSmemLimit) == cudaSuccess && b >= 1 &&
+                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, invariant_measure_count_kernel<true>, kMeasureThreads,
                                                                kCountSmemLimit) == cudaSuccess && b >= 1;
     cudaGetLastError();
     b = 0;
@@ -1041,8 +1152,9 @@ bool count_plan_possible(uint64_t nnz, uint32_t n, uint32_t partial_cap)
 {
   const uint32_t blocks = uint32_t(device_sm_count());
   const uint64_t slots = 2ull * blocks + 2 + (uint64_t(blocks) * kEpochStride + uint64_t(kDepWords) * blocks + 1) / 2;
+  // (and the second halves of 2 x blocks partial sums in pairs)
   return measure_launch().count_ok && nnz > 0 && n <= kCountMaxRows && blocks <= 32u * kDepWords &&
-         slots <= partial_cap &&
+         slots + 2ull * blocks <= partial_cap &&
          (nnz + blocks - 1) / blocks + kMidRow <= uint64_t(kCountMaxChunk) * kMeasureThreads;
 }
 
@@ -1059,22 +1171,22 @@ cudaError_t count_plan(const uint32_t* tptr, const uint32_t* trows, const double
 
 namespace {
 
-size_t count_bytes(uint32_t chunk, uint32_t distinct, uint32_t counts)
+size_t count_bytes(uint32_t chunk, uint32_t distinct, uint32_t counts, bool pair)
 {
   return size_t(chunk) * kMeasureThreads * 4 + size_t(counts) * 8 +
-         std::max<size_t>(size_t(distinct) * 8, size_t(kMeasureThreads) * 12);
+         std::max<size_t>(size_t(distinct) * 8, size_t(kMeasureThreads) * (pair ? 20 : 12));
 }
 
 }  // namespace
 
-uint32_t count_chunk(uint64_t nnz, uint32_t max_row, uint32_t flags, uint32_t distinct, uint32_t largest)
+uint32_t count_chunk(uint64_t nnz, uint32_t max_row, uint32_t flags, uint32_t distinct, uint32_t largest, bool pair)
 {
   const uint32_t blocks = uint32_t(device_sm_count());
   if (flags != 0 || max_row > kMidRow) return 0;
   // a block's rows begin in its share of the entries and have at most kMidRow entries
   const uint64_t most = (nnz + blocks - 1) / blocks + kMidRow;
   const uint32_t chunk = uint32_t((most + 4 * kMeasureThreads - 1) / (4 * kMeasureThreads)) * 4;
-  return chunk <= kCountMaxChunk && count_bytes(chunk, distinct, largest + 1) <= kCountSmemLimit ? chunk : 0;
+  return chunk <= kCountMaxChunk && count_bytes(chunk, distinct, largest + 1, pair) <= kCountSmemLimit ? chunk : 0;
 }
 
 cudaError_t max_row_length(const uint32_t* tptr, uint32_t n, uint32_t* out, cudaStream_t s)
@@ -1105,9 +1217,12 @@ cudaError_t invariant_measure(const uint32_t* tptr, const uint32_t* trows, const
     const uint32_t *pack = plan->pack, *dlist = plan->dlist, *dcount = plan->dcount;
     double points = plan->points;
     uint32_t counts = plan->largest + 1;
-    void* params[] = {&a, &nnz32, &pack, &dlist, &dcount, &cap, &chunk, &points, &counts};
-    return cudaLaunchCooperativeKernel((const void*)invariant_measure_count_kernel, dim3(blocks), dim3(kMeasureThreads),
-                                       params, count_bytes(chunk, plan->distinct, counts), s);
+    double* partial_lo = partial + 2 * size_t(blocks) + 2 + (size_t(epoch_words) + kDepWords * blocks + 1) / 2;
+    void* params[] = {&a, &nnz32, &pack, &dlist, &dcount, &cap, &chunk, &points, &counts, &partial_lo};
+    const void* kernel = plan->pair ? (const void*)invariant_measure_count_kernel<true>
+                                    : (const void*)invariant_measure_count_kernel<false>;
+    return cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(kMeasureThreads), params,
+                                       count_bytes(chunk, plan->distinct, counts, plan->pair), s);
   }
   if (mid_list && long_list && n_long == 0 && measure_on_chip(nnz, 0u, partial_cap)) {
     cudaMemsetAsync(sync_words, 0, 65 * sizeof(unsigned), s);
@@ -1138,7 +1253,7 @@ cudaError_t invariant_measure(const uint32_t* tptr, const uint32_t* trows, const
 
 int measure_partial_slots()
 {
-  return 2 * device_sm_count() * 12;
+  return 2 * device_sm_count() * 14;
 }
 
 }  // namespace b12g

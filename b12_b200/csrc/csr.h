@@ -33,6 +33,7 @@ struct CountPlan {
   uint32_t largest = 0;                // largest count
   uint32_t distinct = 0;               // most of a block
   uint32_t chunk = 0;                  // entries a thread
+  bool pair = false;                   // rows are summed in pairs
 };
 cudaError_t invariant_measure(const uint32_t* tptr, const uint32_t* trows, const double* tvals,
                               const uint32_t* mid_list, uint32_t n_mid, const uint32_t* long_list, uint32_t n_long,
@@ -53,7 +54,7 @@ uint32_t count_distinct_cap(uint64_t nnz);
 cudaError_t count_plan(const uint32_t* tptr, const uint32_t* trows, const double* tvals, uint32_t n, uint64_t nnz,
                        uint32_t points, uint32_t* pack, uint32_t* dlist, uint32_t* dcount, uint32_t* flags,
                        cudaStream_t s);
-uint32_t count_chunk(uint64_t nnz, uint32_t max_row, uint32_t flags, uint32_t distinct, uint32_t largest);
+uint32_t count_chunk(uint64_t nnz, uint32_t max_row, uint32_t flags, uint32_t distinct, uint32_t largest, bool pair);
 // *out = the longest row of the n rows of tptr (asynchronous)
 cudaError_t max_row_length(const uint32_t* tptr, uint32_t n, uint32_t* out, cudaStream_t s);
 
