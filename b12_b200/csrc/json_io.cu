@@ -361,18 +361,22 @@ b12g_status b12g_csr_save_json(const b12g_csr* m, const char* path)
 
 namespace {
 
-// the smallest P <= 255 over which the first values are counts RN(c / P), c = 1..255, as a
-// saved transition matrix's are; 0: none.  (Only a hint: the packing checks every value.)
+// the smallest P <= 255 over which the values are counts RN(c / P), c = 1..255, as a saved
+// transition matrix's are; 0: none.  All of them are looked at: the power iteration sums a
+// matrix of counts in an order of its own, and a loaded matrix gives the same bits as the one
+// that was saved.  (A value that a smaller P did not explain is tried first on the next.)
 uint32_t counts_over(const std::vector<double>& vals)
 {
-  const size_t n = std::min<size_t>(vals.size(), 1024);
-  for (uint32_t p = 1; n && p <= 255; ++p) {
-    size_t i = 0;
-    for (; i < n; ++i) {
-      const double c = std::rint(vals[i] * double(p));
-      if (!(c >= 1.0 && c <= 255.0 && c / double(p) == vals[i])) break;
-    }
-    if (i == n) return p;
+  auto fits = [](double v, uint32_t p) {
+    const double c = std::rint(v * double(p));
+    return c >= 1.0 && c <= 255.0 && c / double(p) == v;
+  };
+  std::vector<double> hard;
+  for (uint32_t p = 1; !vals.empty() && p <= 255; ++p) {
+    if (!std::all_of(hard.begin(), hard.end(), [&](double v) { return fits(v, p); })) continue;
+    const auto bad = std::find_if(vals.begin(), vals.end(), [&](double v) { return !fits(v, p); });
+    if (bad == vals.end()) return p;
+    hard.push_back(*bad);
   }
   return 0;
 }
