@@ -268,9 +268,9 @@ __global__ void __launch_bounds__(512) batch_image_kernel(const BatchArgs a)
 }
 
 
-// The same with the screened evaluation (screen.cuh), a point a thread, and the work queue of
-// the single-tree image kernel (units of 32 points; four at a time while many are left): a
-// step of few points then still fills the GPU.  A block's queue items of 8,192 points left
+// The same with the screened evaluation (screen.cuh), a point a thread, and a work queue of
+// 32-point units (UnitQueue, every piece from the counter; four at a time while many are
+// left): a step of few points then still fills the GPU.  A block's queue items of 8,192 points left
 // all but a few SMs idle in the small steps of served jobs.  16 Lorenz instances of depth 24
 // run in 24.7 ms against 31.1 (FMA) and 45.6 (strict); with five blocks an SM (48 registers,
 // spills) 24.9, with six 25.2.  The forced Duffing ticks of 48 served jobs: 5.4 ms against
@@ -335,16 +335,10 @@ __global__ void __launch_bounds__(256, 4) batch_screen_kernel(const BatchArgs a)
   // and more keep it in 32 bits)
   uint32_t shift = 0;
   while (((total + 31) >> (5 + shift)) >= 0x40000000ull) ++shift;
-  const uint32_t units = uint32_t((total + (32ull << shift) - 1) >> (5 + shift));
-  const uint32_t fine = gridDim.x * (256 / 32) * kScreenFine;
-  const uint32_t coarse_end = units > fine ? units - fine : 0;
-  uint32_t c = 0;
+  UnitQueue<kScreenTrips, kScreenFine, false> q(a.queue, uint32_t((total + (32ull << shift) - 1) >> (5 + shift)));
   ScreenTrial trial;
-  for (;;) {
-    const uint32_t size = c < coarse_end ? kScreenTrips : 1u;
-    if (lane == 0) c = atomicAdd(a.queue, size);
-    c = __shfl_sync(0xFFFFFFFFu, c, 0);
-    if (c >= units) break;
+  for (bool more = q.any(); more; more = q.next()) {
+    const uint32_t c = q.at, size = q.size;
     const uint64_t g = (uint64_t(c) << (5 + shift)) + uint64_t(lane);
     uint32_t child, k;
     if (total <= 0xFFFFFFFFull - 64ull * kScreenTrips) {

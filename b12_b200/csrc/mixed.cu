@@ -889,8 +889,8 @@ __global__ void __launch_bounds__(kThreads) mixed_image_kernel(const MixedArgs a
   }
 }
 
-// modes 0 and 1 with the screened evaluation and the image kernel's work queue (units of 32
-// points, four at a time while many are left).  Bound by FP64 issue, like that kernel; the
+// modes 0 and 1 with the screened evaluation and a work queue of 32-point units (UnitQueue,
+// every piece from the counter; four at a time while many are left).  Bound by FP64 issue, like that kernel; the
 // leaves' centres come from a table of one pass over the leaves instead of being rebuilt for
 // every point.  Six selective steps of Lorenz (FMA) from depth 20: 1.95 ms against 2.46 (five
 // blocks an SM 1.99, six 2.01).
@@ -903,19 +903,13 @@ __global__ void __launch_bounds__(kThreads, kScreenBlocks) mixed_screen_kernel(c
   const uint64_t P = a.points, total = uint64_t(a.n_src) * P;
   const uint32_t P32 = uint32_t(P);
   const int lane = threadIdx.x & 31;
-  constexpr uint32_t kTrips = 4, kFine = 4;
+  constexpr uint32_t kTrips = 4, kFine = 4;      // as for the image kernel
   uint32_t shift = 0;
   while (((total + 31) >> (5 + shift)) >= 0x40000000ull) ++shift;
-  const uint32_t units = uint32_t((total + (32ull << shift) - 1) >> (5 + shift));
-  const uint32_t fine = gridDim.x * (kThreads / 32) * kFine;
-  const uint32_t coarse_end = units > fine ? units - fine : 0;
-  uint32_t c = 0;
+  UnitQueue<kTrips, kFine, false> q(a.work, uint32_t((total + (32ull << shift) - 1) >> (5 + shift)));
   ScreenTrial trial;
-  for (;;) {
-    const uint32_t size = c < coarse_end ? kTrips : 1u;
-    if (lane == 0) c = atomicAdd(a.work, size);
-    c = __shfl_sync(0xFFFFFFFFu, c, 0);
-    if (c >= units) break;
+  for (bool more = q.any(); more; more = q.next()) {
+    const uint32_t c = q.at, size = q.size;
     const uint64_t g = (uint64_t(c) << (5 + shift)) + uint64_t(lane);
     uint32_t rank, k;
     if (total <= 0xFFFFFFFFull - 64ull * kTrips) {
