@@ -270,10 +270,10 @@ __global__ void __launch_bounds__(512) batch_image_kernel(const BatchArgs a)
 
 // The same with the screened evaluation (screen.cuh), a point a thread, and a work queue of
 // 32-point units (UnitQueue, every piece from the counter; four at a time while many are
-// left): a step of few points then still fills the GPU.  A block's queue items of 8,192 points left
-// all but a few SMs idle in the small steps of served jobs.  16 Lorenz instances of depth 24
-// run in 24.7 ms against 31.1 (FMA) and 45.6 (strict); with five blocks an SM (48 registers,
-// spills) 24.9, with six 25.2.  The forced Duffing ticks of 48 served jobs: 5.4 ms against
+// left): a step of few points then still fills the GPU.  A block's queue items of 8,192 points
+// left all but a few SMs idle in the small steps of served jobs.  16 Lorenz instances of depth
+// 24 run in 25.1 ms against 31.1 (FMA) and 45.6 (strict); five blocks an SM (48 registers,
+// spills) take 1 % longer, six 2 %.  The forced Duffing ticks of 48 served jobs: 5.4 ms against
 // 32.3 (the shape with four points a thread).
 constexpr uint32_t kScreenTrips = 4, kScreenFine = 4;
 
@@ -354,7 +354,6 @@ __global__ void __launch_bounds__(256, 4) batch_screen_kernel(const BatchArgs a)
     for (uint32_t trip = 0; trip < (size << shift); ++trip) {
       const bool active = g + 32ull * trip < total;
       uint32_t t = kInvalidIndex;
-      bool failed = false;
       if (active) {
         const uint64_t code = (__ldg(a.codes + (child >> 1)) << 1) | (child & 1u);
         const int depth = uni ? a.depth : int(__ldg(a.inst_depth + inst));
@@ -364,7 +363,6 @@ __global__ void __launch_bounds__(256, 4) batch_screen_kernel(const BatchArgs a)
         const ScreenRec* rec = a.screen + inst;
         const bool tried = trial.on() && __ldg(&rec->on) != 0u;
         const bool sure = tried && screened_point<Map>(rec, a.sk, a.sA, a.map, pts, P, k, sb, tb, inside);
-        failed = tried && !sure;
         if (!sure) {
           undecided += tried ? 1u : 0u;
           const uint64_t cc[1] = {child};
@@ -381,7 +379,6 @@ __global__ void __launch_bounds__(256, 4) batch_screen_kernel(const BatchArgs a)
           if (p != kInvalidIndex) t = 2u * p + uint32_t(tcode & 1u);
         }
       }
-      if constexpr (ScreenTrial::by_unit(D)) trial.note(failed, 1);
       if (t < kOutsideIndex) a.hit[t] = 1;
       if (a.targets && active) {
         const uint64_t base = __ldg(a.tgt_base + inst);
@@ -391,7 +388,7 @@ __global__ void __launch_bounds__(256, 4) batch_screen_kernel(const BatchArgs a)
       while (k >= P) { k -= P; ++child; }
       while (inst + 1 < a.n_inst && (child >> 1) >= off_s[inst + 1]) ++inst;
     }
-    if constexpr (!ScreenTrial::by_unit(D)) trial.note(undecided, size << shift);
+    trial.note(undecided, size << shift);
   }
 }
 
@@ -471,8 +468,8 @@ __global__ void copy_finished_kernel(const uint64_t* code, const uint8_t* flags,
 }
 
 // Bound by FP64 issue.  kScreen: with the screened evaluation of the instance's last step;
-// the matrices of 32 Lorenz instances of depths 18 to 22 (5^3 points a box) take 3.35 ms
-// against 3.86 (FMA) and 5.57 (strict), of 16 forced Duffing ones of depths 15 to 18 0.82
+// the matrices of 32 Lorenz instances of depths 18 to 22 (5^3 points a box) take 3.60 ms
+// against 3.86 (FMA) and 5.57 (strict), of 16 forced Duffing ones of depths 15 to 18 0.83
 // against 1.32.  A record serves a whole row, so its fields are read from L1 per point.
 template<class Map, class Grid, bool kScreen>
 __global__ void __launch_bounds__(256, kScreen ? 4 : 1) batch_rows_kernel(const BatchRowArgs a)

@@ -1011,9 +1011,10 @@ __device__ __forceinline__ void duffing_apply_multi(const MapParams& m, const do
 // tree's capacity paid an atomic at one address, however little there was to do.
 // Every lane of the warp calls next().
 // kOwnFirst = false: they do (Mark mode, whose launches are large and whose kernel is short
-// of registers: the continuation 9.25 ms against 10.18 with own first pieces).  The image
-// launches of a Henon job of 20 steps take 90 us against 160, of a depth-22 forced Duffing
-// job 1.41 ms against 1.45, of a depth-27 Lorenz job 5.47 against 5.52.
+// of registers: the continuation 9.27 ms against 10.18 with own first pieces, and the batched
+// and mixed-depth kernels).  Own first pieces took the image launches of a Henon job of 20
+// steps from 160 to 90 us, of a depth-22 forced Duffing job from 1.45 to 1.41 ms, of a
+// depth-27 Lorenz job from 5.52 to 5.47.
 template<uint32_t kTake, uint32_t kFine, bool kOwnFirst = true>
 struct UnitQueue {
   uint32_t* counter;

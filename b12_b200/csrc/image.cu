@@ -151,10 +151,10 @@ struct PointImage {
 constexpr uint32_t kPointTable = 2048;  // doubles of grid-point table per block (16 KB)
 constexpr int kChunkTrips = 4;          // units (a point a lane) a warp takes at a time from the work queue;
                                         // twice as many in Mark mode, whose points are short and whose
-                                        // launches large (the continuation 9.26 ms, with four 9.46)
-constexpr int kFineUnits = 4;           // units a warp left in the queue when it takes single ones (1: a
-                                        // depth-22 forced Duffing job's image launches 1.64 ms, 4: 1.48, 8: 1.45,
-                                        // while the continuation's take 11.07, 11.13 and 11.47 ms)
+                                        // launches large (the continuation 9.27 ms, with four 9.46)
+constexpr int kFineUnits = 4;           // units a warp left in the queue when it takes single ones: more suit a
+                                        // forced Duffing job's small launches (1, 4 and 8 in ratio: 1.11, 1,
+                                        // 0.98), fewer the continuation's large ones (0.995, 1, 1.03)
 
 // fills `pts` with the P x D grid points when they fit (returns true), else with the
 // 1-D coordinates for the per-point path
@@ -180,7 +180,7 @@ __device__ __forceinline__ bool load_points(const GridParams& g, uint64_t P, dou
 // image launches of a depth-27 job take 5.52 ms against 6.58 (FMA) and 10.21 (strict).  Four
 // blocks an SM, 64 registers: the coefficients stay in registers over the unrolled steps
 // (five blocks with 48: 5.72 ms, three: 5.52).  Mark mode (the continuation, short points):
-// five blocks, 9.46 ms against 9.62 with four.
+// five blocks, 9.27 ms, 2 % less than with four.
 template<class Map, class Grid, ImageMode M, bool kScreen>
 __global__ void __launch_bounds__(kThreads, !kScreen ? 6 : M == ImageMode::Mark ? 5 : 4) image_points_kernel(const ImageArgs a)
 {
@@ -223,8 +223,8 @@ __global__ void __launch_bounds__(kThreads, !kScreen ? 6 : M == ImageMode::Mark 
   const bool table = load_points<Grid, Map::D>(a.grid, a.points, pts);   // (ends with a block barrier)
 
   // Mark mode: the warp's new boxes (the same in every lane), added to the launch's count at
-  // the end (an atomic for every warp with a new box held the continuation's image launches
-  // at 10.8 ms; without them 9.6)
+  // the end (an atomic for every warp with a new box cost the continuation's image launches
+  // an eighth of their time)
   uint32_t new_boxes = 0;
   // (the coupled Duffing continuation always tries: its points are short and few of them stay
   // undecided; 10.68 ms, with the trial 10.85)

@@ -121,9 +121,9 @@ __host__ __device__ __forceinline__ void lorenz_screen_step(const K* k, T (&x)[3
 // Stormer-Verlet of H = |p|^2/2 - q1^2/2 + q1^4/4 + 1.69 q2^2/2 + 0.1 q1^2 q2^2 with
 // Q1 = h q1, Q2 = sqrt(0.2) h q2, P1 = h^2 p1, P2 = sqrt(0.2) h^2 p2: a drift is Q + P and a
 // kick P1 += Q1 (h^2 - Q1^2 - Q2^2), P2 += Q2 (-1.69 h^2 - 0.2 Q1^2).  The half drifts of
-// consecutive steps join: 7 operations a step.  The image launches of the depth-24
-// continuation take 11.0 ms against 15.5 with these steps alone (9.26 with the counting and
-// the codes of the Mark launches made cheaper: the Philox points and the marking dominate).
+// consecutive steps join: 7 operations a step.  These steps alone took the
+// image launches of the depth-24 continuation from 15.5 to 11.0 ms; the Philox points and the
+// marking are most of what is left.
 // k: h^2, 0.2, -(1.69 + 0.2) h^2
 template<class T, class K>
 __host__ __device__ __forceinline__ void duffing_screen_kick(const K* k, T (&x)[4])
@@ -152,9 +152,9 @@ __host__ __device__ __forceinline__ void duffing_screen_half_drift(T (&x)[4])
 // X = c sqrt(beta) x and V = c^2 sqrt(beta) x': c X' = V and
 //   c V' = -c delta V - X (c^2 alpha + X^2) + F(t),
 // RK4 put together as for Lorenz: 25 operations a step and the two of F = k[3] cos at the
-// middle and the end.  f0, f1, f2: F at the stages' times.  The image launches of a
-// depth-19 job take 2.03 ms against 3.85, of a depth-22 one 2.72 against 5.44, with these
-// steps alone (0.86 and 1.47 with the work queue of 32-point units: small launches).
+// middle and the end.  f0, f1, f2: F at the stages' times.  These steps
+// alone took the image launches of a depth-19 job from 3.85 to 2.03 ms, of a depth-22 one from
+// 5.44 to 2.72 (0.80 and 1.40 with the work queue of 32-point units: small launches).
 // k: -c^2 alpha, -c delta, 1 - c delta, c^3 sqrt(beta) gamma, 1 / 3
 template<class T, class K>
 __host__ __device__ __forceinline__ void forced_screen_step(const K* k, const T& f0, const T& f1, const T& f2,
@@ -294,9 +294,9 @@ template<> struct Screen<ForcedDuffingMap> {
 // another one, or more, for 31.  Two, since 4 % of the points are undecided in the usual
 // forced Duffing jobs, where trying still pays.  Counted by pieces, not by points, since the
 // points' loop is bound by its instructions (a vote for every 32 points cost a Lorenz job of
-// depth 27 1.2 %), but in the two-dimensional image launches, whose points are longer and
+// depth 27 1.2 %), but in a tree's two-dimensional image launches, whose points are longer and
 // launches smaller, by units of 32 points (a forced Duffing job of depth 19: 1,142 us, by
-// pieces 1,222, always trying 1,174).
+// pieces 1,222, always trying 1,174; the batches' launches lose 1 to 2 % either way).
 // Images of 250,000 Lorenz boxes (125 points, h = 0.02, radius 10 around 0; 3 % of the points
 // decided): 2.92 ms (strict) and 1.86 (FMA), always trying 4.21 and 3.17, never 2.82 and 1.75.
 // `undecided`: the lane's undecided points of the piece's `tries`.  Every lane calls note()
