@@ -924,7 +924,7 @@ b12g_status ensure_transpose(b12g_csr* m)
     const bool on_chip = measure_on_chip(m->nnz, max_row, uint32_t(measure_partial_slots()));
     if (pack)
       m->plan = CountPlan{m->pack.p, m->dlist.p, m->dcount.p, double(m->count_points), got[3], got[2],
-                          count_chunk(m->nnz, max_row, got[1], got[2], got[3], !on_chip), !on_chip};
+                          count_chunk(m->nnz, max_row, got[1], got[2], got[3]), !on_chip};
     if (m->plan.chunk || on_chip) {
       // the power iteration keeps the matrix on chip and reads no row-class lists
       m->n_mid = 0;

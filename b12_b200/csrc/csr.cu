@@ -795,8 +795,9 @@ __global__ void __launch_bounds__(kMeasureThreads, 1) invariant_measure_count_ke
   double* s_v = s_val + counts;
   // after an iteration's walk the staged values' place holds the runs' first parts
   double* s_head = s_v;
-  double* s_head_lo = s_v + kMeasureThreads;      // kPair only
-  uint32_t* s_head_end = reinterpret_cast<uint32_t*>(s_v + (kPair ? 2 : 1) * kMeasureThreads);
+  // bit 0: the run ends the row; kPair, the other bits: the part's second half relative to its
+  // first as a float (8 more bytes a thread would not fit beside 52 entries)
+  uint32_t* s_head_end = reinterpret_cast<uint32_t*>(s_v + kMeasureThreads);
   __shared__ double red[kMeasureThreads / 32], red_lo[kPair ? kMeasureThreads / 32 : 1];
   __shared__ uint32_t s_bnd[32 * kDepWords + 1];
   __shared__ uint32_t s_dep[kDepWords];
@@ -951,18 +952,24 @@ __global__ void __launch_bounds__(kMeasureThreads, 1) invariant_measure_count_ke
     __syncthreads();
     if (any && head_open) {
       // (a run inside one row has its whole sum in acc and leaves the row open)
-      s_head[t] = first ? acc : head;
-      if constexpr (kPair) s_head_lo[t] = first ? acc_lo : head_lo;
-      s_head_end[t] = first && tail_open ? 0u : 1u;
+      const double h = first ? acc : head;
+      s_head[t] = h;
+      uint32_t end = first && tail_open ? 0u : 1u;
+      if constexpr (kPair)
+        if (precise && h != 0.0)
+          end |= __float_as_uint(__double2float_rn(__ddiv_rn(first ? acc_lo : head_lo, h))) & ~1u;
+      s_head_end[t] = end;
     }
     __syncthreads();
     if (any && tail_open && !(first && head_open)) {
       // this run holds the row's first entry: add the later runs' parts in order
       double sum = acc, sum_lo = acc_lo;
       for (uint32_t j = t + 1; j < blockDim.x; ++j) {
-        if (precise) two_add(s_head[j], s_head_lo[j], sum, sum_lo);
-        else sum = __dadd_rn(sum, s_head[j]);
-        if (s_head_end[j]) break;
+        const uint32_t end = s_head_end[j];
+        const double h = s_head[j];
+        if (precise) two_add(h, __dmul_rn(double(__uint_as_float(end & ~1u)), h), sum, sum_lo);
+        else sum = __dadd_rn(sum, h);
+        if (end & 1u) break;
       }
       if (precise) sum = __dadd_rn(sum, sum_lo);
       __stcg(wc + row, sum);
@@ -1171,22 +1178,22 @@ cudaError_t count_plan(const uint32_t* tptr, const uint32_t* trows, const double
 
 namespace {
 
-size_t count_bytes(uint32_t chunk, uint32_t distinct, uint32_t counts, bool pair)
+size_t count_bytes(uint32_t chunk, uint32_t distinct, uint32_t counts)
 {
   return size_t(chunk) * kMeasureThreads * 4 + size_t(counts) * 8 +
-         std::max<size_t>(size_t(distinct) * 8, size_t(kMeasureThreads) * (pair ? 20 : 12));
+         std::max<size_t>(size_t(distinct) * 8, size_t(kMeasureThreads) * 12);
 }
 
 }  // namespace
 
-uint32_t count_chunk(uint64_t nnz, uint32_t max_row, uint32_t flags, uint32_t distinct, uint32_t largest, bool pair)
+uint32_t count_chunk(uint64_t nnz, uint32_t max_row, uint32_t flags, uint32_t distinct, uint32_t largest)
 {
   const uint32_t blocks = uint32_t(device_sm_count());
   if (flags != 0 || max_row > kMidRow) return 0;
   // a block's rows begin in its share of the entries and have at most kMidRow entries
   const uint64_t most = (nnz + blocks - 1) / blocks + kMidRow;
   const uint32_t chunk = uint32_t((most + 4 * kMeasureThreads - 1) / (4 * kMeasureThreads)) * 4;
-  return chunk <= kCountMaxChunk && count_bytes(chunk, distinct, largest + 1, pair) <= kCountSmemLimit ? chunk : 0;
+  return chunk <= kCountMaxChunk && count_bytes(chunk, distinct, largest + 1) <= kCountSmemLimit ? chunk : 0;
 }
 
 cudaError_t max_row_length(const uint32_t* tptr, uint32_t n, uint32_t* out, cudaStream_t s)
@@ -1222,7 +1229,7 @@ cudaError_t invariant_measure(const uint32_t* tptr, const uint32_t* trows, const
     const void* kernel = plan->pair ? (const void*)invariant_measure_count_kernel<true>
                                     : (const void*)invariant_measure_count_kernel<false>;
     return cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(kMeasureThreads), params,
-                                       count_bytes(chunk, plan->distinct, counts, plan->pair), s);
+                                       count_bytes(chunk, plan->distinct, counts), s);
   }
   if (mid_list && long_list && n_long == 0 && measure_on_chip(nnz, 0u, partial_cap)) {
     cudaMemsetAsync(sync_words, 0, 65 * sizeof(unsigned), s);

@@ -54,7 +54,7 @@ uint32_t count_distinct_cap(uint64_t nnz);
 cudaError_t count_plan(const uint32_t* tptr, const uint32_t* trows, const double* tvals, uint32_t n, uint64_t nnz,
                        uint32_t points, uint32_t* pack, uint32_t* dlist, uint32_t* dcount, uint32_t* flags,
                        cudaStream_t s);
-uint32_t count_chunk(uint64_t nnz, uint32_t max_row, uint32_t flags, uint32_t distinct, uint32_t largest, bool pair);
+uint32_t count_chunk(uint64_t nnz, uint32_t max_row, uint32_t flags, uint32_t distinct, uint32_t largest);
 // *out = the longest row of the n rows of tptr (asynchronous)
 cudaError_t max_row_length(const uint32_t* tptr, uint32_t n, uint32_t* out, cudaStream_t s);
 

@@ -27,7 +27,8 @@ def measure_in_80_bits(n, rowptr, cols, vals, iters):
 # u / 2 in the mean square; a row averages the earlier iterates' errors over its ten sources and
 # more (0.2 u).  Together 0.8 u: 0.9e-16.  (One sum from start to end gives 1.3 to 2.0e-16.)
 @pytest.mark.parametrize("n,P,spread,iters,seed", [(300000, 16, 40, 40, 1), (300000, 16, 9, 25, 2),
-                                                   (260000, 16, 60, 24, 3), (600000, 16, 40, 17, 4)])
+                                                   (260000, 16, 60, 24, 3), (600000, 16, 40, 17, 4),
+                                                   (265000, 32, 120, 20, 5)])
 def test_measure_of_a_large_matrix(n, P, spread, iters, seed):
     m = matrix(near(np.arange(n), n, np.random.default_rng(seed), P, spread), n)
     rowptr, cols, vals = m.to_host()
