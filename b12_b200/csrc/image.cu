@@ -175,7 +175,7 @@ __device__ __forceinline__ bool load_points(const GridParams& g, uint64_t P, dou
 }
 
 // Bound by instruction issue: an FP64 instruction holds its scheduler for two cycles and
-// any other for one.  kScreen: the screened evaluation (screen.cuh), 735 FP64 and about 330
+// any other for one.  kScreen: the screened evaluation (screen.cuh), 736 FP64 and about 310
 // other instructions per 32 Lorenz points against 942 and 290 (FMA) or 1,600 (strict); the
 // image launches of a depth-27 job take 5.52 ms against 6.58 (FMA) and 10.21 (strict).  Four
 // blocks an SM, 64 registers: the coefficients stay in registers over the unrolled steps
